@@ -283,6 +283,7 @@ struct DControl {
   unsigned long long max_failed;
   unsigned long long* stop;
   const unsigned long long* abort;
+  int regen; /* lanes still under way at which a warp takes new paths */
 };
 
 /* Path tracking (ssol_path_tracker): the realisations of launch index

@@ -72,10 +72,7 @@ static int launch_batch_noalloc_variant
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   const int block = cfg.block_size > 0 ? cfg.block_size : MAX_BLOCK;
   if(block > MAX_BLOCK || block % 32) return (int)cudaErrorInvalidValue;
-  const size_t smem = (size_t)((2 * NGLOBAL + PS_COUNT) * block) * sizeof(double)
-                    + (size_t)SMEM_STACK * block * sizeof(int)
-                    + (size_t)(block / 32) * 2 * (2 * NGLOBAL + cfg.rcv_doubles) * sizeof(double)
-                    + (size_t)(block / 32) * 2 * sizeof(DScene<R>);
+  const size_t smem = path_smem(FEAT, block) + (size_t)(block / 32) * 2 * sizeof(DScene<R>);
   raise_smem_limit<BatchTag<R, MINB, FEAT>>(batch_kernel<R, MINB, FEAT>, dev);
   int per_sm = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor
@@ -101,8 +98,9 @@ static int launch_batch_noalloc_variant
   batch_kernel<R, MINB, FEAT><<<(unsigned)blocks, block, smem, s>>>
     (scenes, tallies, scratch + NOALLOC_PREFIX, scratch + NOALLOC_FIRSTS, nitems,
      seed, cfg.max_segments, scratch + NOALLOC_NEXT,
-     reinterpret_cast<DStats*>(scratch + NOALLOC_STATS), cfg.rcv_doubles,
+     reinterpret_cast<DStats*>(scratch + NOALLOC_STATS), regen_lanes(cfg.features),
      nullptr, nullptr, nullptr); /* id order: the coherent order needs scratch */
+  finish_batch<R>(scenes, tallies, nitems, cfg.max_nrcv, s);
   return (int)cudaGetLastError();
 }
 

@@ -18,11 +18,11 @@
  *   sun direction samplers src/ssol_ranst_sun_dir.c:177-310
  * Tallies are FP64 (sum w, sum w^2) of each realisation's total, exactly the
  * deferred mc_data semantics of src/ssol_estimator_c.h:59-126: a path keeps
- * its per-receiver contributions in registers until it ends, applies the
- * Russian-roulette factor, then commits. Global quantities are reduced per
- * warp with __shfl_xor_sync and committed once per block; receiver-side sums
- * go through shared memory; sparse ones (per sampled instance, per primitive)
- * use FP64 atomics.
+ * its per-receiver contributions until it ends, applies the Russian-roulette
+ * factor, then commits. The paths of a warp commit together: sums of the
+ * global quantities and of the warp's sampled instance are added up by FP64
+ * tensor-core products (commit_warp), the sparse ones (per primitive) by FP64
+ * reductions in device memory.
  *
  * Geometry, sampling and BSDFs run in the template type R (float for the
  * plain build, double for the all-FP64 build); quadric roots found in FP32 get
@@ -36,6 +36,7 @@
 #include "philox.h"
 
 #include <cuda_runtime.h>
+#include <algorithm>
 #include <float.h>
 #include <math.h>
 
@@ -725,7 +726,12 @@ __device__ bool trace_ray
  * blockDim): the first receiver entry's 6 values, the 3 global quantities
  * accumulated along the path and the cosine factor */
 enum : int { PS_V0 = 0, PS_ABS = 6, PS_ATM = 7, PS_OTHER = 8, PS_COS = 9,
-             PS_UV = 10, PS_COUNT = 11 };
+             PS_UV = 10 };
+/* Path sums a kernel variant keeps: PS_UV only with shading attributes
+ * (without it three blocks of 256 threads of the plain kernel fit the SM's
+ * 132 KB shared-memory configuration) */
+__host__ __device__ constexpr int ps_count(int feat)
+{ return feat & FEAT_ATTRIBUTES ? 11 : 10; }
 
 /* Barycentric weights (b1, b2) of vertices 1 and 2 of triangle gid at the
  * point x of its plane */
@@ -932,12 +938,12 @@ __device__ __noinline__ bool shade
  *
  * Each warp iteration casts exactly one ray per active lane, from a single
  * call site: the shadow ray of a new path (any hit) or the next segment of a
- * path (closest hit). Around it, lanes regenerate (fetch a new realisation
- * through a warp-aggregated atomic counter), interact with the surface they
- * reached, or commit a finished path. Lanes never wait for the longest path
- * of their warp, and lanes in different phases still trace together.
+ * path (closest hit). Lanes start together, cast their shadow rays together
+ * and then each segment; those that have ended wait (regen_lanes), commit
+ * together and take the next realisations through a warp-aggregated atomic
+ * counter.
  ******************************************************************************/
-enum : int { PH_NONE = 0, PH_SHADOW = 1, PH_BOUNCE = 2 };
+enum : int { PH_NONE = 0, PH_SHADOW = 1, PH_BOUNCE = 2, PH_ENDED = 3 };
 enum : int {
   END_NONE = 0, END_SHADOW, END_MISS, END_ZERO, END_KILL, END_FAIL
 };
@@ -946,11 +952,7 @@ enum : int {
  * kept in local memory: only paths reaching several receivers touch them */
 constexpr int MAX_EXTRA = 7;
 
-__device__ __forceinline__ void red_add(double* p, double v)
-{
-  if(v != 0.0) atomicAdd(p, v);
-}
-/* The same into device memory, as a reduction (no value comes back): an
+/* Sums into device memory, as reductions (no value comes back): an
  * atomicAdd through a pointer that may address shared memory is a generic
  * atomic whose sector returns to L1 */
 __device__ __forceinline__ void red_add_global(double* p, double v)
@@ -959,24 +961,18 @@ __device__ __forceinline__ void red_add_global(double* p, double v)
     asm volatile("red.global.add.f64 [%0], %1;"
                  :: "l"(__cvta_generic_to_global(p)), "d"(v) : "memory");
 }
-__device__ __forceinline__ void red_add_shared(double* p, double v)
+__device__ __forceinline__ void red_count_global(unsigned long long* p, unsigned long long n)
 {
-  if(v != 0.0)
-    asm volatile("red.shared.add.f64 [%0], %1;"
-                 :: "r"((unsigned)__cvta_generic_to_shared(p)), "d"(v) : "memory");
-}
-__device__ __forceinline__ void red_inc_global(unsigned long long* p)
-{
-  asm volatile("red.global.add.u64 [%0], 1;"
-               :: "l"(__cvta_generic_to_global(p)) : "memory");
+  asm volatile("red.global.add.u64 [%0], %1;"
+               :: "l"(__cvta_generic_to_global(p)), "l"(n) : "memory");
 }
 
 /* (w, w^2) of the 10 receiver quantities of one path, from its 6
  * accumulated values (MC_RECEIVER_DATA order, src/ssol_solver.c:735-755:
  * incoming, incoming if no atmosphere loss, if no field loss, lost in the
- * field, lost in the atmosphere, then the same 5 absorbed), added to dst. The values travel as scalars, so that
- * none of them goes through local memory. */
-template<bool GLOBAL>
+ * field, lost in the atmosphere, then the same 5 absorbed), added to dst in
+ * device memory. The values travel as scalars, so that none of them goes
+ * through local memory. */
 static __device__ __noinline__ void commit10
   (double* dst, double v0, double v1, double v2, double v3, double v4, double v5,
    double f)
@@ -985,36 +981,18 @@ static __device__ __noinline__ void commit10
                             f * v3, f * v4, f * v5, f * (v5 - v3), f * (v4 - v3)};
 #pragma unroll
   for(int k = 0; k < NRCV_Q; ++k) {
-    if(GLOBAL) {
-      red_add_global(dst + 2 * k, q[k]);
-      red_add_global(dst + 2 * k + 1, q[k] * q[k]);
-    } else {
-      red_add(dst + 2 * k, q[k]);
-      red_add(dst + 2 * k + 1, q[k] * q[k]);
-    }
+    red_add_global(dst + 2 * k, q[k]);
+    red_add_global(dst + 2 * k + 1, q[k] * q[k]);
   }
 }
-/* GLOBAL: dst is device memory (else shared or device memory) */
-template<bool GLOBAL>
 __device__ __forceinline__ void commit10(double* dst, const double v[6], double f)
 {
-  commit10<GLOBAL>(dst, v[0], v[1], v[2], v[3], v[4], v[5], f);
-}
-
-/* dst: shared memory when `shared`, else device memory */
-static __device__ __noinline__ void flush_racc(double* dst, const double* racc, bool shared)
-{
-  if(shared) {
-#pragma unroll 1
-    for(int k = 0; k < 2 * NRCV_Q; ++k) red_add_shared(dst + k, racc[k]);
-  } else {
-#pragma unroll 1
-    for(int k = 0; k < 2 * NRCV_Q; ++k) red_add_global(dst + k, racc[k]);
-  }
+  commit10(dst, v[0], v[1], v[2], v[3], v[4], v[5], f);
 }
 
 template<class R> struct PathState {
   int phase;
+  int end; /* END_* of a path in PH_ENDED */
   int samp;
   int tslot; /* tracked path slot, -1 if not tracked */
   uint32_t tseq; /* vertices recorded so far */
@@ -1223,143 +1201,308 @@ __device__ int interact
   return END_NONE;
 }
 
-/* What commit_path_pe reads of a finished path */
-struct PathEnd {
-  int end; /* END_* */
-  int samp, score, nent, r0, p0;
-  bool overflow;
-  double w_end; /* weight shadowed (END_SHADOW) or missing (END_MISS) */
-};
+/* Running sums of a warp, kept in shared memory as the accumulators of four
+ * FP64 tensor-core tiles (8 rows of 8 partial sums, two per lane):
+ *   tile 0: (w, w^2) of the global quantities absorbed by receivers,
+ *           missing, atmosphere, other, of item `gitem`;
+ *   tile 1: cosine and shadowed of sampled instance `samp` of item `item`
+ *           (rows 0-3), then, with tiles 2 and 3, the 10 receiver quantities
+ *           of its slot `rbase` of samp_rcv (rows 4-7, 0-7, 0-7).
+ * Only these are summed: a receiver side's totals are the sums of its
+ * samp_rcv slots over the sampled instances, and the global cosine and
+ * shadowed those of the samp slots, which finish_tallies adds up once a
+ * launch.
+ *
+ * A commit is the sum of 32 lanes' values into few addresses: bound by the
+ * atomics when each path sends its own (25 reductions a path to one sampled
+ * instance's slots; with a single mirror every path of the GPU to the same
+ * 25 addresses), by instructions when summed by shuffles (5 steps of two
+ * per value). A product with a one-row matrix sums 32 lanes in one
+ * instruction and keeps the running sum in its accumulator, in full FP64.
+ * With the lock-step paths (regen_lanes): one mirror, 1e6 paths, 4.05 ->
+ * 0.55 ms; field, 1e8 paths, 149 -> 92 ms (110 by the lock step alone). */
+struct WarpKeys { int gitem, item, samp, rbase; };
+constexpr int TILES = 4;
 
-template<class R>
-__device__ __forceinline__ PathEnd path_end(const PathState<R>& p, int end)
+/* Row `row` (0..7) of a tile += the sum of v over the 32 lanes: an m8n8k4
+ * product whose A is one in that row and zero elsewhere, and whose B holds
+ * the lanes' values. v must be finite (0 x inf would reach every row). */
+__device__ __forceinline__ void tile_add(double2& d, int row, unsigned lane, double v)
 {
-  PathEnd e;
-  e.end = p.overflow ? END_FAIL : end;
-  e.samp = p.samp;
-  e.score = p.score;
-  e.nent = p.nent;
-  e.r0 = p.r0;
-  e.p0 = p.p0;
-  e.overflow = p.overflow;
-  e.w_end = end == END_MISS && p.virt ? p.inc0 : p.prev[0];
-  return e;
+  const double a = (int)(lane >> 2) == row ? 1.0 : 0.0;
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 "
+               "{%0, %1}, {%2}, {%3}, {%0, %1};"
+               : "+d"(d.x), "+d"(d.y) : "d"(a), "d"(v));
+}
+/* Sum of the lane's row (lane / 4) */
+__device__ __forceinline__ double tile_row_sum(double2 d)
+{
+  double v = d.x + d.y;
+  v += __shfl_xor_sync(0xffffffffu, v, 1);
+  v += __shfl_xor_sync(0xffffffffu, v, 2);
+  return v;
 }
 
-/* Commit a finished path: FP64 (w, w^2) of its totals, x 2^score for
- * roulette survivors (src/ssol_solver.c:1087-1108). Returns the receiver
- * side of the thread's running sums `racc` after the commit. */
-template<class R>
-__device__ __noinline__ int commit_path_pe
-  (const DScene<R>& S, const DTallies& T, const PathEnd& pe, double* acc,
-   double* ps, int stride, double* smem_rcv, const int* xr, const int* xp,
-   const double (*xv)[6], double* racc, int racc_slot, const DControl* ctl)
+/* The warp's tiles into the tallies they are keyed by: tile 0, the samp
+ * rows, or the samp_rcv rows; all lanes call it */
+static __device__ __noinline__ void flush_global
+  (const DTallies* tallies, const WarpKeys* wk, double2* tile)
 {
-  const int end = pe.end;
-  red_inc_global(&T.nb_samples[pe.samp]);
-  if(end == END_FAIL) {
+  const unsigned lane = threadIdx.x & 31u;
+  const double v = tile_row_sum(tile[0]);
+  const int row = (int)(lane >> 2);
+  if((lane & 3u) == 0u && wk->gitem >= 0)
+    red_add_global(tallies[wk->gitem].global + (row < 2 ? 2 * G_ABS_RCV : 2 * G_MISSING - 2) + row,
+                   v);
+  tile[0] = make_double2(0.0, 0.0);
+}
+static __device__ __noinline__ void flush_samp
+  (const DTallies* tallies, const WarpKeys* wk, double2* tile, int stride, bool rcv_only)
+{
+  const unsigned lane = threadIdx.x & 31u;
+  const int row = (int)(lane >> 2);
+  double v[3];
+#pragma unroll
+  for(int k = 0; k < 3; ++k) v[k] = tile_row_sum(tile[(k + 1) * stride]);
+  if((lane & 3u) == 0u && wk->item >= 0) {
+    const DTallies& T = tallies[wk->item];
+    if(row < 4) {
+      if(!rcv_only) red_add_global(T.samp + (size_t)wk->samp * 4 + row, v[0]);
+    }
+    if(wk->rbase >= 0) {
+      double* dst = T.samp_rcv + (size_t)wk->rbase * NRCV_Q * 2;
+      if(row >= 4) red_add_global(dst + row - 4, v[0]);
+      red_add_global(dst + 4 + row, v[1]);
+      red_add_global(dst + 12 + row, v[2]);
+    }
+  }
+  if(row >= 4 || !rcv_only) tile[stride] = make_double2(0.0, 0.0);
+  tile[2 * stride] = tile[3 * stride] = make_double2(0.0, 0.0);
+}
+
+/* Lanes of one sampled instance below which their sums go straight to
+ * device memory (id-ordered launches, whose lanes sample all over the
+ * scene) */
+constexpr int MIN_GROUP = 4;
+
+/* Commit the finished paths of the lanes with `ended`: FP64 (w, w^2) of each
+ * path's totals, x 2^score for roulette survivors (src/ssol_solver.c:
+ * 1087-1108). All lanes of the warp call it converged. The lanes of one
+ * sampled instance (in the coherent order nearly always the whole warp) add
+ * through the warp's tiles, the others, and any path with a weight that is
+ * not finite, through reductions of their own. */
+template<class R>
+static __device__ __noinline__ void commit_warp
+  (int nrcv, const DTallies* tallies, int item, const PathState<R>& p, bool ended,
+   const double* ps, int stride, double2* tile, WarpKeys* wk, const int* xr,
+   const int* xp, const double (*xv)[6], const DControl* ctl)
+{
+  const unsigned FULL = 0xffffffffu;
+  const unsigned lane = threadIdx.x & 31u;
+  const DTallies& T = tallies[item];
+  const int end = p.overflow ? END_FAIL : p.end;
+  const bool good = ended && end != END_FAIL && end != END_KILL;
+  if(ended && end == END_FAIL) {
     /* The failure that reaches the limit stops the launch's work fetch
      * (src/ssol_solver.c:1240-1245) */
     const unsigned long long nf = atomicAdd(&T.counters[0], 1ull) + 1ull;
     if(ctl && ctl->stop && nf >= ctl->max_failed) atomicExch(ctl->stop, 1ull);
-    if(pe.overflow) atomicAdd(&T.counters[2], 1ull);
-    return racc_slot;
+    if(p.overflow) atomicAdd(&T.counters[2], 1ull);
   }
-  if(end == END_KILL) {
-    atomicAdd(&T.counters[1], 1ull);
-    return racc_slot;
-  }
-  const double f = (double)(1ull << pe.score);
-  const double g[NGLOBAL] = {
-    ps[PS_COS * stride], ps[PS_ABS * stride],
-    end == END_SHADOW ? pe.w_end : 0.0,
-    end == END_MISS ? pe.w_end : 0.0,
-    ps[PS_ATM * stride], ps[PS_OTHER * stride]};
-  if(acc) {
+  if(ended && end == END_KILL) atomicAdd(&T.counters[1], 1ull);
+  const int samp = ended ? p.samp : -1;
+  const int nent = good ? p.nent : 0;
+  const int r0 = nent ? p.r0 : -1;
+  double f = 0, wcos = 0, wabs = 0, wsh = 0, wmiss = 0, watm = 0, woth = 0;
+  double q[NRCV_Q] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
+  double chk = 0;
+  if(good) {
+    f = (double)(1ull << p.score);
+    wcos = f * ps[PS_COS * stride];
+    wabs = f * ps[PS_ABS * stride];
+    watm = f * ps[PS_ATM * stride];
+    woth = f * ps[PS_OTHER * stride];
+    const double w_end = f * (end == END_MISS && p.virt ? p.inc0 : p.prev[0]);
+    if(end == END_SHADOW) wsh = w_end;
+    if(end == END_MISS) wmiss = w_end;
+    chk = wcos * wcos + wabs * wabs + watm * watm + woth * woth + w_end * w_end;
+    if(nent == 1) {
+      const double a0 = ps[(PS_V0 + 0) * stride], a1 = ps[(PS_V0 + 1) * stride];
+      const double a2 = ps[(PS_V0 + 2) * stride], a3 = ps[(PS_V0 + 3) * stride];
+      const double a4 = ps[(PS_V0 + 4) * stride], a5 = ps[(PS_V0 + 5) * stride];
+      q[0] = f * a0; q[1] = f * a1; q[2] = f * a2;
+      q[3] = f * (a2 - a0); q[4] = f * (a1 - a0);
+      q[5] = f * a3; q[6] = f * a4; q[7] = f * a5;
+      q[8] = f * (a5 - a3); q[9] = f * (a4 - a3);
 #pragma unroll
-    for(int q = 0; q < NGLOBAL; ++q) {
-      const double w = f * g[q];
-      acc[(2 * q) * stride] += w;
-      acc[(2 * q + 1) * stride] += w * w;
+      for(int k = 0; k < NRCV_Q; ++k) chk += q[k] * q[k];
     }
   }
-  {
-    const double wc = f * g[G_COS], ws = f * g[G_SHADOW];
-    double* sp = T.samp + (size_t)pe.samp * 4;
-    red_add_global(sp + 0, wc);
-    red_add_global(sp + 1, wc * wc);
-    red_add_global(sp + 2, ws);
-    red_add_global(sp + 3, ws * ws);
+  /* Finite, and its squares too */
+  const bool tame = chk < 1e300;
+
+  /* Global quantities, item by item (one, unless a batch's warp straddles
+   * two) */
+  unsigned rest = __ballot_sync(FULL, good && tame);
+#pragma unroll 1
+  while(rest) {
+    const int it = __shfl_sync(FULL, item, __ffs(rest) - 1);
+    const bool in = good && tame && item == it;
+    rest &= ~__ballot_sync(FULL, in);
+    if(wk->gitem != it) {
+      flush_global(tallies, wk, tile);
+      __syncwarp();
+      if(lane == 0) wk->gitem = it;
+      __syncwarp();
+    }
+    double2 d = tile[0];
+    tile_add(d, 0, lane, in ? wabs : 0.0);
+    tile_add(d, 1, lane, in ? wabs * wabs : 0.0);
+    tile_add(d, 2, lane, in ? wmiss : 0.0);
+    tile_add(d, 3, lane, in ? wmiss * wmiss : 0.0);
+    tile_add(d, 4, lane, in ? watm : 0.0);
+    tile_add(d, 5, lane, in ? watm * watm : 0.0);
+    tile_add(d, 6, lane, in ? woth : 0.0);
+    tile_add(d, 7, lane, in ? woth * woth : 0.0);
+    tile[0] = d;
   }
-  if(pe.nent == 0) return racc_slot;
-  double* rbase = smem_rcv ? smem_rcv : T.rcv;
-  if(pe.nent == 1) {
+  if(good && !tame) {
+    const double g[4] = {wabs, wmiss, watm, woth};
+    const int at[4] = {G_ABS_RCV, G_MISSING, G_ATM, G_OTHER};
+    for(int k = 0; k < 4; ++k) {
+      red_add_global(T.global + 2 * at[k], g[k]);
+      red_add_global(T.global + 2 * at[k] + 1, g[k] * g[k]);
+    }
+  }
+
+  /* Sampled instances and their receivers: at most two of a warp's sampled
+   * instances through the tiles */
+  bool counted = !ended, samp_done = !good, rcv_done = nent != 1;
+  rest = __ballot_sync(FULL, ended);
+#pragma unroll 1
+  for(int pass = 0; pass < 2 && rest; ++pass) {
+    const int leader = __ffs(rest) - 1;
+    const int ks = __shfl_sync(FULL, samp, leader), it = __shfl_sync(FULL, item, leader);
+    const unsigned grp = __ballot_sync(FULL, ended && samp == ks && item == it);
+    if(__popc(grp) < MIN_GROUP) break;
+    rest &= ~grp;
+    const bool in = ((grp >> lane) & 1u) && tame;
+    if((int)lane == leader) red_count_global(&T.nb_samples[ks], (unsigned long long)__popc(grp));
+    const unsigned have = __ballot_sync(FULL, in && nent == 1);
+    int rb = have ? __shfl_sync(FULL, samp * nrcv + r0, __ffs(have) - 1) : -1;
+    const bool on_r = in && nent == 1 && samp * nrcv + r0 == rb;
+    if(wk->item != it || wk->samp != ks) {
+      flush_samp(tallies, wk, tile, stride, false);
+      __syncwarp();
+      if(lane == 0) { wk->item = it; wk->samp = ks; wk->rbase = rb; }
+    } else if(rb >= 0 && wk->rbase != rb) {
+      flush_samp(tallies, wk, tile, stride, true);
+      __syncwarp();
+      if(lane == 0) wk->rbase = rb;
+    }
+    __syncwarp();
+    double2 d = tile[stride];
+    tile_add(d, 0, lane, in ? wcos : 0.0);
+    tile_add(d, 1, lane, in ? wcos * wcos : 0.0);
+    tile_add(d, 2, lane, in ? wsh : 0.0);
+    tile_add(d, 3, lane, in ? wsh * wsh : 0.0);
+    if(rb >= 0) {
+      double2 e = tile[2 * stride], h = tile[3 * stride];
+      double v[NRCV_Q];
+#pragma unroll
+      for(int k = 0; k < NRCV_Q; ++k) v[k] = on_r ? q[k] : 0.0;
+#pragma unroll
+      for(int k = 0; k < 4; ++k) {
+        if(k < 2) {
+          tile_add(d, 4 + 2 * k, lane, v[k]);
+          tile_add(d, 5 + 2 * k, lane, v[k] * v[k]);
+        }
+        tile_add(e, 2 * k, lane, v[2 + k]);
+        tile_add(e, 2 * k + 1, lane, v[2 + k] * v[2 + k]);
+        tile_add(h, 2 * k, lane, v[6 + k]);
+        tile_add(h, 2 * k + 1, lane, v[6 + k] * v[6 + k]);
+      }
+      tile[2 * stride] = e;
+      tile[3 * stride] = h;
+    }
+    tile[stride] = d;
+    counted = counted || ((grp >> lane) & 1u);
+    samp_done = samp_done || in;
+    rcv_done = rcv_done || on_r;
+  }
+  if(!counted) red_count_global(&T.nb_samples[samp], 1ull);
+  if(!samp_done) {
+    double* sp = T.samp + (size_t)samp * 4;
+    red_add_global(sp + 0, wcos);
+    red_add_global(sp + 1, wcos * wcos);
+    red_add_global(sp + 2, wsh);
+    red_add_global(sp + 3, wsh * wsh);
+  }
+  if(nent == 1) {
     const double a0 = ps[(PS_V0 + 0) * stride], a1 = ps[(PS_V0 + 1) * stride];
     const double a2 = ps[(PS_V0 + 2) * stride], a3 = ps[(PS_V0 + 3) * stride];
     const double a4 = ps[(PS_V0 + 4) * stride], a5 = ps[(PS_V0 + 5) * stride];
-    if(racc) {
-      /* The thread's running sums of one receiver side, flushed when the
-       * side changes: no atomics while its paths keep reaching it */
-      if(racc_slot != pe.r0) {
-        if(racc_slot >= 0)
-          flush_racc(rbase + (size_t)racc_slot * NRCV_Q * 2, racc, smem_rcv != nullptr);
-        racc_slot = pe.r0;
-#pragma unroll
-        for(int k = 0; k < 2 * NRCV_Q; ++k) racc[k] = 0.0;
+    if(!rcv_done)
+      commit10(T.samp_rcv + ((size_t)samp * nrcv + r0) * NRCV_Q * 2, a0, a1, a2, a3, a4, a5, f);
+    if(p.p0 >= 0)
+      commit10(T.prim + (size_t)p.p0 * NRCV_Q * 2, a0, a1, a2, a3, a4, a5, f);
+  } else if(nent > 1) {
+    double v0[6];
+    for(int k = 0; k < 6; ++k) v0[k] = ps[(PS_V0 + k) * stride];
+    /* Several entries: sum per receiver side and per primitive before
+     * squaring (deferred mc_data semantics) */
+    for(int e = 0; e < nent; ++e) {
+      const int re = e == 0 ? r0 : xr[e - 1];
+      bool seen = false;
+      for(int k = 0; k < e && !seen; ++k) seen = (k == 0 ? r0 : xr[k - 1]) == re;
+      if(!seen) {
+        double v[6] = {0, 0, 0, 0, 0, 0};
+        for(int k = e; k < nent; ++k) {
+          if((k == 0 ? r0 : xr[k - 1]) != re) continue;
+          for(int c = 0; c < 6; ++c) v[c] += k == 0 ? v0[c] : xv[k - 1][c];
+        }
+        commit10(T.samp_rcv + ((size_t)samp * nrcv + re) * NRCV_Q * 2, v, f);
       }
-      const double q[NRCV_Q] = {f * a0, f * a1, f * a2, f * (a2 - a0), f * (a1 - a0),
-                                f * a3, f * a4, f * a5, f * (a5 - a3), f * (a4 - a3)};
-#pragma unroll
-      for(int k = 0; k < NRCV_Q; ++k) {
-        racc[2 * k] += q[k];
-        racc[2 * k + 1] += q[k] * q[k];
+      const int prim = e == 0 ? p.p0 : xp[e - 1];
+      if(prim >= 0) {
+        /* (receiver side, primitive) keys are unique among the entries */
+        commit10(T.prim + (size_t)prim * NRCV_Q * 2, e == 0 ? v0 : xv[e - 1], f);
       }
-    } else {
-      commit10<false>(rbase + (size_t)pe.r0 * NRCV_Q * 2, a0, a1, a2, a3, a4, a5, f);
-    }
-    commit10<true>(T.samp_rcv + ((size_t)pe.samp * S.nrcv + pe.r0) * NRCV_Q * 2,
-                   a0, a1, a2, a3, a4, a5, f);
-    if(pe.p0 >= 0)
-      commit10<true>(T.prim + (size_t)pe.p0 * NRCV_Q * 2, a0, a1, a2, a3, a4, a5, f);
-    return racc_slot;
-  }
-  double v0[6];
-  for(int q = 0; q < 6; ++q) v0[q] = ps[(PS_V0 + q) * stride];
-  /* Several entries: sum per receiver side and per primitive before
-   * squaring (deferred mc_data semantics) */
-  const int n = pe.nent;
-  for(int e = 0; e < n; ++e) {
-    const int re = e == 0 ? pe.r0 : xr[e - 1];
-    bool seen = false;
-    for(int k = 0; k < e && !seen; ++k) seen = (k == 0 ? pe.r0 : xr[k - 1]) == re;
-    if(!seen) {
-      double v[6] = {0, 0, 0, 0, 0, 0};
-      for(int k = e; k < n; ++k) {
-        if((k == 0 ? pe.r0 : xr[k - 1]) != re) continue;
-        for(int q = 0; q < 6; ++q) v[q] += k == 0 ? v0[q] : xv[k - 1][q];
-      }
-      commit10<false>(rbase + (size_t)re * NRCV_Q * 2, v, f);
-      commit10<true>(T.samp_rcv + ((size_t)pe.samp * S.nrcv + re) * NRCV_Q * 2, v, f);
-    }
-    const int prim = e == 0 ? pe.p0 : xp[e - 1];
-    if(prim >= 0) {
-      /* (receiver side, primitive) keys are unique among the entries */
-      commit10<true>(T.prim + (size_t)prim * NRCV_Q * 2, e == 0 ? v0 : xv[e - 1], f);
     }
   }
-  return racc_slot;
+  __syncwarp();
 }
 
-/* commit_path_pe on a path state; two out-of-line levels, as measured
- * fastest (with the path end passed by value, 354 against 486 Mpaths/s) */
+/* The sums that follow from others, once a launch (block y: the item): a
+ * receiver side's from its samp_rcv slots, the global cosine and shadowed
+ * from the samp slots. Block x < nrcv: that receiver side; the last one: the
+ * globals. */
+constexpr int FINISH_LANES = 48; /* sampled instances in flight per quantity */
 template<class R>
-__device__ __noinline__ int commit_path
-  (const DScene<R>& S, const DTallies& T, const PathState<R>& p, int end, double* acc,
-   double* ps, int stride, double* smem_rcv, const int* xr, const int* xp,
-   const double (*xv)[6], double* racc, int racc_slot, const DControl* ctl)
+__global__ void __launch_bounds__(FINISH_LANES * NRCV_Q * 2) finish_tallies
+  (const DScene<R>* scenes, const DTallies* tallies, const DTallies one, int nrcv,
+   int nsampled)
 {
-  const PathEnd pe = path_end(p, end);
-  return commit_path_pe(S, T, pe, acc, ps, stride, smem_rcv, xr, xp, xv, racc, racc_slot, ctl);
+  __shared__ double part[FINISH_LANES][NRCV_Q * 2];
+  const DTallies& T = tallies ? tallies[blockIdx.y] : one;
+  if(scenes) { nrcv = scenes[blockIdx.y].nrcv; nsampled = scenes[blockIdx.y].nsampled; }
+  const int r = (int)blockIdx.x;
+  const int q = threadIdx.x % (NRCV_Q * 2), l = threadIdx.x / (NRCV_Q * 2);
+  const bool glob = r == (int)gridDim.x - 1;
+  if(!glob && r >= nrcv) return;
+  const double* src = glob ? T.samp + q : T.samp_rcv + (size_t)r * NRCV_Q * 2 + q;
+  const size_t step = glob ? 4 : (size_t)nrcv * NRCV_Q * 2;
+  double v = 0;
+  if(!glob || q < 4)
+#pragma unroll 4
+    for(int s = l; s < nsampled; s += FINISH_LANES) v += src[(size_t)s * step];
+  part[l][q] = v;
+  __syncthreads();
+  if(l) return;
+  v = 0;
+  for(int k = 0; k < FINISH_LANES; ++k) v += part[k][q];
+  if(!glob) T.rcv[(size_t)r * NRCV_Q * 2 + q] = v;
+  else if(q < 4) T.global[q < 2 ? 2 * G_COS + q : 2 * G_SHADOW + q - 2] = v;
 }
 
 /*******************************************************************************
@@ -1378,8 +1521,22 @@ __device__ __forceinline__ unsigned long long warp_sum_u64(unsigned long long v)
   return v;
 }
 
-constexpr int SMEM_RCV_MAX = 16;
 constexpr int MAX_BLOCK = 256;
+/* The paths of a warp advance together: its ended lanes wait until few are
+ * still under way, then commit at once and start the next realisations
+ * together. In the coherent order the lanes of a warp start on one heliostat,
+ * so their shadow rays, and then their reflected rays, are nearly parallel
+ * and visit the same nodes; refilling each lane as it ended (the former rule)
+ * mixed shadow and path rays in every cast. `few`: none for the first
+ * REGEN_AGE casts of meshes, 8 with quadrics or dielectrics, whose paths are
+ * longer and uneven; after REGEN_AGE casts at least REGEN_LATE, so that deep
+ * paths do not hold a warp. Field, 1e8 paths, lanes 32 (refill at once) / 16 /
+ * 8 / 2 / 0: 145 / 107 / 97.0 / 94.5 / 92.5 ms; beam-down, 6e7: 216 / 161 /
+ * 160 / 169 / 175 ms; a matte cavity, 1e7: 13.9 / 12.4 / 13.7 / 17.4 / 21.0,
+ * with 2 and then more after 3 casts 12.9. */
+constexpr int REGEN_AGE = 3, REGEN_LATE = 12;
+static int regen_lanes(int features)
+{ return features & (FEAT_QUADRIC | FEAT_DIELECTRIC) ? 8 : 0; }
 /* SMs per item group of the batched kernel's work order: small items
  * (fewer than BATCH_LARGE_ITEM realisations on average) by groups of 8 SMs,
  * larger ones by 16. Measured on 256 field items (Mpaths/s, groups of 8 /
@@ -1425,23 +1582,23 @@ realisation_kernel
    const uint4* sorted_draw, const uint32_t* sorted_off, uint32_t seg_mul,
    const DControl ctl)
 {
-  /* Shared memory: per-thread FP64 global sums [12][blockDim], per-thread
-   * path sums [10][blockDim], the receiver-side sums, the first traversal
-   * stack entries [8][blockDim]; shared memory left unused goes to the L1
-   * cache */
-  extern __shared__ double smem[];
-  __shared__ double red[MAX_BLOCK / 32][2 * NGLOBAL];
+  /* Shared memory: per-thread FP64 path sums [ps_count][blockDim], the
+   * warps' tally tiles [TILES][blockDim], the first traversal stack entries
+   * [SMEM_STACK][blockDim]; shared memory left unused goes to the L1 cache */
+  extern __shared__ double2 smem[];
+  __shared__ double red[MAX_BLOCK / 32][8];
+  __shared__ WarpKeys keys[MAX_BLOCK / 32];
+  __shared__ DTallies tallies;
   const int bd = blockDim.x, tid = threadIdx.x;
   const unsigned lane = tid & 31u;
-  const bool use_smem_rcv = S.nrcv <= SMEM_RCV_MAX;
-  double* acc = smem + tid;
-  double* ps = smem + 2 * NGLOBAL * bd + tid;
-  double* smem_rcv = use_smem_rcv ? smem + (2 * NGLOBAL + PS_COUNT) * bd : nullptr;
-  const int rcv_doubles = use_smem_rcv ? S.nrcv * NRCV_Q * 2 : 0;
-  int* stack = reinterpret_cast<int*>(smem + (2 * NGLOBAL + PS_COUNT) * bd
-                                      + rcv_doubles) + tid;
-  for(int q = 0; q < 2 * NGLOBAL; ++q) acc[q * bd] = 0;
-  for(int i = tid; i < rcv_doubles; i += bd) smem_rcv[i] = 0;
+  double2* tile = smem + tid;
+  double* ps = reinterpret_cast<double*>(smem + TILES * bd) + tid;
+  int* stack = reinterpret_cast<int*>(reinterpret_cast<double*>(smem + TILES * bd)
+                                      + ps_count(FEAT) * bd) + tid;
+  WarpKeys* wk = keys + (tid >> 5);
+  for(int k = 0; k < TILES; ++k) tile[k * bd] = make_double2(0.0, 0.0);
+  if(lane == 0) *wk = {0, 0, -1, -1};
+  if(tid == 0) tallies = T;
   __syncthreads();
 
   Rng rng;
@@ -1454,8 +1611,6 @@ realisation_kernel
   uint32_t bounces = 0, npaths = 0;
   int xr[MAX_EXTRA], xp[MAX_EXTRA];
   double xv[MAX_EXTRA][6];
-  double racc[2 * NRCV_Q];
-  int racc_slot = -1;
 
   /* Coherent order: the warp's current segment [seg_cur, seg_end) of the
    * sorted realisations */
@@ -1463,10 +1618,21 @@ realisation_kernel
   const uint32_t nseg = (uint32_t)((count + SORT_SEG - 1) / SORT_SEG);
   const bool polled = ctl.stop || ctl.abort;
   uint32_t fetches = 0;
+  int age = 0; /* casts since the warp last took realisations */
 
   for(;;) {
-    /* Regeneration: idle lanes take the next realisations */
-    const unsigned need = __ballot_sync(0xffffffffu, p.phase == PH_NONE && !done);
+    /* The warp's paths advance together (regen_lanes) */
+    unsigned need = 0;
+    if(__popc(__ballot_sync(0xffffffffu, p.phase == PH_SHADOW || p.phase == PH_BOUNCE))
+       <= (age <= REGEN_AGE ? ctl.regen : max(ctl.regen, REGEN_LATE))) {
+      age = 0;
+      if(__any_sync(0xffffffffu, p.phase == PH_ENDED)) {
+        commit_warp(S.nrcv, &tallies, 0, p, p.phase == PH_ENDED, ps, bd, tile, wk, xr, xp, xv,
+                    &ctl);
+        if(p.phase == PH_ENDED) p.phase = PH_NONE;
+      }
+      need = __ballot_sync(0xffffffffu, p.phase == PH_NONE && !done);
+    }
     bool start = false;
     uint64_t off = 0;
     U32x4 r0;
@@ -1562,12 +1728,13 @@ realisation_kernel
         }
       }
     }
-    if(!__any_sync(0xffffffffu, p.phase != PH_NONE)) break;
+    if(!__any_sync(0xffffffffu, p.phase == PH_SHADOW || p.phase == PH_BOUNCE)) break;
+    ++age;
 
     /* One ray per active lane */
     Hit<R> h;
     bool found = false;
-    if(p.phase != PH_NONE) {
+    if(p.phase == PH_SHADOW || p.phase == PH_BOUNCE) {
       const bool shadow = p.phase == PH_SHADOW;
       SelfInfo self;
       self.gid = p.gid;
@@ -1651,21 +1818,18 @@ realisation_kernel
           : (end == END_FAIL || p.overflow) ? 3 : (p.nent > 0 ? 2 : 0);
         tr.path_nv[p.tslot] = (int32_t)p.tseq;
       }
-      racc_slot = commit_path(S, T, p, end, acc, ps, bd, smem_rcv, xr, xp, xv,
-                              racc, racc_slot, &ctl);
-      p.phase = PH_NONE;
+      p.end = end;
+      p.phase = PH_ENDED;
     }
   }
 
-  if(racc_slot >= 0)
-    flush_racc((use_smem_rcv ? smem_rcv : T.rcv) + (size_t)racc_slot * NRCV_Q * 2, racc,
-               use_smem_rcv);
-
-  /* Warp then block reduction of the global sums, one commit per block */
+  /* The warps' tiles: the sampled instance's, then the global sums through a
+   * block reduction */
   const int warp = tid >> 5;
-  for(int q = 0; q < 2 * NGLOBAL; ++q) {
-    const double s = warp_sum(acc[q * bd]);
-    if(lane == 0) red[warp][q] = s;
+  flush_samp(&tallies, wk, tile, bd, false);
+  {
+    const double v = tile_row_sum(tile[0]);
+    if((lane & 3u) == 0u) red[warp][lane >> 2] = v;
   }
   unsigned long long c[6] = {cnt.rays, cnt.nodes, cnt.tris, cnt.quads,
                              bounces, npaths};
@@ -1675,12 +1839,11 @@ realisation_kernel
     for(int q = 0; q < 6; ++q) if(c[q]) atomicAdd(st + q, c[q]);
   }
   __syncthreads();
-  if(tid < 2 * NGLOBAL) {
+  if(tid < 8) {
     double v = 0;
     for(int w = 0; w < (bd >> 5); ++w) v += red[w][tid];
-    red_add_global(T.global + tid, v);
+    red_add_global(T.global + (tid < 2 ? 2 * G_ABS_RCV : 2 * G_MISSING - 2) + tid, v);
   }
-  for(int i = tid; i < rcv_doubles; i += bd) red_add_global(T.rcv + i, smem_rcv[i]);
 }
 
 /* Batched form: several scenes (e.g. one re-aimed field per sun position)
@@ -1697,36 +1860,28 @@ batch_kernel
    const unsigned long long* __restrict__ prefix,
    const unsigned long long* __restrict__ firsts, int nitems, uint64_t seed,
    unsigned long long max_segments, unsigned long long* next_items,
-   DStats* stats, int rcvd, const uint32_t* __restrict__ sorted_off,
+   DStats* stats, int regen, const uint32_t* __restrict__ sorted_off,
    const uint4* __restrict__ sorted_draw, const uint32_t* __restrict__ seg_mul)
 {
-  extern __shared__ double smem[];
+  extern __shared__ double2 smem[];
+  __shared__ WarpKeys keys[MAX_BLOCK / 32];
   const int bd = blockDim.x, tid = threadIdx.x;
   const unsigned lane = tid & 31u;
-  double* acc = smem + tid;
-  double* ps = smem + 2 * NGLOBAL * bd + tid;
-  int* stack = reinterpret_cast<int*>(smem + (2 * NGLOBAL + PS_COUNT) * bd) + tid;
-  for(int q = 0; q < 2 * NGLOBAL; ++q) acc[q * bd] = 0;
-  int acc_item = -1;
-  /* Global and receiver sums: every path adds to the same few addresses of
-   * its item, so they are gathered per warp in two shared-memory slots
-   * tagged with an item (the warp's current item and the previous one, for
-   * the paths still running across an item boundary) and flushed to the
-   * item's tallies when the warp moves on: one device atomic per warp and
-   * address for each item instead of one per thread. A slot holds the
-   * 2 x NGLOBAL global sums, then `rcvd` receiver sums. Tags change only
-   * where the warp is converged. */
-  const int ss = 2 * NGLOBAL + rcvd;
-  double* wslots = reinterpret_cast<double*>(
-    reinterpret_cast<int*>(smem + (2 * NGLOBAL + PS_COUNT) * bd) + SMEM_STACK * bd)
-    + (size_t)(tid >> 5) * 2 * ss;
-  for(int i = (int)lane; i < 2 * ss; i += 32) wslots[i] = 0;
-  /* Copies of the two tagged items' scene records, so that lanes on those
-   * items read their scene from shared memory instead of device memory */
+  double2* tile = smem + tid;
+  double* ps = reinterpret_cast<double*>(smem + TILES * bd) + tid;
+  int* stack = reinterpret_cast<int*>(reinterpret_cast<double*>(smem + TILES * bd)
+                                      + ps_count(FEAT) * bd) + tid;
+  WarpKeys* wk = keys + (tid >> 5);
+  for(int k = 0; k < TILES; ++k) tile[k * bd] = make_double2(0.0, 0.0);
+  if(lane == 0) *wk = {-1, -1, -1, -1};
+  /* Two slots per warp tagged with an item (its current item and the
+   * previous one, for the paths still running across an item boundary) hold
+   * copies of the items' scene records, so that lanes on those items read
+   * their scene from shared memory instead of device memory. Tags change
+   * only where the warp is converged. */
   DScene<R>* wscene = reinterpret_cast<DScene<R>*>(
-    reinterpret_cast<double*>(reinterpret_cast<int*>(smem + (2 * NGLOBAL + PS_COUNT) * bd)
-                              + SMEM_STACK * bd) + (size_t)(bd >> 5) * 2 * ss)
-    + (size_t)(tid >> 5) * 2;
+    reinterpret_cast<int*>(reinterpret_cast<double*>(smem + TILES * bd) + ps_count(FEAT) * bd)
+    + SMEM_STACK * bd) + (size_t)(tid >> 5) * 2;
   __syncwarp();
   int stag[2] = {-1, -1};
   int cur = 0;
@@ -1770,22 +1925,21 @@ batch_kernel
   uint32_t bounces = 0, npaths = 0;
   int xr[MAX_EXTRA], xp[MAX_EXTRA];
   double xv[MAX_EXTRA][6];
-  /* Running sums of one (item, receiver side), as in realisation_kernel;
-   * flushed into the item's warp slot (or its tallies) when either changes */
-  double racc[2 * NRCV_Q];
-  int racc_slot = -1, racc_item = -1;
-  auto racc_flush = [&]() {
-    if(racc_slot < 0) return;
-    const bool in_slot = rcvd && (racc_item == stag[cur] || racc_item == stag[cur ^ 1]);
-    double* dst = rcvd && racc_item == stag[cur] ? wslots + cur * ss + 2 * NGLOBAL
-      : rcvd && racc_item == stag[cur ^ 1] ? wslots + (cur ^ 1) * ss + 2 * NGLOBAL
-      : tallies[racc_item].rcv;
-    flush_racc(dst + (size_t)racc_slot * NRCV_Q * 2, racc, in_slot);
-    racc_slot = -1;
-  };
+  int age = 0; /* casts since the warp last took realisations */
 
   for(;;) {
-    const unsigned need = __ballot_sync(0xffffffffu, p.phase == PH_NONE && !done);
+    /* The warp's paths advance together (regen_lanes) */
+    unsigned need = 0;
+    if(__popc(__ballot_sync(0xffffffffu, p.phase == PH_SHADOW || p.phase == PH_BOUNCE))
+       <= (age <= REGEN_AGE ? regen : max(regen, REGEN_LATE))) {
+      age = 0;
+      if(__any_sync(0xffffffffu, p.phase == PH_ENDED)) {
+        commit_warp(scene_of(it).nrcv, tallies, it, p, p.phase == PH_ENDED, ps, bd, tile, wk,
+                    xr, xp, xv, (const DControl*)nullptr);
+        if(p.phase == PH_ENDED) p.phase = PH_NONE;
+      }
+      need = __ballot_sync(0xffffffffu, p.phase == PH_NONE && !done);
+    }
     if(need) {
       const int leader = __ffs(need) - 1;
       unsigned long long base = 0;
@@ -1817,21 +1971,6 @@ batch_kernel
         } else if(g < prefix[item + 1] - prefix[item]) {
           /* lanes past the item's end take work at the next fetch */
           it = item;
-          if(it != acc_item) {
-            if(acc_item >= 0) {
-              double* sl = acc_item == stag[cur] ? wslots + cur * ss
-                : acc_item == stag[cur ^ 1] ? wslots + (cur ^ 1) * ss : nullptr;
-              for(int q = 0; q < 2 * NGLOBAL; ++q) {
-                const double v = acc[q * bd];
-                if(v != 0.0) {
-                  if(sl) atomicAdd(sl + q, v);
-                  else red_add(tallies[acc_item].global + q, v);
-                }
-                acc[q * bd] = 0;
-              }
-            }
-            acc_item = it;
-          }
           /* Coherent order: the item's full warp segments of SORT_SEG
            * sorted realisations in a strided order (so that the warps of an
            * item group spread over its primitives), the ragged last one
@@ -1863,18 +2002,8 @@ batch_kernel
         const int newest = got ? wit : -1;
         if(newest >= 0 && newest != stag[cur]) {
           const int prv = cur ^ 1;
-          double* sl = wslots + prv * ss;
+          /* every lane's reads of the slot's old scene are done */
           __syncwarp();
-          if(stag[prv] >= 0) {
-            if((int)lane < 2 * NGLOBAL) red_add(tallies[stag[prv]].global + lane, sl[lane]);
-            double* dst = tallies[stag[prv]].rcv;
-            const int nd = rcvd ? scenes[stag[prv]].nrcv * NRCV_Q * 2 : 0;
-            for(int i = (int)lane; i < nd; i += 32) red_add(dst + i, sl[2 * NGLOBAL + i]);
-          }
-          /* The lanes clear other entries than they flushed: every read of
-           * the slot before any clear */
-          __syncwarp();
-          for(int i = (int)lane; i < ss; i += 32) sl[i] = 0;
           {
             const int* src = reinterpret_cast<const int*>(scenes + newest);
             int* dst = reinterpret_cast<int*>(wscene + prv);
@@ -1887,12 +2016,13 @@ batch_kernel
         }
       }
     }
-    if(!__any_sync(0xffffffffu, p.phase != PH_NONE)) break;
+    if(!__any_sync(0xffffffffu, p.phase == PH_SHADOW || p.phase == PH_BOUNCE)) break;
+    ++age;
 
     const DScene<R>& S = scene_of(it);
     Hit<R> h;
     bool found = false;
-    if(p.phase != PH_NONE) {
+    if(p.phase == PH_SHADOW || p.phase == PH_BOUNCE) {
       const bool shadow = p.phase == PH_SHADOW;
       SelfInfo self;
       self.gid = p.gid;
@@ -1959,40 +2089,13 @@ batch_kernel
     if(do_interact)
       end = interact<R, FEAT>(S, rng, p, pos, dir, bounces, max_segments, ps, bd, xr, xp, xv);
     if(end != END_NONE) {
-      double* rb = nullptr;
-      if(rcvd) {
-        if(it == stag[cur]) rb = wslots + cur * ss + 2 * NGLOBAL;
-        else if(it == stag[cur ^ 1]) rb = wslots + (cur ^ 1) * ss + 2 * NGLOBAL;
-      }
-      if(racc_item != it) racc_flush();
-      racc_item = it;
-      racc_slot = commit_path(S, tallies[it], p, end, acc, ps, bd, rb, xr, xp, xv,
-                              racc, racc_slot, (const DControl*)nullptr);
-      p.phase = PH_NONE;
+      p.end = end;
+      p.phase = PH_ENDED;
     }
   }
 
-  racc_flush();
-  if(acc_item >= 0) {
-    double* sl = acc_item == stag[cur] ? wslots + cur * ss
-      : acc_item == stag[cur ^ 1] ? wslots + (cur ^ 1) * ss : nullptr;
-    for(int q = 0; q < 2 * NGLOBAL; ++q) {
-      const double v = acc[q * bd];
-      if(v == 0.0) continue;
-      if(sl) atomicAdd(sl + q, v);
-      else red_add(tallies[acc_item].global + q, v);
-    }
-  }
-  __syncwarp();
-  for(int k = 0; k < 2; ++k) {
-    if(stag[k] < 0) continue;
-    if((int)lane < 2 * NGLOBAL)
-      red_add(tallies[stag[k]].global + lane, wslots[k * ss + lane]);
-    double* dst = tallies[stag[k]].rcv;
-    const int nd = rcvd ? scenes[stag[k]].nrcv * NRCV_Q * 2 : 0;
-    for(int i = (int)lane; i < nd; i += 32)
-      red_add(dst + i, wslots[k * ss + 2 * NGLOBAL + i]);
-  }
+  flush_samp(tallies, wk, tile, bd, false);
+  flush_global(tallies, wk, tile);
   unsigned long long c[6] = {cnt.rays, cnt.nodes, cnt.tris, cnt.quads,
                              bounces, npaths};
   for(int q = 0; q < 6; ++q) c[q] = warp_sum_u64(c[q]);
@@ -2213,6 +2316,14 @@ static void raise_smem_limit(K kernel, int dev)
 template<class R, int MINB, bool TRACK, int FEAT> struct RealisationTag {};
 template<class R, int MINB, int FEAT> struct BatchTag {};
 
+/* Shared memory of a block of the realisation kernels: tally tiles, path
+ * sums, traversal stack */
+static size_t path_smem(int feat, int block)
+{
+  return (size_t)block * (TILES * sizeof(double2) + ps_count(feat) * sizeof(double)
+                          + SMEM_STACK * sizeof(int));
+}
+
 template<class R, int MINB, bool TRACK, int FEAT>
 static int launch_variant
   (const DScene<R>& S, const DTallies& T, uint64_t seed, uint64_t first,
@@ -2224,10 +2335,7 @@ static int launch_variant
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   const int block = cfg.block_size > 0 ? cfg.block_size : MAX_BLOCK;
   if(block > MAX_BLOCK || block % 32) return (int)cudaErrorInvalidValue;
-  const int rcv_doubles = S.nrcv <= SMEM_RCV_MAX ? S.nrcv * NRCV_Q * 2 : 0;
-  const size_t smem = (size_t)((2 * NGLOBAL + PS_COUNT) * block + rcv_doubles)
-                      * sizeof(double)
-                    + (size_t)SMEM_STACK * block * sizeof(int);
+  const size_t smem = path_smem(FEAT, block);
   raise_smem_limit<RealisationTag<R, MINB, TRACK, FEAT>>(realisation_kernel<R, MINB, TRACK, FEAT>, dev);
   int per_sm = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor
@@ -2246,12 +2354,15 @@ static int launch_variant
   ctl.max_failed = cfg.max_failed;
   ctl.stop = cfg.max_failed != ~0ull ? T.counters + 4 : nullptr;
   ctl.abort = cfg.abortable ? T.counters + 5 : nullptr;
+  ctl.regen = regen_lanes(cfg.features);
   if(!sort) {
     /* Work counter of this launch: counters[3] */
     cudaMemsetAsync(T.counters + 3, 0, sizeof(unsigned long long), st);
     realisation_kernel<R, MINB, TRACK, FEAT><<<(unsigned)blocks, block, smem, st>>>
       (S, T, seed, first, count, cfg.max_segments, T.counters + 3, tr, nullptr,
        nullptr, 1u, ctl);
+    finish_tallies<R><<<S.nrcv + 1, FINISH_LANES * NRCV_Q * 2, 0, st>>>
+      (nullptr, nullptr, T, S.nrcv, S.nsampled);
     return (int)cudaGetLastError();
   }
   const uint64_t chunk = count < SORT_CHUNK ? count : SORT_CHUNK;
@@ -2289,6 +2400,8 @@ static int launch_variant
       (S, T, seed, first + c0, n, cfg.max_segments, T.counters + 3, tr, sdraws, soff,
        mul, ctl);
   }
+  finish_tallies<R><<<S.nrcv + 1, FINISH_LANES * NRCV_Q * 2, 0, st>>>
+    (nullptr, nullptr, T, S.nrcv, S.nsampled);
   cudaFreeAsync(buf, st);
   return (int)cudaGetLastError();
 }
@@ -2330,6 +2443,17 @@ static int launch_impl
   }
 }
 
+template<class R>
+static void finish_batch(const DScene<R>* scenes, const DTallies* tallies, int nitems,
+                         int max_nrcv, cudaStream_t st)
+{
+  const DTallies none = {};
+  for(int i = 0; i < nitems; i += 65535)
+    finish_tallies<R><<<dim3((unsigned)max_nrcv + 1, (unsigned)std::min(nitems - i, 65535)),
+                        FINISH_LANES * NRCV_Q * 2, 0, st>>>
+      (scenes + i, tallies + i, none, 0, 0);
+}
+
 template<class R, int MINB, int FEAT>
 static int launch_batch_variant(const BatchLaunch<R>& b, const LaunchConfig& cfg,
                                 void* stream)
@@ -2340,10 +2464,7 @@ static int launch_batch_variant(const BatchLaunch<R>& b, const LaunchConfig& cfg
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   const int block = cfg.block_size > 0 ? cfg.block_size : MAX_BLOCK;
   if(block > MAX_BLOCK || block % 32) return (int)cudaErrorInvalidValue;
-  const size_t smem = (size_t)((2 * NGLOBAL + PS_COUNT) * block) * sizeof(double)
-                    + (size_t)SMEM_STACK * block * sizeof(int)
-                    + (size_t)(block / 32) * 2 * (2 * NGLOBAL + cfg.rcv_doubles) * sizeof(double)
-                    + (size_t)(block / 32) * 2 * sizeof(DScene<R>);
+  const size_t smem = path_smem(FEAT, block) + (size_t)(block / 32) * 2 * sizeof(DScene<R>);
   raise_smem_limit<BatchTag<R, MINB, FEAT>>(batch_kernel<R, MINB, FEAT>, dev);
   int per_sm = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor
@@ -2367,8 +2488,9 @@ static int launch_batch_variant(const BatchLaunch<R>& b, const LaunchConfig& cfg
   cudaMemsetAsync(b.next_items, 0, (size_t)b.nitems * sizeof(unsigned long long), st);
   batch_kernel<R, MINB, FEAT><<<(unsigned)blocks, block, smem, st>>>
     (b.scenes, b.tallies, b.prefix, b.firsts, b.nitems, b.seed, cfg.max_segments,
-     b.next_items, b.stats, cfg.rcv_doubles, o.sorted_off,
+     b.next_items, b.stats, regen_lanes(cfg.features), o.sorted_off,
      reinterpret_cast<const uint4*>(o.sorted_draw), o.seg_mul);
+  finish_batch<R>(b.scenes, b.tallies, b.nitems, cfg.max_nrcv, st);
   return (int)cudaGetLastError();
 }
 

@@ -1893,8 +1893,7 @@ extern "C" res_T ssol_b200_batch_reset(ssol_b200_batch* b, void* stream)
 
 /* The captured graph: work-counter reset + the persistent batch kernel. Its
  * parameters are device pointers only, so one capture serves every launch */
-/* Launch shape of a batch; receiver sums are gathered per warp in shared
- * memory when two slots of the largest item fit in 16 KB per block */
+/* Launch shape of a batch */
 static LaunchConfig batch_config(const ssol_b200_batch* b)
 {
   LaunchConfig cfg;
@@ -1910,9 +1909,7 @@ static LaunchConfig batch_config(const ssol_b200_batch* b)
     nrcv = std::max(nrcv, m.rcv.size());
     cfg.features |= m.features;
   }
-  const size_t rcvd = nrcv * NRCV_Q * 2;
-  const size_t warps = (size_t)(cfg.block_size > 0 ? cfg.block_size : 256) / 32;
-  cfg.rcv_doubles = warps * 2 * rcvd * sizeof(double) <= 16 * 1024 ? (int)rcvd : 0;
+  cfg.max_nrcv = (int)nrcv;
   return cfg;
 }
 
