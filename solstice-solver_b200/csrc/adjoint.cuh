@@ -143,7 +143,7 @@ adjoint_kernel(const DScene<R> S, const AdjointArgs A, uint64_t seed, uint64_t f
     const V3<R> nproxy = ld3(st.n);
     const U32x4 r1 = rng.get(1u, RNG_PRIMARY);
     const V3<R> dir = sample_sun_dir(S, rng, r1);
-    const double wl = sample_wavelength(S, u01d(r1.v[2]));
+    const double wl = S.spectral ? sample_wavelength(S, u01d(r1.v[2])) : 0.0;
     V3<R> N = nproxy;
     if(si.is_punched) {
       const DQuadric<R>& Q = S.quads[si.quadric];

@@ -106,6 +106,12 @@ struct alignas(16) DMaterial {
   int32_t table; /* into shader_tab: (reflectivity, roughness) pairs */
   int32_t slab_medium; /* thin dielectric */
   double thickness;
+  /* Shader values that are the same at every wavelength node (bit 0 of
+   * `uniform`: reflectivity, bit 1: roughness), read with the record instead
+   * of searched in the table */
+  double value[2];
+  int32_t uniform;
+  int32_t pad[3];
 };
 
 /* Instance x shaded shape record: what a hit resolves to */
@@ -228,6 +234,9 @@ template<typename R> struct DScene {
   const R* shader_tab; /* per material: nodes x (reflectivity, roughness) */
   const double* shader_wl; /* sun spectrum wavelength nodes */
   int32_t shader_nodes;
+  /* Some material, medium or baked shader depends on the wavelength; the
+   * paths of a scene without any need not sample theirs */
+  int32_t spectral;
 
   const DSampTri<R>* samp;
   const float* alias_prob;

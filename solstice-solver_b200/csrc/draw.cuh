@@ -289,7 +289,8 @@ __device__ __noinline__ bool draw_radiance
   L = 0;
   double thr = 1;
   bool roulette = false;
-  const double wl = sample_wavelength(S, u01d(rng.get(attempt, RNG_DRAW_WL).v[0]));
+  const double wl = S.spectral
+    ? sample_wavelength(S, u01d(rng.get(attempt, RNG_DRAW_WL).v[0])) : 0.0;
   int medium = S.air_medium;
   SelfInfo self = {-1, -1, 0, true, false};
   const V3<R> up = mk((R)A.up[0], (R)A.up[1], (R)A.up[2]);

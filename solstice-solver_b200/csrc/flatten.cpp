@@ -585,6 +585,16 @@ static res_T flatten_impl
     d.thickness = m->thickness;
     d.table = (int32_t)out.shader_tab.size();
     if(!tabulate_shaders(out, m, dev)) bad_shader = true;
+    d.uniform = 0;
+    d.pad[0] = d.pad[1] = d.pad[2] = 0;
+    for(int q = 0; q < 2; ++q) {
+      const R* tab = out.shader_tab.data() + d.table + q;
+      const size_t n = out.shader_wl.size();
+      bool same = std::isfinite((double)tab[0]);
+      for(size_t k = 1; k < n && same; ++k) same = tab[2 * k] == tab[0];
+      d.value[q] = same ? (double)tab[0] : 0.0;
+      if(same) d.uniform |= 1 << q;
+    }
     const int id = (int)out.mtls.size();
     out.mtls.push_back(d);
     mtl_index.emplace(m, id);

@@ -440,6 +440,10 @@ static void bind_scene(DScene<R>& S, const FlatScene<R>& f, const Blob& b,
   S.bake_tab = (const R*)ptr();
   if(f.tshade.empty()) S.tshade = nullptr;
   S.shader_nodes = (int32_t)f.shader_wl.size();
+  S.spectral = !f.bake_tab.empty();
+  for(const DMaterial& m : f.mtls) S.spectral |= m.uniform != 3;
+  for(const DMedium& m : f.media)
+    S.spectral |= m.extinction.spectrum >= 0 || m.refractive_index.spectrum >= 0;
   S.nsamp = (int32_t)f.samp.size();
   S.sun_type = f.sun_type;
   for(int c = 0; c < 3; ++c) S.sun_dir[c] = f.sun_dir[c];
