@@ -107,11 +107,11 @@ __global__ void __launch_bounds__(256) draft_kernel(const DScene<R> S, const Dra
                     (int)blockDim.x))
         continue;
       const V3<R> wi = normalize(d);
-      V3<R> N = normalize(h.n);
+      V3<R> N = normalize_hit(h.n);
       if(!(dot(N, wi) < R(0))) N = -N;
       R b1, b2;
       N = draw_shading_normal(S, h.gid, o + d * h.t, wi, N, b1, b2);
-      const double c = (double)dot(N, -wi);
+      const double c = (double)dot_yx(N, -wi);
       sum += c > 0.0 ? c : 0.0;
     }
     const double v = sum / (double)A.spp;
@@ -197,7 +197,7 @@ __device__ __forceinline__ R draw_bsdf_sample
   const DMaterial& m = f.m;
   type = 0;
   next_medium = medium;
-  const R ci = dot(wo, N);
+  const R ci = dot_yx(wo, N);
   wi = N;
   if(!(ci > R(0))) return R(0);
   switch(m.type) {
@@ -214,7 +214,7 @@ __device__ __forceinline__ R draw_bsdf_sample
       const R st = sq_rt(tan2) * ct;
       R sp, cp; sincos2pi(uni<R>(r.v[1]), &sp, &cp);
       const V3<R> h = local_to(N, cp * st, sp * st, ct);
-      const R oh = dot(wo, h);
+      const R oh = dot_yx(wo, h);
       wi = h * (R(2) * oh) - wo;
       const R ni = dot(wi, N);
       if(!(oh > R(0)) || !(ni > R(0))) return R(0);
@@ -306,8 +306,8 @@ __device__ __noinline__ bool draw_radiance
       thr *= exp(-kext * (double)h.t);
       if(thr <= 0) break;
     }
-    const V3<R> wo_in = normalize(dir);
-    V3<R> Ng = normalize(h.n);
+    const V3<R> wo_in = normalize_hit(dir);
+    V3<R> Ng = normalize_hit(h.n);
     int side = 1;
     if(!(dot(Ng, wo_in) < R(0))) { side = 2; Ng = -Ng; }
     const V3<R> pos = org + dir * h.t;
@@ -348,7 +348,7 @@ __device__ __noinline__ bool draw_radiance
       w = R(0);
     dir = wi;
     if(type & BXDF_TRANSMISSION) medium = next_medium;
-    const double cn = fabs((double)dot(wi, N));
+    const double cn = fabs((double)dot_yx(wi, N));
     if(!roulette) {
       thr *= cn * (double)w;
     } else {

@@ -19,8 +19,8 @@ struct LaunchConfig {
   unsigned long long max_segments; /* per path segment budget */
   int min_blocks; /* register budget: 1 (255 regs), 2 (128) or 3 (85) */
   int max_nrcv = 0; /* batched launches: the most receiver sides of an item */
-  bool coherent = true; /* plain launches of at least 2^24 realisations run
-                         * in the order of their sampled primitives */
+  bool coherent = true; /* larger plain launches run in the order of their
+                         * sampled primitives */
   /* Plain launches: stop handing out realisations once this many paths
    * have failed (~0: never), or once the host sets the tallies' abort word
    * (when `abortable`) */
@@ -60,15 +60,13 @@ int launch_realisations_nocount_f32
 constexpr uint32_t SORT_SEGMENT = 256;
 
 /* Coherent order of a batched launch (sorted_off null: id order). Per item,
- * from prefix[item] on, sorted_off / sorted_draw hold its realisations'
- * offsets in the item and primary draws (4 words each) in the order of their
- * sampled primitive; seg_mul[item] is the stride of the order in which its
+ * from prefix[item] on, sorted_off holds its realisations' offsets in the item
+ * in the order of their sampled primitive; seg_mul[item] is the stride of the order in which its
  * warp segments are handed out (coprime with its number of full segments);
  * bin_base[item] is its first histogram bin, nbins the bins of all items.
  * hist and bin_off are the presort's histogram and ranges (nbins each). */
 struct BatchOrder {
   uint32_t* sorted_off = nullptr;
-  uint32_t* sorted_draw = nullptr;
   uint32_t* hist = nullptr;
   uint32_t* bin_off = nullptr;
   const uint32_t* bin_base = nullptr;

@@ -99,7 +99,7 @@ static int launch_batch_noalloc_variant
     (scenes, tallies, scratch + NOALLOC_PREFIX, scratch + NOALLOC_FIRSTS, nitems,
      seed, cfg.max_segments, scratch + NOALLOC_NEXT,
      reinterpret_cast<DStats*>(scratch + NOALLOC_STATS), regen_lanes(cfg.features),
-     nullptr, nullptr, nullptr); /* id order: the coherent order needs scratch */
+     nullptr, nullptr); /* id order: the coherent order needs scratch */
   finish_batch<R>(scenes, tallies, nitems, cfg.max_nrcv, s);
   return (int)cudaGetLastError();
 }

@@ -63,10 +63,22 @@ template<class R> __device__ __forceinline__ V3<R> operator-(V3<R> a)
 { return mk(-a.x, -a.y, -a.z); }
 template<class R> __device__ __forceinline__ V3<R> operator*(V3<R> a, R s)
 { return mk(a.x * s, a.y * s, a.z * s); }
+/* Products rounded on their own. The sums below spell out which product is
+ * fused into each addition: left to the compiler, the choice depends on the
+ * code around, and the kernel variants and launch orders would round the same
+ * path differently */
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+/* a0 b0 + a1 b1 + a2 b2 */
+template<class R> __device__ __forceinline__ R sum3(R a0, R b0, R a1, R b1, R a2, R b2)
+{ return fma(a2, b2, fma(a0, b0, mul_rn(a1, b1))); }
 template<class R> __device__ __forceinline__ R dot(V3<R> a, V3<R> b)
-{ return a.x * b.x + a.y * b.y + a.z * b.z; }
+{ return sum3(a.x, b.x, a.y, b.y, a.z, b.z); }
 template<class R> __device__ __forceinline__ V3<R> cross(V3<R> a, V3<R> b)
-{ return mk(a.y*b.z - a.z*b.y, a.z*b.x - a.x*b.z, a.x*b.y - a.y*b.x); }
+{
+  return mk(fma(a.y, b.z, -mul_rn(a.z, b.y)), fma(a.z, b.x, -mul_rn(a.x, b.z)),
+            fma(a.x, b.y, -mul_rn(a.y, b.x)));
+}
 
 __device__ __forceinline__ float rsq(float x) { return rsqrtf(x); }
 __device__ __forceinline__ double rsq(double x) { return rsqrt(x); }
@@ -91,6 +103,16 @@ __device__ __forceinline__ double sn(double x) { return sin(x); }
 
 template<class R> __device__ __forceinline__ V3<R> normalize(V3<R> v)
 { const R len = sq_rt(dot(v, v)); return len > R(0) ? v * (R(1) / len) : v; }
+
+/* A dot product and a normalisation with the first two products in the other
+ * order, where the code has always rounded so */
+template<class R> __device__ __forceinline__ R dot_yx(V3<R> a, V3<R> b)
+{ return sum3(a.y, b.y, a.x, b.x, a.z, b.z); }
+template<class R> __device__ __forceinline__ V3<R> normalize_hit(V3<R> v)
+{
+  const R len = sq_rt(dot_yx(v, v));
+  return len > R(0) ? v * (R(1) / len) : v;
+}
 
 template<class R> __device__ __forceinline__ R uni(uint32_t x);
 template<> __device__ __forceinline__ float uni<float>(uint32_t x)
@@ -206,9 +228,9 @@ template<class R>
 __device__ __forceinline__ V3<R> sun_local_to_world(const DScene<R>& S, V3<R> p)
 {
   const R* B = S.sun_basis;
-  return normalize(mk(B[0] * p.x + B[3] * p.y + B[6] * p.z,
-                      B[1] * p.x + B[4] * p.y + B[7] * p.z,
-                      B[2] * p.x + B[5] * p.y + B[8] * p.z));
+  return normalize(mk(sum3(B[0], p.x, B[3], p.y, B[6], p.z),
+                      sum3(B[1], p.x, B[4], p.y, B[7], p.z),
+                      sum3(B[2], p.x, B[5], p.y, B[8], p.z)));
 }
 
 /* Buie zenith angle by rejection (src/ssol_ranst_sun_dir.c:177-195); the
@@ -298,24 +320,22 @@ __device__ double sample_wavelength(const DScene<R>& S, double u)
 template<class R>
 __device__ __forceinline__ V3<R> xform_point(const R* M, V3<R> p)
 {
-  return mk(M[0] * p.x + M[1] * p.y + M[2] * p.z + M[3],
-            M[4] * p.x + M[5] * p.y + M[6] * p.z + M[7],
-            M[8] * p.x + M[9] * p.y + M[10] * p.z + M[11]);
+  return mk(sum3(M[0], p.x, M[1], p.y, M[2], p.z) + M[3],
+            sum3(M[4], p.x, M[5], p.y, M[6], p.z) + M[7],
+            sum3(M[8], p.x, M[9], p.y, M[10], p.z) + M[11]);
 }
 template<class R>
 __device__ __forceinline__ V3<R> xform_vec(const R* M, V3<R> v)
 {
-  return mk(M[0] * v.x + M[1] * v.y + M[2] * v.z,
-            M[4] * v.x + M[5] * v.y + M[6] * v.z,
-            M[8] * v.x + M[9] * v.y + M[10] * v.z);
+  return mk(sum3(M[0], v.x, M[1], v.y, M[2], v.z), sum3(M[4], v.x, M[5], v.y, M[6], v.z),
+            sum3(M[8], v.x, M[9], v.y, M[10], v.z));
 }
 /* Normal to world: transpose of the world->local linear part */
 template<class R>
 __device__ __forceinline__ V3<R> xform_normal(const R* W, V3<R> n)
 {
-  return mk(W[0] * n.x + W[4] * n.y + W[8] * n.z,
-            W[1] * n.x + W[5] * n.y + W[9] * n.z,
-            W[2] * n.x + W[6] * n.y + W[10] * n.z);
+  return mk(sum3(W[0], n.x, W[4], n.y, W[8], n.z), sum3(W[1], n.x, W[5], n.y, W[9], n.z),
+            sum3(W[2], n.x, W[6], n.y, W[10], n.z));
 }
 
 /* Front normal (local frame, unnormalised) at pl of the general form in
@@ -439,11 +459,9 @@ __device__ __forceinline__ bool side_passes
   return true;
 }
 
-/* Products and differences rounded on their own (no FMA contraction): the
+/* Differences rounded on their own (no FMA contraction): with mul_rn, the
  * edge functions of the watertight test must be exact negations on an edge
  * shared by two triangles */
-__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
-__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ float sub_rn(float a, float b) { return __fsub_rn(a, b); }
 __device__ __forceinline__ double sub_rn(double a, double b) { return __dsub_rn(a, b); }
 
@@ -790,7 +808,8 @@ __device__ __forceinline__ V3<R> local_to(V3<R> n, R x, R y, R z)
 {
   V3<R> b1, b2;
   onb(n, b1, b2);
-  return b1 * x + b2 * y + n * z;
+  return mk(sum3(b1.x, x, b2.x, y, n.x, z), sum3(b1.y, x, b2.y, y, n.y, z),
+            sum3(b1.z, x, b2.z, y, n.z, z));
 }
 
 /* One BSDF sample: the propagated fraction, the outgoing direction, the
@@ -1034,14 +1053,12 @@ __device__ __forceinline__ int sample_prim(const DScene<R>& S, const U32x4& r0)
   return k;
 }
 
-/* point_init (src/ssol_solver.c:207-352) up to the shadow ray; `draw` is the
- * realisation's primary draw when the caller already has it */
+/* point_init (src/ssol_solver.c:207-352) up to the shadow ray */
 template<class R, int FEAT = FEAT_ALL>
 __device__ __forceinline__ void init_path
-  (const DScene<R>& S, const Rng& rng, PathState<R>& p, double* ps, int stride,
-   const U32x4* draw = nullptr)
+  (const DScene<R>& S, const Rng& rng, PathState<R>& p, double* ps, int stride)
 {
-  const U32x4 r0 = draw ? *draw : rng.get(0u, RNG_PRIMARY);
+  const U32x4 r0 = rng.get(0u, RNG_PRIMARY);
   const int k = sample_prim(S, r0);
   const DSampTri<R> st = S.samp[k];
   const R sa = sq_rt(uni<R>(r0.v[2]));
@@ -1555,11 +1572,22 @@ constexpr unsigned long long BATCH_LARGE_ITEM = 400000;
 /* Coherent order (see presort_count) */
 constexpr int SORT_MAX_BINS = 12288; /* shared-memory histogram of primitives */
 constexpr uint64_t SORT_CHUNK = 1ull << 24; /* realisations per sorted chunk */
-/* Smaller launches keep the id order: there the warps get few segments each
- * (the last ones leave lanes idle) and the presort does not pay. On the field
- * (Mpaths/s, sorted against id order): 1e6 paths 596 / 597, 4e6 615 / 632,
- * 8e6 652 / 637, 1.6e7 675 / 640 */
-constexpr uint64_t SORT_MIN = 6000000;
+/* Smaller launches keep the id order: there the presort (25 to 50 us) costs
+ * more than it gives. us a launch, id order / sorted: field of 1000, 1e5
+ * paths 172 / 179, 3e5 389 / 348, 1e6 1088 / 897, 7e6 7036 / 5549; field of
+ * 30, 3e5 565 / 377; beam-down of 1000, 3e5 847 / 948, 1e6 2658 / 2650, 3e6
+ * 7914 / 7262. A single sampled instance has its lanes on one surface already:
+ * one mirror, 1e6, 349 / 377; a dish of 128 triangles, 1e6, 583 / 588, of
+ * 2048, 1041 / 958. */
+constexpr uint64_t SORT_MIN = 200000, SORT_MIN_QUADRIC = 1000000;
+constexpr int SORT_SINGLE = 1024;
+/* Launches that are being captured, whose scratch the graph would hold, sort
+ * from here on only */
+constexpr uint64_t SORT_MIN_CAPTURED = 6000000;
+/* Segments a warp gets on average before they shrink from SORT_SEG to 32
+ * realisations: with 1 / 2 / 4 / 8 the field's 1e6 paths take 1180 / 1007 /
+ * 931 / 899 us, as the last segments leave fewer warps waiting */
+constexpr uint64_t SORT_SHARE = 8;
 constexpr uint32_t SORT_SEG = SORT_SEGMENT; /* sorted realisations per warp segment */
 
 /* Append one vertex of a tracked path (src/ssol_solver.c:909-922, 1014-1019,
@@ -1588,7 +1616,7 @@ realisation_kernel
   (const DScene<R> S, const DTallies T,
    uint64_t seed, uint64_t first, uint64_t count, unsigned long long max_segments,
    unsigned long long* next_path, const DTrack tr,
-   const uint4* sorted_draw, const uint32_t* sorted_off, uint32_t seg_mul,
+   const uint32_t* sorted_off, uint32_t seg_len, uint32_t seg_mul,
    const DControl ctl)
 {
   /* Shared memory: per-thread FP64 path sums [ps_count][blockDim], the
@@ -1624,7 +1652,7 @@ realisation_kernel
   /* Coherent order: the warp's current segment [seg_cur, seg_end) of the
    * sorted realisations */
   uint32_t seg_cur = 0, seg_end = 0;
-  const uint32_t nseg = (uint32_t)((count + SORT_SEG - 1) / SORT_SEG);
+  const uint32_t nseg = sorted_off ? (uint32_t)((count + seg_len - 1) / seg_len) : 0u;
   const bool polled = ctl.stop || ctl.abort;
   uint32_t fetches = 0;
   int age = 0; /* casts since the warp last took realisations */
@@ -1644,7 +1672,6 @@ realisation_kernel
     }
     bool start = false;
     uint64_t off = 0;
-    U32x4 r0;
     /* Early stop: every 8th fetch of the warp reads the stop and abort
      * words (one L2 sector); a halted warp takes no new realisation and ends
      * once its paths in flight end */
@@ -1676,8 +1703,8 @@ realisation_kernel
         if((int)lane == leader) sg = atomicAdd(next_path, 1ull);
         sg = __shfl_sync(0xffffffffu, sg, leader);
         if(sg < nseg) {
-          const uint32_t s0 = (uint32_t)((sg * seg_mul) % nseg) * SORT_SEG;
-          const uint32_t s1 = (uint32_t)min((uint64_t)s0 + SORT_SEG, count);
+          const uint32_t s0 = (uint32_t)((sg * seg_mul) % nseg) * seg_len;
+          const uint32_t s1 = (uint32_t)min((uint64_t)s0 + seg_len, count);
           if(!got && rank - avail < s1 - s0) {
             idx = s0 + (rank - avail);
             got = true;
@@ -1694,10 +1721,8 @@ realisation_kernel
       if(p.phase == PH_NONE && !done) {
         if(got) {
           start = true;
-          /* read once: streaming loads, evicted from L2 first */
+          /* read once: a streaming load, evicted from L2 first */
           off = __ldcs(&sorted_off[idx]);
-          const uint4 d = __ldcs(&sorted_draw[idx]);
-          r0 = {{d.x, d.y, d.z, d.w}};
         } else if(exhausted) {
           done = true;
         }
@@ -1724,8 +1749,7 @@ realisation_kernel
       const uint64_t id = first + off;
       rng.i_lo = (uint32_t)id;
       rng.i_hi = (uint32_t)(id >> 32);
-      if(!sorted_off) r0 = rng.get(0u, RNG_PRIMARY);
-      init_path<R, FEAT>(S, rng, p, ps, bd, &r0);
+      init_path<R, FEAT>(S, rng, p, ps, bd);
       ++npaths;
       if(TRACK) {
         p.tslot = off < tr.npaths ? (int)off : -1;
@@ -1801,7 +1825,7 @@ realisation_kernel
           p.prim = h.prim;
           p.gid = h.gid;
           dir = p.rd;
-          p.N = normalize(h.n);
+          p.N = normalize_hit(h.n);
           pos = p.org + p.rd * h.t;
           if((FEAT & FEAT_ATTRIBUTES) && S.tshade && h.gid >= 0) {
             const float2 uv = tri_uv(S, h.gid, pos);
@@ -1870,7 +1894,7 @@ batch_kernel
    const unsigned long long* __restrict__ firsts, int nitems, uint64_t seed,
    unsigned long long max_segments, unsigned long long* next_items,
    DStats* stats, int regen, const uint32_t* __restrict__ sorted_off,
-   const uint4* __restrict__ sorted_draw, const uint32_t* __restrict__ seg_mul)
+   const uint32_t* __restrict__ seg_mul)
 {
   extern __shared__ double2 smem[];
   __shared__ WarpKeys keys[MAX_BLOCK / 32];
@@ -1985,7 +2009,6 @@ batch_kernel
            * item group spread over its primitives), the ragged last one
            * last; each record gives the realisation and its primary draw */
           uint64_t off = g;
-          U32x4 r0;
           if(sorted_off) {
             const unsigned long long nfull = (prefix[it + 1] - prefix[it]) / SORT_SEG;
             unsigned long long sg = g / SORT_SEG;
@@ -1995,14 +2018,11 @@ batch_kernel
                 : sg * seg_mul[it] % nfull;
             const unsigned long long rec = prefix[it] + sg * SORT_SEG + g % SORT_SEG;
             off = __ldcs(&sorted_off[rec]);
-            const uint4 d = __ldcs(&sorted_draw[rec]);
-            r0 = {{d.x, d.y, d.z, d.w}};
           }
           const uint64_t id = firsts[it] + off;
           rng.i_lo = (uint32_t)id;
           rng.i_hi = (uint32_t)(id >> 32);
-          if(!sorted_off) r0 = rng.get(0u, RNG_PRIMARY);
-          init_path<R, FEAT>(scene_of(it), rng, p, ps, bd, &r0);
+          init_path<R, FEAT>(scene_of(it), rng, p, ps, bd);
           ++npaths;
         }
       }
@@ -2081,7 +2101,7 @@ batch_kernel
           p.prim = h.prim;
           p.gid = h.gid;
           dir = p.rd;
-          p.N = normalize(h.n);
+          p.N = normalize_hit(h.n);
           pos = p.org + p.rd * h.t;
           if((FEAT & FEAT_ATTRIBUTES) && S.tshade && h.gid >= 0) {
             const float2 uv = tri_uv(S, h.gid, pos);
@@ -2120,18 +2140,32 @@ batch_kernel
  * lanes of a warp start on the same or neighbouring heliostats and trace
  * nearly parallel shadow and reflected rays. Every realisation is traced once
  * with its own stream; only the order, and so the order of the FP64 sums,
- * changes. The primary draw travels with the sorted offset so that init_path
- * does not draw it again.
+ * changes. Only the sorted offsets are kept, 4 bytes a realisation: the
+ * kernel draws the primary sample again (one Philox block) rather than read
+ * it back. Bound by the rank atomics in shared memory: 16.8e6 realisations
+ * take 57 us to count and 160 us to scatter (480 with tiles of 4096, which
+ * sent four times the global atomics, and 16 bytes of draws scattered with
+ * each offset).
  ******************************************************************************/
 
-/* Sampled primitive of realisation first + j, counted per block in shared
- * memory */
+/* Bins of the sort: the sampled primitives, 2^shift neighbours to a bin where
+ * there are more than the shared-memory histogram holds (neighbours belong to
+ * one instance or to the next) */
+__host__ __device__ inline int sort_shift(int nsamp)
+{
+  int s = 0;
+  while(((nsamp - 1) >> s) + 1 > SORT_MAX_BINS) ++s;
+  return s;
+}
+
+/* Bin of realisation first + j, counted per block in shared memory */
 template<class R>
 __global__ void __launch_bounds__(256) presort_count
-  (const DScene<R> S, uint64_t seed, uint64_t first, uint32_t n, uint32_t* hist)
+  (const DScene<R> S, uint64_t seed, uint64_t first, uint32_t n, int shift, int nb,
+   uint32_t* hist)
 {
   __shared__ uint32_t h[SORT_MAX_BINS];
-  for(int i = threadIdx.x; i < S.nsamp; i += blockDim.x) h[i] = 0;
+  for(int i = threadIdx.x; i < nb; i += blockDim.x) h[i] = 0;
   __syncthreads();
   Rng rng;
   rng.k0 = (uint32_t)seed;
@@ -2141,91 +2175,86 @@ __global__ void __launch_bounds__(256) presort_count
     const uint64_t id = first + j;
     rng.i_lo = (uint32_t)id;
     rng.i_hi = (uint32_t)(id >> 32);
-    atomicAdd(&h[sample_prim(S, rng.get(0u, RNG_PRIMARY))], 1u);
+    atomicAdd(&h[sample_prim(S, rng.get(0u, RNG_PRIMARY)) >> shift], 1u);
   }
   __syncthreads();
-  for(int i = threadIdx.x; i < S.nsamp; i += blockDim.x)
+  for(int i = threadIdx.x; i < nb; i += blockDim.x)
     if(h[i]) atomicAdd(&hist[i], h[i]);
 }
 
-/* Exclusive prefix sum of the nb histogram bins, one block of 1024 threads */
-static __global__ void __launch_bounds__(1024) presort_scan
-  (const uint32_t* hist, uint32_t* off, int nb)
+/* Exclusive prefix sums of histogram bins: block b scans the bins of item b
+ * of a batch, from its first bin in bin_base to the next item's (`nb` for the
+ * last), starting at prefix[b], the budgets before it; without bin_base one
+ * block scans all `nb` */
+constexpr int SCAN_BLOCK = 512;
+static __global__ void __launch_bounds__(SCAN_BLOCK) presort_scan
+  (const uint32_t* hist, uint32_t* off, int nb, const uint32_t* bin_base,
+   const unsigned long long* prefix)
 {
-  __shared__ uint32_t part[1024];
+  __shared__ uint32_t part[SCAN_BLOCK];
   const int t = threadIdx.x;
-  const int per = (nb + 1023) / 1024;
-  const int b0 = min(t * per, nb), b1 = min(b0 + per, nb);
+  const int first = bin_base ? (int)bin_base[blockIdx.x] : 0;
+  const int last = bin_base && blockIdx.x + 1 < gridDim.x ? (int)bin_base[blockIdx.x + 1] : nb;
+  const int per = (last - first + SCAN_BLOCK - 1) / SCAN_BLOCK;
+  const int b0 = min(first + t * per, last), b1 = min(b0 + per, last);
   uint32_t sum = 0;
   for(int i = b0; i < b1; ++i) sum += hist[i];
   part[t] = sum;
   __syncthreads();
-  for(int d = 1; d < 1024; d <<= 1) {
+  for(int d = 1; d < SCAN_BLOCK; d <<= 1) {
     const uint32_t v = t >= d ? part[t - d] : 0u;
     __syncthreads();
     part[t] += v;
     __syncthreads();
   }
-  uint32_t run = t ? part[t - 1] : 0u;
+  uint32_t run = (t ? part[t - 1] : 0u) + (prefix ? (uint32_t)prefix[blockIdx.x] : 0u);
   for(int i = b0; i < b1; ++i) {
     off[i] = run;
     run += hist[i];
   }
 }
 
-/* Each realisation to the next free place of its primitive's range. A block
- * ranks a tile of SCATTER_PER x 256 realisations in shared memory, reserves
- * one range per primitive of the tile with a single global atomic, then
- * writes: one global atomic per (tile, primitive) instead of one per
- * realisation */
-constexpr int SCATTER_PER = 16;
+/* Each realisation to the next free place of its bin's range. A block ranks a
+ * tile of SCATTER_PER x SCATTER_BLOCK realisations in shared memory, reserves
+ * one range per bin of the tile with a single global atomic, then writes the
+ * realisations' offsets */
+constexpr int SCATTER_PER = 16, SCATTER_BLOCK = 1024;
 
 template<class R>
-__global__ void __launch_bounds__(256) presort_scatter
-  (const DScene<R> S, uint64_t seed, uint64_t first, uint32_t n, uint32_t* off,
-   uint4* out_draws, uint32_t* out_off)
+__global__ void __launch_bounds__(SCATTER_BLOCK) presort_scatter
+  (const DScene<R> S, uint64_t seed, uint64_t first, uint32_t n, int shift, int nb,
+   uint32_t* off, uint32_t* out_off)
 {
   __shared__ uint32_t cnt[SORT_MAX_BINS];
-  const int nb = S.nsamp;
-  const uint32_t tile = 256u * SCATTER_PER;
+  const uint32_t tile = (uint32_t)SCATTER_BLOCK * SCATTER_PER;
   Rng rng;
   rng.k0 = (uint32_t)seed;
   rng.k1 = (uint32_t)(seed >> 32);
-  for(uint32_t t0 = blockIdx.x * tile; t0 < n; t0 += gridDim.x * tile) {
-    for(int i = threadIdx.x; i < nb; i += 256) cnt[i] = 0;
+  for(uint64_t t0 = (uint64_t)blockIdx.x * tile; t0 < n; t0 += (uint64_t)gridDim.x * tile) {
+    for(int i = threadIdx.x; i < nb; i += SCATTER_BLOCK) cnt[i] = 0;
     __syncthreads();
     uint32_t k[SCATTER_PER], rank[SCATTER_PER];
 #pragma unroll
     for(int e = 0; e < SCATTER_PER; ++e) {
-      const uint32_t j = t0 + e * 256u + threadIdx.x;
+      const uint64_t j = t0 + e * SCATTER_BLOCK + threadIdx.x;
       k[e] = 0u;
       rank[e] = 0u;
       if(j < n) {
         const uint64_t id = first + j;
         rng.i_lo = (uint32_t)id;
         rng.i_hi = (uint32_t)(id >> 32);
-        k[e] = (uint32_t)sample_prim(S, rng.get(0u, RNG_PRIMARY));
+        k[e] = (uint32_t)sample_prim(S, rng.get(0u, RNG_PRIMARY)) >> shift;
         rank[e] = atomicAdd(&cnt[k[e]], 1u);
       }
     }
     __syncthreads();
-    for(int i = threadIdx.x; i < nb; i += 256)
+    for(int i = threadIdx.x; i < nb; i += SCATTER_BLOCK)
       if(cnt[i]) cnt[i] = atomicAdd(&off[i], cnt[i]);
     __syncthreads();
-    /* The draws again rather than kept: 16 more registers per realisation
-     * of the tile, or 20 B of scratch per realisation */
 #pragma unroll
     for(int e = 0; e < SCATTER_PER; ++e) {
-      const uint32_t j = t0 + e * 256u + threadIdx.x;
-      if(j < n) {
-        const uint32_t pos = cnt[k[e]] + rank[e];
-        const uint64_t id = first + j;
-        rng.i_lo = (uint32_t)id;
-        rng.i_hi = (uint32_t)(id >> 32);
-        const U32x4 r0 = rng.get(0u, RNG_PRIMARY);
-        out_draws[pos] = make_uint4(r0.v[0], r0.v[1], r0.v[2], r0.v[3]);
-        out_off[pos] = j;
-      }
+      const uint64_t j = t0 + e * SCATTER_BLOCK + threadIdx.x;
+      if(j < n) out_off[cnt[k[e]] + rank[e]] = (uint32_t)j;
     }
     __syncthreads();
   }
@@ -2247,56 +2276,68 @@ __device__ __forceinline__ int batch_item_of
   return lo;
 }
 
-/* Sampled primitive of every realisation of the launch, counted in one
- * histogram whose bins run item by item (bin_base) */
-template<class R>
-__global__ void __launch_bounds__(256) batch_presort_count
+/* The two passes of the batched sort: a block takes tiles of SCATTER_PER x
+ * SCATTER_BLOCK realisations and, item by item of the tile (nearly always
+ * one), ranks the item's realisations by bin in shared memory. SCATTER false:
+ * counts into one histogram whose bins run item by item (bin_base). SCATTER
+ * true: reserves the tile's range of every bin with one global atomic, then
+ * writes the realisations' offsets in their item. (One global atomic per
+ * realisation took 0.64 + 0.95 ms for 25e6 realisations of 32 suns.) */
+template<class R, bool SCATTER>
+__global__ void __launch_bounds__(SCATTER_BLOCK) batch_presort
   (const DScene<R>* scenes, const unsigned long long* prefix,
    const unsigned long long* firsts, int nitems, uint64_t seed,
-   const uint32_t* bin_base, uint32_t* hist)
+   const uint32_t* bin_base, uint32_t* bins, uint32_t* sorted_off)
 {
+  __shared__ uint32_t cnt[SORT_MAX_BINS];
   const unsigned long long total = prefix[nitems];
+  const unsigned long long tile = (unsigned long long)SCATTER_BLOCK * SCATTER_PER;
   Rng rng;
   rng.k0 = (uint32_t)seed;
   rng.k1 = (uint32_t)(seed >> 32);
   int item = 0;
-  for(unsigned long long j = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
-      j < total; j += (unsigned long long)gridDim.x * blockDim.x) {
-    item = batch_item_of(prefix, nitems, j, item);
-    const uint64_t id = firsts[item] + (j - prefix[item]);
-    rng.i_lo = (uint32_t)id;
-    rng.i_hi = (uint32_t)(id >> 32);
-    const int k = sample_prim(scenes[item], rng.get(0u, RNG_PRIMARY));
-    atomicAdd(&hist[bin_base[item] + (uint32_t)k], 1u);
-  }
-}
-
-/* Each realisation to the next free place of its (item, primitive) range,
- * with its offset in the item and its primary draw (drawn again: the
- * scratch keeps only the sorted records, 20 B per realisation) */
-template<class R>
-__global__ void __launch_bounds__(256) batch_presort_scatter
-  (const DScene<R>* scenes, const unsigned long long* prefix,
-   const unsigned long long* firsts, int nitems, uint64_t seed,
-   const uint32_t* bin_base, uint32_t* bin_off, uint32_t* sorted_off,
-   uint4* sorted_draw)
-{
-  const unsigned long long total = prefix[nitems];
-  Rng rng;
-  rng.k0 = (uint32_t)seed;
-  rng.k1 = (uint32_t)(seed >> 32);
-  int item = 0;
-  for(unsigned long long j = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
-      j < total; j += (unsigned long long)gridDim.x * blockDim.x) {
-    item = batch_item_of(prefix, nitems, j, item);
-    const uint64_t id = firsts[item] + (j - prefix[item]);
-    rng.i_lo = (uint32_t)id;
-    rng.i_hi = (uint32_t)(id >> 32);
-    const U32x4 r0 = rng.get(0u, RNG_PRIMARY);
-    const int k = sample_prim(scenes[item], r0);
-    const uint32_t pos = atomicAdd(&bin_off[bin_base[item] + (uint32_t)k], 1u);
-    sorted_off[pos] = (uint32_t)(j - prefix[item]);
-    sorted_draw[pos] = make_uint4(r0.v[0], r0.v[1], r0.v[2], r0.v[3]);
+  for(unsigned long long t0 = blockIdx.x * tile; t0 < total; t0 += gridDim.x * tile) {
+    const unsigned long long t1 = t0 + tile < total ? t0 + tile : total;
+    for(unsigned long long j0 = t0; j0 < t1;) {
+      item = batch_item_of(prefix, nitems, j0, item);
+      const unsigned long long start = prefix[item];
+      const unsigned long long j1 = prefix[item + 1] < t1 ? prefix[item + 1] : t1;
+      const DScene<R>& S = scenes[item];
+      const int shift = sort_shift(S.nsamp), nb = ((S.nsamp - 1) >> shift) + 1;
+      uint32_t* item_bins = bins + bin_base[item];
+      for(int i = threadIdx.x; i < nb; i += SCATTER_BLOCK) cnt[i] = 0;
+      __syncthreads();
+      uint32_t k[SCATTER_PER], rank[SCATTER_PER];
+#pragma unroll
+      for(int e = 0; e < SCATTER_PER; ++e) {
+        const unsigned long long j = j0 + e * SCATTER_BLOCK + threadIdx.x;
+        k[e] = 0u;
+        rank[e] = 0u;
+        if(j < j1) {
+          const uint64_t id = firsts[item] + (j - start);
+          rng.i_lo = (uint32_t)id;
+          rng.i_hi = (uint32_t)(id >> 32);
+          k[e] = (uint32_t)sample_prim(S, rng.get(0u, RNG_PRIMARY)) >> shift;
+          rank[e] = atomicAdd(&cnt[k[e]], 1u);
+        }
+      }
+      __syncthreads();
+      for(int i = threadIdx.x; i < nb; i += SCATTER_BLOCK)
+        if(cnt[i]) {
+          const uint32_t at = atomicAdd(&item_bins[i], cnt[i]);
+          if(SCATTER) cnt[i] = at;
+        }
+      __syncthreads();
+      if(SCATTER) {
+#pragma unroll
+        for(int e = 0; e < SCATTER_PER; ++e) {
+          const unsigned long long j = j0 + e * SCATTER_BLOCK + threadIdx.x;
+          if(j < j1) sorted_off[cnt[k[e]] + rank[e]] = (uint32_t)(j - start);
+        }
+        __syncthreads();
+      }
+      j0 = j1;
+    }
   }
 }
 
@@ -2357,57 +2398,70 @@ static int launch_variant
   if(blocks > needed) blocks = needed;
   if(blocks < 1) blocks = 1;
   const cudaStream_t st = (cudaStream_t)stream;
-  const bool sort = !TRACK && cfg.coherent && count >= SORT_MIN && S.nsamp > 1
-                 && S.nsamp <= SORT_MAX_BINS;
+  uint64_t sort_min = cfg.features & (FEAT_QUADRIC | FEAT_DIELECTRIC) ? SORT_MIN_QUADRIC
+                                                                      : SORT_MIN;
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if(!TRACK && count >= sort_min && count < SORT_MIN_CAPTURED
+  && (cudaStreamIsCapturing(st, &capture) != cudaSuccess
+      || capture != cudaStreamCaptureStatusNone))
+    sort_min = SORT_MIN_CAPTURED;
+  const bool want_sort = !TRACK && cfg.coherent && count >= sort_min
+                      && (S.nsampled > 1 || S.nsamp >= SORT_SINGLE);
   DControl ctl;
   ctl.max_failed = cfg.max_failed;
   ctl.stop = cfg.max_failed != ~0ull ? T.counters + 4 : nullptr;
   ctl.abort = cfg.abortable ? T.counters + 5 : nullptr;
   ctl.regen = regen_lanes(cfg.features);
-  if(!sort) {
+  const uint64_t chunk = count < SORT_CHUNK ? count : SORT_CHUNK;
+  const int shift = sort_shift(S.nsamp);
+  const int nbins = ((S.nsamp - 1) >> shift) + 1;
+  const size_t o_soff = 0;
+  const size_t o_hist = o_soff + align256(chunk * sizeof(uint32_t));
+  const size_t o_off = o_hist + align256((size_t)nbins * sizeof(uint32_t));
+  const size_t bytes = o_off + align256((size_t)nbins * sizeof(uint32_t));
+  cudaMemPool_t pool = want_sort ? sort_pool(dev) : nullptr;
+  unsigned char* buf = nullptr;
+  if(pool && cudaMallocFromPoolAsync((void**)&buf, bytes, pool, st) != cudaSuccess) {
+    /* no room for the scratch: id order */
+    cudaGetLastError();
+    buf = nullptr;
+  }
+  if(!buf) {
     /* Work counter of this launch: counters[3] */
     cudaMemsetAsync(T.counters + 3, 0, sizeof(unsigned long long), st);
     realisation_kernel<R, MINB, TRACK, FEAT><<<(unsigned)blocks, block, smem, st>>>
       (S, T, seed, first, count, cfg.max_segments, T.counters + 3, tr, nullptr,
-       nullptr, 1u, ctl);
+       1u, 1u, ctl);
     finish_tallies<R><<<S.nrcv + 1, FINISH_LANES * NRCV_Q * 2, 0, st>>>
       (nullptr, nullptr, T, S.nrcv, S.nsampled);
     return (int)cudaGetLastError();
   }
-  const uint64_t chunk = count < SORT_CHUNK ? count : SORT_CHUNK;
-  const size_t o_sdraws = 0;
-  const size_t o_soff = o_sdraws + align256(chunk * sizeof(uint4));
-  const size_t o_hist = o_soff + align256(chunk * sizeof(uint32_t));
-  const size_t o_off = o_hist + align256((size_t)S.nsamp * sizeof(uint32_t));
-  const size_t bytes = o_off + align256((size_t)S.nsamp * sizeof(uint32_t));
-  cudaMemPool_t pool = sort_pool(dev);
-  unsigned char* buf = nullptr;
-  if(!pool || cudaMallocFromPoolAsync((void**)&buf, bytes, pool, st) != cudaSuccess)
-    return (int)cudaErrorMemoryAllocation;
-  uint4* sdraws = (uint4*)(buf + o_sdraws);
   uint32_t* soff = (uint32_t*)(buf + o_soff);
   uint32_t* hist = (uint32_t*)(buf + o_hist);
   uint32_t* off = (uint32_t*)(buf + o_off);
-  const unsigned sort_blocks = (unsigned)nsm * 8u;
   for(uint64_t c0 = 0; c0 < count; c0 += chunk) {
     const uint32_t n = (uint32_t)(count - c0 < chunk ? count - c0 : chunk);
-    cudaMemsetAsync(hist, 0, (size_t)S.nsamp * sizeof(uint32_t), st);
-    presort_count<R><<<sort_blocks, 256, 0, st>>>(S, seed, first + c0, n, hist);
-    presort_scan<<<1, 1024, 0, st>>>(hist, off, S.nsamp);
-    presort_scatter<R><<<sort_blocks, 256, 0, st>>>(S, seed, first + c0, n, off, sdraws,
-                                                    soff);
+    cudaMemsetAsync(hist, 0, (size_t)nbins * sizeof(uint32_t), st);
+    presort_count<R><<<(unsigned)nsm * 8u, 256, 0, st>>>(S, seed, first + c0, n, shift, nbins,
+                                                         hist);
+    presort_scan<<<1, SCAN_BLOCK, 0, st>>>(hist, off, nbins, nullptr, nullptr);
+    presort_scatter<R><<<(unsigned)nsm * 2u, SCATTER_BLOCK, 0, st>>>
+      (S, seed, first + c0, n, shift, nbins, off, soff);
     uint64_t nb = (n + block - 1) / block;
     if(nb > blocks) nb = blocks;
     /* Segment s of the launch is segment (s x mul) mod nseg of the sorted
      * order, mul coprime with nseg and near nseg / golden ratio */
-    const uint32_t nseg = (uint32_t)((n + SORT_SEG - 1) / SORT_SEG);
+    const uint64_t share = n / (nb * (uint64_t)(block / 32) * SORT_SHARE);
+    const uint32_t seg_len =
+      (uint32_t)std::min<uint64_t>(std::max<uint64_t>(share / 32, 1) * 32, SORT_SEG);
+    const uint32_t nseg = (uint32_t)((n + seg_len - 1) / seg_len);
     uint32_t mul = (uint32_t)(0.6180339887 * nseg) | 1u;
     while(nseg > 1 && std::gcd(mul, nseg) != 1u) mul += 2;
     if(nseg <= 1) mul = 1;
     cudaMemsetAsync(T.counters + 3, 0, sizeof(unsigned long long), st);
     realisation_kernel<R, MINB, TRACK, FEAT><<<(unsigned)nb, block, smem, st>>>
-      (S, T, seed, first + c0, n, cfg.max_segments, T.counters + 3, tr, sdraws, soff,
-       mul, ctl);
+      (S, T, seed, first + c0, n, cfg.max_segments, T.counters + 3, tr, soff,
+       seg_len, mul, ctl);
   }
   finish_tallies<R><<<S.nrcv + 1, FINISH_LANES * NRCV_Q * 2, 0, st>>>
     (nullptr, nullptr, T, S.nrcv, S.nsampled);
@@ -2485,20 +2539,18 @@ static int launch_batch_variant(const BatchLaunch<R>& b, const LaunchConfig& cfg
   const cudaStream_t st = (cudaStream_t)stream;
   const BatchOrder& o = b.order;
   if(o.sorted_off) {
-    const unsigned sort_blocks = (unsigned)nsm * 8u;
     cudaMemsetAsync(o.hist, 0, (size_t)o.nbins * sizeof(uint32_t), st);
-    batch_presort_count<R><<<sort_blocks, 256, 0, st>>>
-      (b.scenes, b.prefix, b.firsts, b.nitems, b.seed, o.bin_base, o.hist);
-    presort_scan<<<1, 1024, 0, st>>>(o.hist, o.bin_off, (int)o.nbins);
-    batch_presort_scatter<R><<<sort_blocks, 256, 0, st>>>
-      (b.scenes, b.prefix, b.firsts, b.nitems, b.seed, o.bin_base, o.bin_off,
-       o.sorted_off, reinterpret_cast<uint4*>(o.sorted_draw));
+    batch_presort<R, false><<<(unsigned)nsm * 2u, SCATTER_BLOCK, 0, st>>>
+      (b.scenes, b.prefix, b.firsts, b.nitems, b.seed, o.bin_base, o.hist, nullptr);
+    presort_scan<<<(unsigned)b.nitems, SCAN_BLOCK, 0, st>>>
+      (o.hist, o.bin_off, (int)o.nbins, o.bin_base, b.prefix);
+    batch_presort<R, true><<<(unsigned)nsm * 2u, SCATTER_BLOCK, 0, st>>>
+      (b.scenes, b.prefix, b.firsts, b.nitems, b.seed, o.bin_base, o.bin_off, o.sorted_off);
   }
   cudaMemsetAsync(b.next_items, 0, (size_t)b.nitems * sizeof(unsigned long long), st);
   batch_kernel<R, MINB, FEAT><<<(unsigned)blocks, block, smem, st>>>
     (b.scenes, b.tallies, b.prefix, b.firsts, b.nitems, b.seed, cfg.max_segments,
-     b.next_items, b.stats, regen_lanes(cfg.features), o.sorted_off,
-     reinterpret_cast<const uint4*>(o.sorted_draw), o.seg_mul);
+     b.next_items, b.stats, regen_lanes(cfg.features), o.sorted_off, o.seg_mul);
   finish_batch<R>(b.scenes, b.tallies, b.nitems, cfg.max_nrcv, st);
   return (int)cudaGetLastError();
 }

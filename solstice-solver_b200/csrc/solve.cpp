@@ -1402,7 +1402,7 @@ struct ssol_b200_batch {
   size_t scene_alloc = 0, tally_alloc = 0; /* bytes of d_scene, d_tally */
   /* Coherent order: sampled triangles per item, their histogram bins (all
    * items), per item its first bin and its segment stride (in d_tally), and
-   * the presort's scratch (20 B per realisation, grown on demand) */
+   * the presort's scratch (4 B per realisation, grown on demand) */
   std::vector<uint32_t> nsamp;
   uint32_t nbins = 0;
   uint32_t* d_bin_base = nullptr;
@@ -1923,10 +1923,7 @@ static BatchOrder batch_order(const ssol_b200_batch* b, bool sorted)
 {
   BatchOrder o;
   if(!sorted) return o;
-  const unsigned long long cap = b->sort_cap;
-  unsigned char* p = (unsigned char*)b->d_sort;
-  o.sorted_draw = (uint32_t*)p;
-  o.sorted_off = (uint32_t*)(p + cap * 16);
+  o.sorted_off = (uint32_t*)b->d_sort;
   o.hist = b->d_hist;
   o.bin_off = b->d_bin_off;
   o.bin_base = b->d_bin_base;
@@ -1966,9 +1963,12 @@ static res_T batch_graph(ssol_b200_batch* b, const ssp_rng* rng, cudaStream_t s,
 }
 
 /* Launches of at least BATCH_SORT_MIN realisations run in the coherent order
- * (up to BATCH_SORT_MAX: the scratch takes 20 B per realisation, and the
- * sorted offsets are 32-bit) */
-constexpr unsigned long long BATCH_SORT_MIN = 1ull << 22;
+ * (up to BATCH_SORT_MAX: the scratch takes 4 B per realisation, and the
+ * sorted offsets are 32-bit). us a launch, id order / sorted, 4 / 32 / 256
+ * suns of 1000 heliostats: 3e5 realisations 437 / 411, 466 / 486, 655 / 775;
+ * 1e6 1209 / 976, 1249 / 1141, 1494 / 1514; 8e6 8851 / 6640, 8988 / 7060,
+ * 9209 / 8187 */
+constexpr unsigned long long BATCH_SORT_MIN = 1ull << 20;
 constexpr unsigned long long BATCH_SORT_MAX = 1ull << 29;
 
 /* Whether this launch runs in the coherent order; grows the scratch (and
@@ -1981,14 +1981,12 @@ static bool batch_prepare_order(ssol_b200_batch* b, unsigned long long total)
     /* one allocation for several launches: a quarter more than asked */
     unsigned long long cap = total + total / 4;
     if(cap > BATCH_SORT_MAX) cap = BATCH_SORT_MAX;
-    /* a multiple of 256: the offsets after the draws start on 256 bytes */
-    cap = (cap + 255) & ~255ull;
     void* p = nullptr;
-    if(dev_alloc(b->dev, &p, (size_t)cap * 20) != cudaSuccess) return false;
+    if(dev_alloc(b->dev, &p, (size_t)cap * sizeof(uint32_t)) != cudaSuccess) return false;
     if(b->graph_exec) { cudaGraphExecDestroy(b->graph_exec); b->graph_exec = nullptr; }
     dev_free(b->dev, b->d_sort, b->sort_alloc);
     b->d_sort = p;
-    b->sort_alloc = (size_t)cap * 20;
+    b->sort_alloc = (size_t)cap * sizeof(uint32_t);
     b->sort_cap = cap;
   }
   /* Per item, the stride of its full segments' order: near n / golden
