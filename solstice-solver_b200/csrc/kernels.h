@@ -197,6 +197,7 @@ struct AdjointArgs {
   double target; /* uniform target flux density */
   double inv_n; /* 1 / realisations */
   double map_scale; /* 1 / (realisations x cell area) */
+  int features; /* FEAT_* bits the scene needs */
 };
 
 /* One adjoint pass (0: objective and map, 1: gradients) */

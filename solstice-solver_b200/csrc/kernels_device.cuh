@@ -2374,6 +2374,74 @@ static size_t path_smem(int feat, int block)
                           + SMEM_STACK * sizeof(int));
 }
 
+/* Scratch and kernels of the coherent order of one chunk of a launch */
+struct SortScratch {
+  unsigned char* buf = nullptr; /* null: id order */
+  uint32_t* sorted_off = nullptr;
+  uint32_t* hist = nullptr;
+  uint32_t* off = nullptr;
+  int shift = 0, nbins = 0;
+};
+template<class R>
+static SortScratch sort_alloc(const DScene<R>& S, uint64_t chunk, int dev, cudaStream_t st)
+{
+  SortScratch q;
+  q.shift = sort_shift(S.nsamp);
+  q.nbins = ((S.nsamp - 1) >> q.shift) + 1;
+  const size_t o_hist = align256(chunk * sizeof(uint32_t));
+  const size_t o_off = o_hist + align256((size_t)q.nbins * sizeof(uint32_t));
+  const size_t bytes = o_off + align256((size_t)q.nbins * sizeof(uint32_t));
+  cudaMemPool_t pool = sort_pool(dev);
+  if(!pool || cudaMallocFromPoolAsync((void**)&q.buf, bytes, pool, st) != cudaSuccess) {
+    /* no room for the scratch: id order */
+    cudaGetLastError();
+    q.buf = nullptr;
+    return q;
+  }
+  q.sorted_off = (uint32_t*)q.buf;
+  q.hist = (uint32_t*)(q.buf + o_hist);
+  q.off = (uint32_t*)(q.buf + o_off);
+  return q;
+}
+template<class R>
+static void sort_launch(const SortScratch& q, const DScene<R>& S, uint64_t seed, uint64_t first,
+                        uint32_t n, int nsm, cudaStream_t st)
+{
+  cudaMemsetAsync(q.hist, 0, (size_t)q.nbins * sizeof(uint32_t), st);
+  presort_count<R><<<(unsigned)nsm * 8u, 256, 0, st>>>(S, seed, first, n, q.shift, q.nbins,
+                                                       q.hist);
+  presort_scan<<<1, SCAN_BLOCK, 0, st>>>(q.hist, q.off, q.nbins, nullptr, nullptr);
+  presort_scatter<R><<<(unsigned)nsm * 2u, SCATTER_BLOCK, 0, st>>>
+    (S, seed, first, n, q.shift, q.nbins, q.off, q.sorted_off);
+}
+/* Realisations of a warp segment for n realisations on `warps` warps */
+static uint32_t segment_length(uint64_t n, uint64_t warps)
+{
+  const uint64_t share = n / (warps * SORT_SHARE) / 32;
+  return (uint32_t)std::min<uint64_t>(std::max<uint64_t>(share, 1) * 32, SORT_SEG);
+}
+/* Segment s of a launch is segment (s x mul) mod nseg of the sorted order,
+ * mul coprime with nseg and near nseg / golden ratio */
+static uint32_t segment_stride(uint32_t nseg)
+{
+  if(nseg <= 1) return 1;
+  uint32_t mul = (uint32_t)(0.6180339887 * nseg) | 1u;
+  while(std::gcd(mul, nseg) != 1u) mul += 2;
+  return mul;
+}
+/* Whether a launch of `count` realisations runs in the coherent order */
+template<class R>
+static bool sort_pays(const DScene<R>& S, uint64_t count, int features, cudaStream_t st)
+{
+  const uint64_t least = features & (FEAT_QUADRIC | FEAT_DIELECTRIC) ? SORT_MIN_QUADRIC
+                                                                     : SORT_MIN;
+  if(count < least || (S.nsampled <= 1 && S.nsamp < SORT_SINGLE)) return false;
+  if(count >= SORT_MIN_CAPTURED) return true;
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(st, &capture) == cudaSuccess
+      && capture == cudaStreamCaptureStatusNone;
+}
+
 template<class R, int MINB, bool TRACK, int FEAT>
 static int launch_variant
   (const DScene<R>& S, const DTallies& T, uint64_t seed, uint64_t first,
@@ -2398,35 +2466,16 @@ static int launch_variant
   if(blocks > needed) blocks = needed;
   if(blocks < 1) blocks = 1;
   const cudaStream_t st = (cudaStream_t)stream;
-  uint64_t sort_min = cfg.features & (FEAT_QUADRIC | FEAT_DIELECTRIC) ? SORT_MIN_QUADRIC
-                                                                      : SORT_MIN;
-  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-  if(!TRACK && count >= sort_min && count < SORT_MIN_CAPTURED
-  && (cudaStreamIsCapturing(st, &capture) != cudaSuccess
-      || capture != cudaStreamCaptureStatusNone))
-    sort_min = SORT_MIN_CAPTURED;
-  const bool want_sort = !TRACK && cfg.coherent && count >= sort_min
-                      && (S.nsampled > 1 || S.nsamp >= SORT_SINGLE);
   DControl ctl;
   ctl.max_failed = cfg.max_failed;
   ctl.stop = cfg.max_failed != ~0ull ? T.counters + 4 : nullptr;
   ctl.abort = cfg.abortable ? T.counters + 5 : nullptr;
   ctl.regen = regen_lanes(cfg.features);
   const uint64_t chunk = count < SORT_CHUNK ? count : SORT_CHUNK;
-  const int shift = sort_shift(S.nsamp);
-  const int nbins = ((S.nsamp - 1) >> shift) + 1;
-  const size_t o_soff = 0;
-  const size_t o_hist = o_soff + align256(chunk * sizeof(uint32_t));
-  const size_t o_off = o_hist + align256((size_t)nbins * sizeof(uint32_t));
-  const size_t bytes = o_off + align256((size_t)nbins * sizeof(uint32_t));
-  cudaMemPool_t pool = want_sort ? sort_pool(dev) : nullptr;
-  unsigned char* buf = nullptr;
-  if(pool && cudaMallocFromPoolAsync((void**)&buf, bytes, pool, st) != cudaSuccess) {
-    /* no room for the scratch: id order */
-    cudaGetLastError();
-    buf = nullptr;
-  }
-  if(!buf) {
+  SortScratch sort;
+  if(!TRACK && cfg.coherent && sort_pays(S, count, cfg.features, st))
+    sort = sort_alloc(S, chunk, dev, st);
+  if(!sort.buf) {
     /* Work counter of this launch: counters[3] */
     cudaMemsetAsync(T.counters + 3, 0, sizeof(unsigned long long), st);
     realisation_kernel<R, MINB, TRACK, FEAT><<<(unsigned)blocks, block, smem, st>>>
@@ -2436,36 +2485,21 @@ static int launch_variant
       (nullptr, nullptr, T, S.nrcv, S.nsampled);
     return (int)cudaGetLastError();
   }
-  uint32_t* soff = (uint32_t*)(buf + o_soff);
-  uint32_t* hist = (uint32_t*)(buf + o_hist);
-  uint32_t* off = (uint32_t*)(buf + o_off);
   for(uint64_t c0 = 0; c0 < count; c0 += chunk) {
     const uint32_t n = (uint32_t)(count - c0 < chunk ? count - c0 : chunk);
-    cudaMemsetAsync(hist, 0, (size_t)nbins * sizeof(uint32_t), st);
-    presort_count<R><<<(unsigned)nsm * 8u, 256, 0, st>>>(S, seed, first + c0, n, shift, nbins,
-                                                         hist);
-    presort_scan<<<1, SCAN_BLOCK, 0, st>>>(hist, off, nbins, nullptr, nullptr);
-    presort_scatter<R><<<(unsigned)nsm * 2u, SCATTER_BLOCK, 0, st>>>
-      (S, seed, first + c0, n, shift, nbins, off, soff);
+    sort_launch(sort, S, seed, first + c0, n, nsm, st);
     uint64_t nb = (n + block - 1) / block;
     if(nb > blocks) nb = blocks;
-    /* Segment s of the launch is segment (s x mul) mod nseg of the sorted
-     * order, mul coprime with nseg and near nseg / golden ratio */
-    const uint64_t share = n / (nb * (uint64_t)(block / 32) * SORT_SHARE);
-    const uint32_t seg_len =
-      (uint32_t)std::min<uint64_t>(std::max<uint64_t>(share / 32, 1) * 32, SORT_SEG);
+    const uint32_t seg_len = segment_length(n, nb * (uint64_t)(block / 32));
     const uint32_t nseg = (uint32_t)((n + seg_len - 1) / seg_len);
-    uint32_t mul = (uint32_t)(0.6180339887 * nseg) | 1u;
-    while(nseg > 1 && std::gcd(mul, nseg) != 1u) mul += 2;
-    if(nseg <= 1) mul = 1;
     cudaMemsetAsync(T.counters + 3, 0, sizeof(unsigned long long), st);
     realisation_kernel<R, MINB, TRACK, FEAT><<<(unsigned)nb, block, smem, st>>>
-      (S, T, seed, first + c0, n, cfg.max_segments, T.counters + 3, tr, soff,
-       seg_len, mul, ctl);
+      (S, T, seed, first + c0, n, cfg.max_segments, T.counters + 3, tr,
+       sort.sorted_off, seg_len, segment_stride(nseg), ctl);
   }
   finish_tallies<R><<<S.nrcv + 1, FINISH_LANES * NRCV_Q * 2, 0, st>>>
     (nullptr, nullptr, T, S.nrcv, S.nsampled);
-  cudaFreeAsync(buf, st);
+  cudaFreeAsync(sort.buf, st);
   return (int)cudaGetLastError();
 }
 

@@ -1212,6 +1212,7 @@ extern "C" res_T ssol_solve_adjoint
   A.target = map->target;
   A.inv_n = 1.0 / (double)n;
   A.map_scale = 1.0 / ((double)n * cw * ch);
+  A.features = plan->meta.features;
 
   std::vector<double> h_map(ncell), h_sums(3);
   unsigned long long h_cnt[4] = {0, 0, 0, 0};
