@@ -17,7 +17,8 @@ struct LaunchConfig {
   int grid_blocks; /* 0 => SMs x resident blocks x waves */
   int waves; /* persistent grid multiplier, 0 => 1 */
   unsigned long long max_segments; /* per path segment budget */
-  int min_blocks; /* register budget: 1 (255 regs), 2 (128) or 3 (85) */
+  int min_blocks; /* register budget: 1 (255 regs), 2 (128) or 3 (64 in FP32,
+                   * four blocks of 256 threads per SM; 80 in FP64) */
   int max_nrcv = 0; /* batched launches: the most receiver sides of an item */
   bool coherent = true; /* larger plain launches run in the order of their
                          * sampled primitives */

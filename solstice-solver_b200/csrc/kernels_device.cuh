@@ -147,7 +147,7 @@ struct Rng {
  * Scalar data and media
  ******************************************************************************/
 /* Clamped linear interpolation (src/ssol_spectrum.c:57-89) */
-__device__ __forceinline__ double interp_clamped
+static __device__ __noinline__ double interp_clamped
   (const double* w, const double* v, int n, double x)
 {
   int lo = 0, hi = n; /* first index with w[i] >= x */
@@ -174,12 +174,9 @@ __device__ __forceinline__ double data_value
 /* Shader value of a material at wavelength wl: index 0 reflectivity,
  * 1 roughness */
 template<class R>
-__device__ __forceinline__ R shader_lerp
-  (const DScene<R>& S, const R* tab, int which, double wl)
+__device__ __noinline__ R shader_lerp(const double* w, int n, const R* tab, int which, double wl)
 {
-  const int n = S.shader_nodes;
   if(n == 1) return tab[which];
-  const double* w = S.shader_wl;
   int lo = 0, hi = n;
   while(lo < hi) {
     const int mid = (lo + hi) >> 1;
@@ -202,7 +199,7 @@ __device__ __forceinline__ R shader_value
   (const DScene<R>& S, const DMaterial& m, int which, double wl)
 {
   if((m.uniform >> which) & 1) return (R)m.value[which];
-  return shader_lerp(S, S.shader_tab + m.table, which, wl);
+  return shader_lerp(S.shader_wl, S.shader_nodes, S.shader_tab + m.table, which, wl);
 }
 
 /* Shader value baked at the vertices of a triangle side (offset `bake` in
@@ -214,9 +211,9 @@ __device__ __forceinline__ R baked_value
 {
   const R* tab = S.bake_tab + bake;
   const int stride = 2 * S.shader_nodes;
-  const R v0 = shader_lerp(S, tab, which, wl);
-  const R v1 = shader_lerp(S, tab + stride, which, wl);
-  const R v2 = shader_lerp(S, tab + 2 * stride, which, wl);
+  const R v0 = shader_lerp(S.shader_wl, S.shader_nodes, tab, which, wl);
+  const R v1 = shader_lerp(S.shader_wl, S.shader_nodes, tab + stride, which, wl);
+  const R v2 = shader_lerp(S.shader_wl, S.shader_nodes, tab + 2 * stride, which, wl);
   return v0 * (R(1) - b1 - b2) + v1 * b1 + v2 * b2;
 }
 
@@ -235,12 +232,10 @@ __device__ __forceinline__ V3<R> sun_local_to_world(const DScene<R>& S, V3<R> p)
 
 /* Buie zenith angle by rejection (src/ssol_ranst_sun_dir.c:177-195); the
  * draws of attempt k come from event 2 + k of the primary domain */
-template<class R>
-__device__ __noinline__ double buie_theta(const DScene<R>& S, const Rng rng)
+static __device__ __noinline__ double buie_theta
+  (double thetaSD, double dCSSD, double gamma, double ek1000g, double alpha, double h1,
+   double h2, double p1, const Rng rng)
 {
-  const double thetaSD = S.buie[0], dCSSD = S.buie[1], gamma = S.buie[2];
-  const double ek1000g = S.buie[3], alpha = S.buie[4];
-  const double h1 = S.buie[5], h2 = S.buie[6], p1 = S.buie[7];
   double theta = 0;
   for(uint32_t k = 0; k < 64; ++k) {
     const U32x4 r = rng.get(2u + k, RNG_PRIMARY);
@@ -261,42 +256,38 @@ __device__ __noinline__ double buie_theta(const DScene<R>& S, const Rng rng)
 }
 
 template<class R>
-__device__ V3<R> sample_sun_dir(const DScene<R>& S, const Rng& rng, U32x4 r)
+__device__ __forceinline__ V3<R> sample_sun_dir(const DScene<R>& S, const Rng& rng, U32x4 r)
 {
-  switch(S.sun_type) {
-    case SUN_PILLBOX: {
-      const R sin2 = uni<R>(r.v[0]) * S.sun_param;
-      const R st = sq_rt(sin2), ct = sq_rt(R(1) - sin2);
-      R sp, cp; sincos2pi(uni<R>(r.v[1]), &sp, &cp);
-      return sun_local_to_world(S, mk(cp * st, sp * st, ct));
-    }
-    case SUN_GAUSSIAN: {
-      /* 1 - u keeps the log argument in (0, 1] */
-      R st = S.sun_param * sq_rt(R(-2) * lg(R(1) - uni<R>(r.v[0])));
-      st = st < R(1) ? st : R(1);
-      const R ct = sq_rt(R(1) - st * st > R(0) ? R(1) - st * st : R(0));
-      R sp, cp; sincos2pi(uni<R>(r.v[1]), &sp, &cp);
-      return sun_local_to_world(S, mk(cp * st, sp * st, ct));
-    }
-    case SUN_BUIE: {
-      const R theta = (R)buie_theta(S, rng);
-      R sp, cp; sincos2pi(uni<R>(r.v[1]), &sp, &cp);
-      const R st = sn(theta), ct = cs(theta);
-      return sun_local_to_world(S, mk(st * sp, st * cp, ct));
-    }
-    default:
-      return ld3(S.sun_dir);
+  if(S.sun_type == SUN_DIRAC) return ld3(S.sun_dir);
+  R st, ct;
+  if(S.sun_type == SUN_PILLBOX) {
+    const R sin2 = uni<R>(r.v[0]) * S.sun_param;
+    st = sq_rt(sin2);
+    ct = sq_rt(R(1) - sin2);
+  } else if(S.sun_type == SUN_GAUSSIAN) {
+    /* 1 - u keeps the log argument in (0, 1] */
+    st = S.sun_param * sq_rt(R(-2) * lg(R(1) - uni<R>(r.v[0])));
+    st = st < R(1) ? st : R(1);
+    ct = sq_rt(R(1) - st * st > R(0) ? R(1) - st * st : R(0));
+  } else {
+    const R theta = (R)buie_theta(S.buie[0], S.buie[1], S.buie[2], S.buie[3], S.buie[4],
+                                  S.buie[5], S.buie[6], S.buie[7], rng);
+    st = sn(theta);
+    ct = cs(theta);
   }
+  /* One copy of the azimuth and of the frame for every sunshape */
+  R sp, cp; sincos2pi(uni<R>(r.v[1]), &sp, &cp);
+  const R x = cp * st, y = sp * st;
+  const bool buie = S.sun_type == SUN_BUIE;
+  return sun_local_to_world(S, mk(buie ? y : x, buie ? x : y, ct));
 }
 
 /* Piecewise linear density over the sun spectrum nodes: pick the interval by
  * its trapezoid mass, then invert the quadratic CDF inside it */
-template<class R>
-__device__ double sample_wavelength(const DScene<R>& S, double u)
+static __device__ __noinline__ double sample_wavelength
+  (const double* nodes, const double* pdf, const double* cdf, int n, double u)
 {
-  const int n = S.wl_count;
-  if(n == 1) return S.wl_nodes[0];
-  const double* cdf = S.wl_cdf;
+  if(n == 1) return nodes[0];
   int lo = 0, hi = n - 1; /* interval j with cdf[j] <= u < cdf[j+1] */
   while(hi - lo > 1) {
     const int mid = (lo + hi) >> 1;
@@ -304,15 +295,18 @@ __device__ double sample_wavelength(const DScene<R>& S, double u)
   }
   const double mass = cdf[lo + 1] - cdf[lo];
   const double r = mass > 0 ? fmin(fmax((u - cdf[lo]) / mass, 0.0), 1.0) : 0;
-  const double a = S.wl_pdf[lo], b = S.wl_pdf[lo + 1];
+  const double a = pdf[lo], b = pdf[lo + 1];
   double t;
   if(a == b) t = r;
   else {
     const double den = a + sqrt(a * a + r * (b * b - a * a));
     t = den > 0 ? r * (a + b) / den : r;
   }
-  return S.wl_nodes[lo] + t * (S.wl_nodes[lo + 1] - S.wl_nodes[lo]);
+  return nodes[lo] + t * (nodes[lo + 1] - nodes[lo]);
 }
+template<class R>
+__device__ __forceinline__ double sample_wavelength(const DScene<R>& S, double u)
+{ return sample_wavelength(S.wl_nodes, S.wl_pdf, S.wl_cdf, S.wl_count, u); }
 
 /*******************************************************************************
  * Punched quadrics (src/ssol_shape.c:236-285, 864-1135, 1408-1494)
@@ -663,14 +657,15 @@ __device__ __forceinline__ bool slab
 
 /* The builder bounds the BVH depth to 30, so a traversal never holds more
  * than 30 deferred nodes. The first SMEM_STACK entries live in shared
- * memory; the rare deeper ones in a per-thread array (local memory), which
- * leaves shared memory to the L1 cache that holds the BVH. With 5 entries
- * three blocks of 256 threads of the realisation kernel (53.4 KB each, plus
- * the 1 KB the SM reserves per block) fit the 164 KB shared-memory
- * configuration of the SM, which leaves 92 KB of L1 instead of 60: field
- * 535 -> 550 Mpaths/s (8 entries needed the 196 KB configuration). */
+ * memory; the rarer deeper ones in a per-thread array (local memory), which
+ * leaves shared memory to the L1 cache that holds the BVH. With 3 entries
+ * four blocks of 256 threads of the realisation kernel (40.4 KB each, with
+ * the 1 KB the SM reserves) fit the 164 KB shared-memory configuration of the
+ * SM, which leaves 92 KB of L1; with 4 or 5 they need the 196 KB one. Field,
+ * 1e8 paths, 2 / 3 / 4 / 5 entries: 64.2 / 64.2 / 65.5 / 65.6 ms; beam-down,
+ * 6e7: 89.1 / 89.0 / 90.7 / 90.8 ms. */
 constexpr int STACK_SIZE = 32;
-constexpr int SMEM_STACK = 5;
+constexpr int SMEM_STACK = 3;
 
 /* Closest accepted hit, or the first accepted hit when `any` (shadow rays).
  * Deferred node i < SMEM_STACK of this thread is stack[i * stride] in shared
@@ -697,53 +692,61 @@ __device__ bool trace_ray
   best.t = rmax<R>();
   bool found = false;
   int spill[STACK_SIZE - SMEM_STACK];
-  int sp = 0;
-  int node = 0;
+  int sp = 0, node = 0;
+  /* The hit leaves of the node last visited, slot 0's first: primitive counts
+   * and references */
+  int lc0 = 0, lf0 = 0, lc1 = 0, lf1 = 0;
+  /* A lane visits nodes until one has hit leaves, then waits for the other
+   * lanes' leaves, so that a warp tests its primitives together: testing them
+   * inside the node loop had nearly every visit of the warp wait for some
+   * lane's test. Each lane still meets nodes and primitives in the same order.
+   * Beam-down, 6e7 paths, 115 -> 104 ms; the field is neutral. */
   for(;;) {
-    const DNode<R> N = load_node(S.nodes + node);
-    if(!(FEAT & FEAT_NOCOUNT)) ++cnt.nodes;
-    R te[2];
-    bool h[2];
-    h[0] = slab(N.lo[0], N.hi[0], inv, oinv, tmin, best.t, te[0])
-        && N.count[0] >= 0;
-    h[1] = slab(N.lo[1], N.hi[1], inv, oinv, tmin, best.t, te[1])
-        && N.count[1] >= 0;
-    /* The hit leaves, slot 0 then slot 1, through one loop so that the
-     * primitive tests are inlined once (a loop over k would be unrolled
-     * and hold two copies of each) */
-    unsigned leaves = (h[0] && N.count[0] > 0 ? 1u : 0u) | (h[1] && N.count[1] > 0 ? 2u : 0u);
-    while(leaves) {
-      const bool k1 = (leaves & 1u) == 0u;
-      leaves &= leaves - 1u;
-      const int lc = k1 ? N.count[1] : N.count[0];
-      const int first = k1 ? N.child[1] : N.child[0];
-      for(int p = 0; p < lc; ++p) {
-        const uint32_t ref = lc == 1 ? (uint32_t)first : S.primrefs[first + p];
-        if(!(FEAT & FEAT_QUADRIC) || primref_kind(ref) == PRIM_TRIANGLE) {
-          if(!(FEAT & FEAT_NOCOUNT)) ++cnt.tris;
-          test_triangle(S, (int)primref_index(ref), o, d, sh, tmin, eps,
-                        self, best, found);
-        } else {
-          if(!(FEAT & FEAT_NOCOUNT)) ++cnt.quads;
-          test_quadric(S, (int)primref_index(ref), o, d, tmin, self,
-                       best, found);
-        }
-        if(any && found) return true;
+    while(lc0 == 0 && node >= 0) {
+      const DNode<R> N = load_node(S.nodes + node);
+      if(!(FEAT & FEAT_NOCOUNT)) ++cnt.nodes;
+      R te[2];
+      bool h[2];
+      h[0] = slab(N.lo[0], N.hi[0], inv, oinv, tmin, best.t, te[0])
+          && N.count[0] >= 0;
+      h[1] = slab(N.lo[1], N.hi[1], inv, oinv, tmin, best.t, te[1])
+          && N.count[1] >= 0;
+      const bool l0 = h[0] && N.count[0] > 0, l1 = h[1] && N.count[1] > 0;
+      lc0 = l0 ? N.count[0] : l1 ? N.count[1] : 0;
+      lf0 = l0 ? N.child[0] : N.child[1];
+      lc1 = l0 && l1 ? N.count[1] : 0;
+      lf1 = N.child[1];
+      const bool in0 = h[0] && N.count[0] == 0, in1 = h[1] && N.count[1] == 0;
+      if(in0 && in1) {
+        const bool first0 = te[0] <= te[1];
+        const int far = first0 ? N.child[1] : N.child[0];
+        if(sp < SMEM_STACK) stack[(sp++) * stride] = far;
+        else if(sp < STACK_SIZE) spill[(sp++) - SMEM_STACK] = far;
+        node = first0 ? N.child[0] : N.child[1];
+      } else if(in0 || in1) {
+        node = in0 ? N.child[0] : N.child[1];
+      } else if(sp == 0) {
+        node = -1;
+      } else {
+        --sp;
+        node = sp < SMEM_STACK ? stack[sp * stride] : spill[sp - SMEM_STACK];
       }
     }
-    const bool in0 = h[0] && N.count[0] == 0, in1 = h[1] && N.count[1] == 0;
-    if(in0 && in1) {
-      const bool first0 = te[0] <= te[1];
-      const int far = first0 ? N.child[1] : N.child[0];
-      if(sp < SMEM_STACK) stack[(sp++) * stride] = far;
-      else if(sp < STACK_SIZE) spill[(sp++) - SMEM_STACK] = far;
-      node = first0 ? N.child[0] : N.child[1];
-    } else if(in0 || in1) {
-      node = in0 ? N.child[0] : N.child[1];
-    } else {
-      if(sp == 0) break;
-      --sp;
-      node = sp < SMEM_STACK ? stack[sp * stride] : spill[sp - SMEM_STACK];
+    if(lc0 == 0) break;
+    const int lc = lc0, first = lf0;
+    lc0 = lc1;
+    lf0 = lf1;
+    lc1 = 0;
+    for(int p = 0; p < lc; ++p) {
+      const uint32_t ref = lc == 1 ? (uint32_t)first : S.primrefs[first + p];
+      if(!(FEAT & FEAT_QUADRIC) || primref_kind(ref) == PRIM_TRIANGLE) {
+        if(!(FEAT & FEAT_NOCOUNT)) ++cnt.tris;
+        test_triangle(S, (int)primref_index(ref), o, d, sh, tmin, eps, self, best, found);
+      } else {
+        if(!(FEAT & FEAT_NOCOUNT)) ++cnt.quads;
+        test_quadric(S, (int)primref_index(ref), o, d, tmin, self, best, found);
+      }
+      if(any && found) return true;
     }
   }
   return found;
@@ -814,11 +817,16 @@ __device__ __forceinline__ V3<R> local_to(V3<R> n, R x, R y, R z)
 
 /* One BSDF sample: the propagated fraction, the outgoing direction, the
  * sampled component (BXDF_*, 0 if none) and the medium beyond, through
- * references; false on an inconsistent medium (RES_BAD_OP). Out of line, to
- * keep the hot loop short. (Returning these as a struct by value measured
- * slower: 354 against 486 Mpaths/s on the field.) */
+ * references; false on an inconsistent medium (RES_BAD_OP). Inlined: a call
+ * that takes the scene by reference gives every thread a copy of the kernel's
+ * scene parameter in local memory (field, 1e8 paths, 73.8 -> 70.3 ms without
+ * it), and spills the registers it may use. What scenes seldom need (spectral
+ * tables, wavelengths, Buie's rejection loop, further receiver hits of a path)
+ * stays out of line, as the bounce loop is bound by instruction fetch: 77.6
+ * -> 73.9 ms. With the commit inlined as well: 70.2 -> 67.7 ms, beam-down,
+ * 6e7, 104 -> 96 ms. */
 template<class R, int FEAT = FEAT_ALL>
-__device__ __noinline__ bool shade
+__device__ __forceinline__ bool shade
   (const DScene<R>& S, const Rng& rng, uint32_t scatter, int mtl_idx,
    int medium, double wl, V3<R> wo, V3<R> Ng, R& prop, V3<R>& out,
    int& type, int& next_medium, int gid, int side, const double* ps, int stride)
@@ -973,7 +981,8 @@ __device__ __noinline__ bool shade
  ******************************************************************************/
 enum : int { PH_NONE = 0, PH_SHADOW = 1, PH_BOUNCE = 2, PH_ENDED = 3 };
 enum : int {
-  END_NONE = 0, END_SHADOW, END_MISS, END_ZERO, END_KILL, END_FAIL
+  END_NONE = 0, END_SHADOW, END_MISS, END_ZERO, END_KILL, END_FAIL,
+  END_OVERFLOW /* a failure: more receiver entries than a path keeps */
 };
 
 /* Extra (receiver side, primitive) entries of one path beyond the first,
@@ -1124,18 +1133,12 @@ __device__ __forceinline__ void init_path
   p.phase = PH_SHADOW;
 }
 
+/* A path's receiver hits beyond its first */
 template<class R>
-__device__ __forceinline__ void add_entry
+__device__ __noinline__ void add_entry_again
   (PathState<R>& p, int rslot, int pslot, const double v[6], double* ps,
    int stride, int* xr, int* xp, double (*xv)[6])
 {
-  if(p.nent == 0) {
-    p.nent = 1;
-    p.r0 = rslot;
-    p.p0 = pslot;
-    for(int q = 0; q < 6; ++q) ps[(PS_V0 + q) * stride] = v[q];
-    return;
-  }
   if(p.r0 == rslot && p.p0 == pslot) {
     for(int q = 0; q < 6; ++q) ps[(PS_V0 + q) * stride] += v[q];
     return;
@@ -1152,6 +1155,21 @@ __device__ __forceinline__ void add_entry
   xp[e] = pslot;
   for(int q = 0; q < 6; ++q) xv[e][q] = v[q];
   ++p.nent;
+}
+
+template<class R>
+__device__ __forceinline__ void add_entry
+  (PathState<R>& p, int rslot, int pslot, const double v[6], double* ps,
+   int stride, int* xr, int* xp, double (*xv)[6])
+{
+  if(p.nent == 0) {
+    p.nent = 1;
+    p.r0 = rslot;
+    p.p0 = pslot;
+    for(int q = 0; q < 6; ++q) ps[(PS_V0 + q) * stride] = v[q];
+    return;
+  }
+  add_entry_again(p, rslot, pslot, v, ps, stride, xr, xp, xv);
 }
 
 /* One surface interaction (src/ssol_solver.c:939-1011): extinction of the
@@ -1311,44 +1329,52 @@ static __device__ __noinline__ void flush_samp
  * scene) */
 constexpr int MIN_GROUP = 4;
 
+/* A path's end: what commit_warp reads of it stays in p (the weight
+ * shadowed or missing in prev[0]) */
+template<class R>
+__device__ __forceinline__ void path_ended(PathState<R>& p, int end)
+{
+  if(end == END_MISS && p.virt) p.prev[0] = p.inc0;
+  p.end = p.overflow ? END_OVERFLOW : end;
+  p.phase = PH_ENDED;
+}
+
 /* Commit the finished paths of the lanes with `ended`: FP64 (w, w^2) of each
  * path's totals, x 2^score for roulette survivors (src/ssol_solver.c:
  * 1087-1108). All lanes of the warp call it converged. The lanes of one
  * sampled instance (in the coherent order nearly always the whole warp) add
  * through the warp's tiles, the others, and any path with a weight that is
  * not finite, through reductions of their own. */
-template<class R>
-static __device__ __noinline__ void commit_warp
-  (int nrcv, const DTallies* tallies, int item, const PathState<R>& p, bool ended,
-   const double* ps, int stride, double2* tile, WarpKeys* wk, const int* xr,
+static __device__ __forceinline__ void commit_warp
+  (int nrcv, const DTallies* tallies, int item, bool ended, int end, int p_samp, int score,
+   int p_nent, int p_r0, int p0, double weight, const double* ps, int stride, double2* tile, WarpKeys* wk, const int* xr,
    const int* xp, const double (*xv)[6], const DControl* ctl)
 {
   const unsigned FULL = 0xffffffffu;
   const unsigned lane = threadIdx.x & 31u;
   const DTallies& T = tallies[item];
-  const int end = p.overflow ? END_FAIL : p.end;
-  const bool good = ended && end != END_FAIL && end != END_KILL;
-  if(ended && end == END_FAIL) {
+  const bool good = ended && end < END_KILL;
+  if(ended && end >= END_FAIL) {
     /* The failure that reaches the limit stops the launch's work fetch
      * (src/ssol_solver.c:1240-1245) */
     const unsigned long long nf = atomicAdd(&T.counters[0], 1ull) + 1ull;
     if(ctl && ctl->stop && nf >= ctl->max_failed) atomicExch(ctl->stop, 1ull);
-    if(p.overflow) atomicAdd(&T.counters[2], 1ull);
+    if(end == END_OVERFLOW) atomicAdd(&T.counters[2], 1ull);
   }
   if(ended && end == END_KILL) atomicAdd(&T.counters[1], 1ull);
-  const int samp = ended ? p.samp : -1;
-  const int nent = good ? p.nent : 0;
-  const int r0 = nent ? p.r0 : -1;
+  const int samp = ended ? p_samp : -1;
+  const int nent = good ? p_nent : 0;
+  const int r0 = nent ? p_r0 : -1;
   double f = 0, wcos = 0, wabs = 0, wsh = 0, wmiss = 0, watm = 0, woth = 0;
   double q[NRCV_Q] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
   double chk = 0;
   if(good) {
-    f = (double)(1ull << p.score);
+    f = (double)(1ull << score);
     wcos = f * ps[PS_COS * stride];
     wabs = f * ps[PS_ABS * stride];
     watm = f * ps[PS_ATM * stride];
     woth = f * ps[PS_OTHER * stride];
-    const double w_end = f * (end == END_MISS && p.virt ? p.inc0 : p.prev[0]);
+    const double w_end = f * weight;
     if(end == END_SHADOW) wsh = w_end;
     if(end == END_MISS) wmiss = w_end;
     chk = wcos * wcos + wabs * wabs + watm * watm + woth * woth + w_end * w_end;
@@ -1470,8 +1496,8 @@ static __device__ __noinline__ void commit_warp
     const double a4 = ps[(PS_V0 + 4) * stride], a5 = ps[(PS_V0 + 5) * stride];
     if(!rcv_done)
       commit10(T.samp_rcv + ((size_t)samp * nrcv + r0) * NRCV_Q * 2, a0, a1, a2, a3, a4, a5, f);
-    if(p.p0 >= 0)
-      commit10(T.prim + (size_t)p.p0 * NRCV_Q * 2, a0, a1, a2, a3, a4, a5, f);
+    if(p0 >= 0)
+      commit10(T.prim + (size_t)p0 * NRCV_Q * 2, a0, a1, a2, a3, a4, a5, f);
   } else if(nent > 1) {
     double v0[6];
     for(int k = 0; k < 6; ++k) v0[k] = ps[(PS_V0 + k) * stride];
@@ -1489,7 +1515,7 @@ static __device__ __noinline__ void commit_warp
         }
         commit10(T.samp_rcv + ((size_t)samp * nrcv + re) * NRCV_Q * 2, v, f);
       }
-      const int prim = e == 0 ? p.p0 : xp[e - 1];
+      const int prim = e == 0 ? p0 : xp[e - 1];
       if(prim >= 0) {
         /* (receiver side, primitive) keys are unique among the entries */
         commit10(T.prim + (size_t)prim * NRCV_Q * 2, e == 0 ? v0 : xv[e - 1], f);
@@ -1611,7 +1637,7 @@ __device__ __forceinline__ void track_vertex
 }
 
 template<class R, int MINB, bool TRACK, int FEAT>
-__global__ void __launch_bounds__(MAX_BLOCK, MINB)
+__global__ void __launch_bounds__(MAX_BLOCK, sizeof(R) == 4 && MINB == 3 ? 4 : MINB)
 realisation_kernel
   (const DScene<R> S, const DTallies T,
    uint64_t seed, uint64_t first, uint64_t count, unsigned long long max_segments,
@@ -1664,19 +1690,19 @@ realisation_kernel
        <= (age <= REGEN_AGE ? ctl.regen : max(ctl.regen, REGEN_LATE))) {
       age = 0;
       if(__any_sync(0xffffffffu, p.phase == PH_ENDED)) {
-        commit_warp(S.nrcv, &tallies, 0, p, p.phase == PH_ENDED, ps, bd, tile, wk, xr, xp, xv,
-                    &ctl);
+        commit_warp(S.nrcv, &tallies, 0, p.phase == PH_ENDED, p.end, p.samp, p.score, p.nent,
+                    p.r0, p.p0, p.prev[0], ps, bd, tile, wk, xr, xp, xv, &ctl);
         if(p.phase == PH_ENDED) p.phase = PH_NONE;
       }
       need = __ballot_sync(0xffffffffu, p.phase == PH_NONE && !done);
     }
     bool start = false;
     uint64_t off = 0;
-    /* Early stop: every 8th fetch of the warp reads the stop and abort
-     * words (one L2 sector); a halted warp takes no new realisation and ends
+    /* Early stop: every 4th fetch of the warp (of 32 realisations or so)
+     * reads the stop and abort words (one L2 sector); a halted warp takes no new realisation and ends
      * once its paths in flight end */
     bool halt = false;
-    if(need && polled && (fetches++ & 7u) == 0u) {
+    if(need && polled && (fetches++ & 3u) == 0u) {
       const int leader = __ffs(need) - 1;
       int h = 0;
       if((int)lane == leader) {
@@ -1851,8 +1877,7 @@ realisation_kernel
           : (end == END_FAIL || p.overflow) ? 3 : (p.nent > 0 ? 2 : 0);
         tr.path_nv[p.tslot] = (int32_t)p.tseq;
       }
-      p.end = end;
-      p.phase = PH_ENDED;
+      path_ended(p, end);
     }
   }
 
@@ -1887,7 +1912,7 @@ realisation_kernel
  * to another item. The launch's total is prefix[nitems], read from device
  * memory so that a captured CUDA graph replays with new budgets. */
 template<class R, int MINB, int FEAT>
-__global__ void __launch_bounds__(MAX_BLOCK, MINB)
+__global__ void __launch_bounds__(MAX_BLOCK, sizeof(R) == 4 && MINB == 3 ? 4 : MINB)
 batch_kernel
   (const DScene<R>* __restrict__ scenes, const DTallies* __restrict__ tallies,
    const unsigned long long* __restrict__ prefix,
@@ -1967,8 +1992,9 @@ batch_kernel
        <= (age <= REGEN_AGE ? regen : max(regen, REGEN_LATE))) {
       age = 0;
       if(__any_sync(0xffffffffu, p.phase == PH_ENDED)) {
-        commit_warp(scene_of(it).nrcv, tallies, it, p, p.phase == PH_ENDED, ps, bd, tile, wk,
-                    xr, xp, xv, (const DControl*)nullptr);
+        commit_warp(scene_of(it).nrcv, tallies, it, p.phase == PH_ENDED, p.end, p.samp, p.score,
+                    p.nent, p.r0, p.p0, p.prev[0], ps, bd, tile, wk, xr, xp, xv,
+                    (const DControl*)nullptr);
         if(p.phase == PH_ENDED) p.phase = PH_NONE;
       }
       need = __ballot_sync(0xffffffffu, p.phase == PH_NONE && !done);
@@ -2118,8 +2144,7 @@ batch_kernel
     if(do_interact)
       end = interact<R, FEAT>(S, rng, p, pos, dir, bounces, max_segments, ps, bd, xr, xp, xv);
     if(end != END_NONE) {
-      p.end = end;
-      p.phase = PH_ENDED;
+      path_ended(p, end);
     }
   }
 

@@ -40,7 +40,7 @@ PHILOX_HD U32x4 philox4x32_10
 {
   const uint32_t M0 = 0xD2511F53u, M1 = 0xCD9E8D57u;
   const uint32_t W0 = 0x9E3779B9u, W1 = 0xBB67AE85u;
-#pragma unroll
+#pragma unroll 2
   for(int r = 0; r < 10; ++r) {
     if(r) { k0 += W0; k1 += W1; }
     uint32_t hi0, lo0, hi1, lo1;

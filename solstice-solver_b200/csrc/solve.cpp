@@ -265,10 +265,10 @@ struct ssol_b200_plan {
   size_t bvh2_alloc = 0;
 };
 
-/* Default register budget: 3 blocks of 256 threads per SM (80 registers) in
- * FP32, whose feature variants spill little there and gain from 24 warps
- * per SM (field 532 against 483 Mpaths/s at 2, beam-down 174 against 167);
- * 2 in FP64, whose registers are twice as wide */
+/* Default register budget: 3 in FP32 (64 registers, four blocks of 256 threads
+ * per SM: field, 1e8 paths, 64.2 ms against 76.0 at 2, 128 registers;
+ * beam-down, 6e7, 89 against 102); 2 in FP64, whose registers are twice as
+ * wide */
 static int default_min_blocks(ssol_b200_precision p)
 {
   return p == SSOL_B200_FP32 ? 3 : 2;
