@@ -118,7 +118,7 @@ struct AdjointGrad { int slot; double abs_a, abs_b, spill_a, spill_b; };
 template<class R, int PASS, int FEAT>
 __device__ __forceinline__ void adjoint_path
   (const DScene<R>& S, const AdjointArgs& A, const Rng& rng, AdjointSums& sums,
-   AdjointGrad& grad, Counters& cnt, int* stack, int stride)
+   AdjointGrad& grad, Counters& cnt)
 {
   /* Primary sample: the draws and arithmetic of init_path */
   const U32x4 r0 = rng.get(0u, RNG_PRIMARY);
@@ -191,7 +191,7 @@ __device__ __forceinline__ void adjoint_path
   self.side = side;
   self.discard_virtual = true;
   self.reversed = true;
-  if(trace_ray<R, FEAT>(S, pos, -dir, R(0), self, true, h, cnt, stack, stride)) return;
+  if(trace_ray<R, FEAT>(S, pos, -dir, R(0), self, true, h, cnt)) return;
 
   /* Mirror reflection with the draws of shade() (scatter event 0) */
   const R refl = bake >= 0 ? baked_value(S, bake, 0, wl, b1, b2)
@@ -233,7 +233,7 @@ __device__ __forceinline__ void adjoint_path
   const V3<R> rd = mk((R)out.x.v, (R)out.y.v, (R)out.z.v);
   self.discard_virtual = false;
   self.reversed = false;
-  const bool found = trace_ray<R, FEAT>(S, pos, rd, R(0), self, false, h, cnt, stack, stride);
+  const bool found = trace_ray<R, FEAT>(S, pos, rd, R(0), self, false, h, cnt);
   bool on_rcv = false;
   int hside = 1;
   if(found) {
@@ -351,17 +351,15 @@ __device__ __forceinline__ void adjoint_flush(const AdjointArgs& A, int slot, do
 /* Warps take segments of seg_len realisations of the launch's order, spread
  * by the stride seg_mul. Bound by the latency of the two casts: in id order
  * each lane traced another part of the field and sent four atomics to its
- * heliostat's slots; sorted, 1e7 paths of 1000 heliostats take 6.0 and 7.2 ms
- * a pass (10.4 and 12.1), the sort 0.15. Two blocks per SM (128 registers):
- * with one, 8 warps per SM hid the BVH loads. */
+ * heliostat's slots. 1e7 paths of 1000 heliostats, ms a pass: id order 10.4
+ * and 12.1; sorted 6.0 and 7.2 (the sort 0.15); with the deferred nodes in
+ * local memory 4.65 and 5.8; and with 4 blocks of 64 registers an SM instead
+ * of 2 of 128 in the mesh variant, 3.9 and 5.2 (3 blocks 4.2 and 5.3). */
 template<class R, int PASS, int FEAT>
-__global__ void __launch_bounds__(MAX_BLOCK, 2)
+__global__ void __launch_bounds__(MAX_BLOCK, FEAT == 0 ? 4 : 2)
 adjoint_kernel(const DScene<R> S, const AdjointArgs A, uint64_t seed, uint64_t first,
                uint32_t count, const uint32_t* sorted_off, uint32_t seg_len, uint32_t seg_mul)
 {
-  __shared__ int stack_sm[SMEM_STACK * MAX_BLOCK];
-  int* stack = stack_sm + threadIdx.x;
-  const int stride = blockDim.x;
   const uint32_t lane = threadIdx.x & 31u;
   Counters cnt = {0, 0, 0, 0};
   Rng rng;
@@ -381,7 +379,7 @@ adjoint_kernel(const DScene<R> S, const AdjointArgs A, uint64_t seed, uint64_t f
         const uint64_t id = first + (sorted_off ? __ldcs(sorted_off + b + lane) : b + lane);
         rng.i_lo = (uint32_t)id;
         rng.i_hi = (uint32_t)(id >> 32);
-        adjoint_path<R, PASS, FEAT>(S, A, rng, sums, g, cnt, stack, stride);
+        adjoint_path<R, PASS, FEAT>(S, A, rng, sums, g, cnt);
       }
       if(PASS == 0) continue;
       __syncwarp();

@@ -54,12 +54,12 @@ __device__ __forceinline__ void camera_ray(const DrawArgs& A, float sx, float sy
 
 /* Shading normal of a hit (surface_fragment_setup, src/ssol_material.c:
  * 630-654): the interpolated vertex normal turned toward -dir, else N */
-template<class R>
+template<class R, int FEAT>
 __device__ __forceinline__ V3<R> draw_shading_normal
   (const DScene<R>& S, int gid, V3<R> pos, V3<R> dir, V3<R> N, R& b1, R& b2)
 {
   b1 = b2 = R(0);
-  if(!S.tshade || gid < 0) return N;
+  if(!(FEAT & FEAT_ATTRIBUTES) || !S.tshade || gid < 0) return N;
   const float2 uv = tri_uv(S, gid, pos);
   b1 = (R)uv.x;
   b2 = (R)uv.y;
@@ -84,10 +84,9 @@ __device__ __forceinline__ void draw_flush(unsigned long long* ctr, const uint32
 }
 
 /* ssol_draw_draft: Li and draw_pixel of src/ssol_draw_draft.c:37-142 */
-template<class R>
+template<class R, int FEAT>
 __global__ void __launch_bounds__(256) draft_kernel(const DScene<R> S, const DrawArgs A)
 {
-  extern __shared__ int draw_stack[];
   int px, py;
   draw_pixel_of(blockIdx.x, threadIdx.x, A.width, px, py);
   const bool valid = px < A.width && py < A.height;
@@ -103,14 +102,12 @@ __global__ void __launch_bounds__(256) draft_kernel(const DScene<R> S, const Dra
       const V3<R> o = mk((R)A.cam_pos[0], (R)A.cam_pos[1], (R)A.cam_pos[2]);
       const V3<R> d = mk((R)df[0], (R)df[1], (R)df[2]);
       Hit<R> h;
-      if(!trace_ray(S, o, d, R(0), self, false, h, cnt, draw_stack + threadIdx.x,
-                    (int)blockDim.x))
-        continue;
+      if(!trace_ray<R, FEAT>(S, o, d, R(0), self, false, h, cnt)) continue;
       const V3<R> wi = normalize(d);
       V3<R> N = normalize_hit(h.n);
       if(!(dot(N, wi) < R(0))) N = -N;
       R b1, b2;
-      N = draw_shading_normal(S, h.gid, o + d * h.t, wi, N, b1, b2);
+      N = draw_shading_normal<R, FEAT>(S, h.gid, o + d * h.t, wi, N, b1, b2);
       const double c = (double)dot_yx(N, -wi);
       sum += c > 0.0 ? c : 0.0;
     }
@@ -189,7 +186,7 @@ __device__ __forceinline__ R draw_bsdf_eval(const DrawBsdf<R>& f, V3<R> wo, V3<R
 
 /* ssf_bsdf_sample: direction wi and weight R (src/ssol_draw_pt.c:257-264);
  * next_medium follows material_get_next_medium on a transmission */
-template<class R>
+template<class R, int FEAT>
 __device__ __forceinline__ R draw_bsdf_sample
   (const DScene<R>& S, const DrawBsdf<R>& f, const U32x4& r, int medium, double wl,
    V3<R> wo, V3<R> N, V3<R>& wi, int& type, int& next_medium)
@@ -230,6 +227,7 @@ __device__ __forceinline__ R draw_bsdf_sample
       return f.refl;
     }
     case MTL_DIELECTRIC: {
+      if(!(FEAT & FEAT_DIELECTRIC)) return R(0);
       const R eta_i = (R)data_value(S, S.media[m.out_medium].refractive_index, wl);
       const R eta_t = (R)data_value(S, S.media[m.in_medium].refractive_index, wl);
       const R eta = eta_i / eta_t;
@@ -250,6 +248,7 @@ __device__ __forceinline__ R draw_bsdf_sample
       return R(1);
     }
     case MTL_THIN_DIELECTRIC: {
+      if(!(FEAT & FEAT_DIELECTRIC)) return R(0);
       const R eta_i = (R)data_value(S, S.media[m.out_medium].refractive_index, wl);
       const R eta_t = (R)data_value(S, S.media[m.slab_medium].refractive_index, wl);
       const R alpha = (R)data_value(S, S.media[m.slab_medium].extinction, wl);
@@ -280,11 +279,10 @@ __device__ __forceinline__ R draw_bsdf_sample
 
 /* Li of src/ssol_draw_pt.c:124-290 for one attempt. Returns false on an
  * inconsistent medium (RES_BAD_OP), which the caller retries. */
-template<class R>
-__device__ __noinline__ bool draw_radiance
+template<class R, int FEAT>
+__device__ __forceinline__ bool draw_radiance
   (const DScene<R>& S, const DrawArgs& A, const Rng& rng, uint32_t attempt,
-   V3<R> org, V3<R> dir, double& L, Counters& cnt, uint32_t& bounces,
-   int* stack, int stride)
+   V3<R> org, V3<R> dir, double& L, Counters& cnt, uint32_t& bounces)
 {
   L = 0;
   double thr = 1;
@@ -297,7 +295,7 @@ __device__ __noinline__ bool draw_radiance
   const V3<R> to_sun = -ld3(S.sun_dir);
   for(int b = 0; b < DRAW_MAX_BOUNCES; ++b) {
     Hit<R> h;
-    if(!trace_ray(S, org, dir, R(0), self, false, h, cnt, stack, stride)) {
+    if(!trace_ray<R, FEAT>(S, org, dir, R(0), self, false, h, cnt)) {
       if(dot(dir, up) > R(0)) L += thr * 1e-1;
       break;
     }
@@ -312,10 +310,11 @@ __device__ __noinline__ bool draw_radiance
     if(!(dot(Ng, wo_in) < R(0))) { side = 2; Ng = -Ng; }
     const V3<R> pos = org + dir * h.t;
     R b1, b2;
-    const V3<R> N = draw_shading_normal(S, h.gid, pos, wo_in, Ng, b1, b2);
+    const V3<R> N = draw_shading_normal<R, FEAT>(S, h.gid, pos, wo_in, Ng, b1, b2);
     if(dot(N, wo_in) > R(0)) break;
     const DShadedInst& si = S.sinsts[h.sinst];
-    const int bake = S.tshade && h.gid >= 0 ? S.tshade[h.gid].bake[side - 1] : -1;
+    const int bake = (FEAT & FEAT_ATTRIBUTES) && S.tshade && h.gid >= 0
+      ? S.tshade[h.gid].bake[side - 1] : -1;
     const DrawBsdf<R> f = draw_bsdf(S, si.mtl[side - 1], bake, wl, b1, b2);
     /* src/ssol_material.c:97-101 */
     if(f.m.type == MTL_DIELECTRIC && medium != f.m.out_medium) return false;
@@ -332,7 +331,7 @@ __device__ __noinline__ bool draw_radiance
         const R fv = draw_bsdf_eval(f, wo, N, to_sun);
         if(fv > R(0)) {
           Hit<R> hs;
-          if(!trace_ray(S, org, to_sun, R(0), self, true, hs, cnt, stack, stride))
+          if(!trace_ray<R, FEAT>(S, org, to_sun, R(0), self, true, hs, cnt))
             L += thr * (double)(fv * c);
         }
       }
@@ -340,7 +339,7 @@ __device__ __noinline__ bool draw_radiance
     const uint32_t ev = (attempt << 20) | (uint32_t)b;
     V3<R> wi;
     int type, next_medium;
-    R w = draw_bsdf_sample(S, f, rng.get(ev, RNG_DRAW_BSDF), medium, wl, wo, N, wi,
+    R w = draw_bsdf_sample<R, FEAT>(S, f, rng.get(ev, RNG_DRAW_BSDF), medium, wl, wo, N, wi,
                            type, next_medium);
     /* Wrong hemisphere for the sampled component, against Ng */
     const R cg = dot(Ng, wi);
@@ -361,11 +360,15 @@ __device__ __noinline__ bool draw_radiance
   return true;
 }
 
-/* ssol_draw_pt: draw_pixel of src/ssol_draw_pt.c:292-350 */
-template<class R>
-__global__ void __launch_bounds__(256) pt_kernel(const DScene<R> S, const DrawArgs A)
+/* ssol_draw_pt: draw_pixel of src/ssol_draw_pt.c:292-350. Bound by latency: the
+ * radiance loop out of line, with a copy of the scene record per thread, took
+ * 12.8 ms for the 1080p field view at 16 samples; inlined and without the code
+ * for quadrics, dielectrics and attributes 7.0 (96 registers), and in 64
+ * registers, four blocks an SM, 6.0 (80: 6.3). The draft's kernel, 0.62 ->
+ * 0.42 ms, is fastest in the registers it takes by itself (64). */
+template<class R, int FEAT>
+__global__ void __launch_bounds__(256, FEAT == 0 ? 4 : 1) pt_kernel(const DScene<R> S, const DrawArgs A)
 {
-  extern __shared__ int draw_stack[];
   int px, py;
   draw_pixel_of(blockIdx.x, threadIdx.x, A.width, px, py);
   const bool valid = px < A.width && py < A.height;
@@ -392,8 +395,7 @@ __global__ void __launch_bounds__(256) pt_kernel(const DScene<R> S, const DrawAr
       double L = 0;
       bool ok = false;
       for(uint32_t a = 0; a < (uint32_t)DRAW_MAX_FAILURES && !ok; ++a)
-        ok = draw_radiance(S, A, rng, a, o, d, L, cnt, bounces,
-                           draw_stack + threadIdx.x, (int)blockDim.x);
+        ok = draw_radiance<R, FEAT>(S, A, rng, a, o, d, L, cnt, bounces);
       if(!ok) failed = true;
       else sum += L;
     }
@@ -410,16 +412,31 @@ __global__ void __launch_bounds__(256) pt_kernel(const DScene<R> S, const DrawAr
   draw_flush(A.counters, c6);
 }
 
+template<class R, int FEAT>
+static void launch_draw_variant(const DScene<R>& S, const DrawArgs& A, bool pt, unsigned grid,
+                                cudaStream_t st)
+{
+  if(pt) pt_kernel<R, FEAT><<<grid, 256, 0, st>>>(S, A);
+  else draft_kernel<R, FEAT><<<grid, 256, 0, st>>>(S, A);
+}
+
+/* FP32 scenes of meshes with mirror and matte materials only get a variant
+ * without the code for the rest */
 template<class R>
 static int launch_draw(const DScene<R>& S, const DrawArgs& A, bool pt, void* stream)
 {
   if(A.width <= 0 || A.height <= 0 || A.spp <= 0) return (int)cudaErrorInvalidValue;
   const long long ntx = (A.width + 15) / 16, nty = (A.height + 15) / 16;
   if(ntx * nty > 0x7fffffffLL) return (int)cudaErrorInvalidValue;
-  const dim3 grid((unsigned)(ntx * nty));
-  const size_t smem = (size_t)SMEM_STACK * 256 * sizeof(int);
-  if(pt) pt_kernel<R><<<grid, 256, smem, (cudaStream_t)stream>>>(S, A);
-  else draft_kernel<R><<<grid, 256, smem, (cudaStream_t)stream>>>(S, A);
+  const unsigned grid = (unsigned)(ntx * nty);
+  const cudaStream_t st = (cudaStream_t)stream;
+  if constexpr(sizeof(R) == sizeof(float)) {
+    if(A.features == 0) {
+      launch_draw_variant<R, 0>(S, A, pt, grid, st);
+      return (int)cudaGetLastError();
+    }
+  }
+  launch_draw_variant<R, FEAT_ALL>(S, A, pt, grid, st);
   return (int)cudaGetLastError();
 }
 

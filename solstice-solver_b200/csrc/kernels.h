@@ -223,6 +223,7 @@ struct DrawArgs {
   uint64_t seed;
   double* pixels;
   unsigned long long* counters;
+  int features; /* FEAT_* bits the scene needs */
 };
 
 int launch_draft_f32(const DScene<float>& S, const DrawArgs& A, void* stream);

@@ -656,24 +656,18 @@ __device__ __forceinline__ bool slab
 }
 
 /* The builder bounds the BVH depth to 30, so a traversal never holds more
- * than 30 deferred nodes. The first SMEM_STACK entries live in shared
- * memory; the rarer deeper ones in a per-thread array (local memory), which
- * leaves shared memory to the L1 cache that holds the BVH. With 3 entries
- * four blocks of 256 threads of the realisation kernel (40.4 KB each, with
- * the 1 KB the SM reserves) fit the 164 KB shared-memory configuration of the
- * SM, which leaves 92 KB of L1; with 4 or 5 they need the 196 KB one. Field,
- * 1e8 paths, 2 / 3 / 4 / 5 entries: 64.2 / 64.2 / 65.5 / 65.6 ms; beam-down,
- * 6e7: 89.1 / 89.0 / 90.7 / 90.8 ms. */
+ * than 30 deferred nodes. They live in a per-thread array: the few entries in
+ * use stay in L1, one line a warp where its lanes are equally deep, and the
+ * loop has no second place to look. With the first 3 / 5 entries in shared
+ * memory the field's 1e8 paths take 64.4 / 65.6 ms, without 63.4; beam-down,
+ * 6e7, 89.6 / 90.8 and 87.9. */
 constexpr int STACK_SIZE = 32;
-constexpr int SMEM_STACK = 3;
 
-/* Closest accepted hit, or the first accepted hit when `any` (shadow rays).
- * Deferred node i < SMEM_STACK of this thread is stack[i * stride] in shared
- * memory, deeper ones go to `spill`. */
+/* Closest accepted hit, or the first accepted hit when `any` (shadow rays) */
 template<class R, int FEAT = FEAT_ALL>
 __device__ bool trace_ray
   (const DScene<R>& S, V3<R> o, V3<R> d, R tmin, const SelfInfo& self,
-   bool any, Hit<R>& best, Counters& cnt, int* stack, int stride)
+   bool any, Hit<R>& best, Counters& cnt)
 {
   if(!(FEAT & FEAT_NOCOUNT)) ++cnt.rays;
   /* A zero direction component would make lo * inv - o * inv an inf - inf
@@ -691,7 +685,7 @@ __device__ bool trace_ray
   const Shear<R> sh = make_shear(d);
   best.t = rmax<R>();
   bool found = false;
-  int spill[STACK_SIZE - SMEM_STACK];
+  int stack[STACK_SIZE];
   int sp = 0, node = 0;
   /* The hit leaves of the node last visited, slot 0's first: primitive counts
    * and references */
@@ -720,8 +714,7 @@ __device__ bool trace_ray
       if(in0 && in1) {
         const bool first0 = te[0] <= te[1];
         const int far = first0 ? N.child[1] : N.child[0];
-        if(sp < SMEM_STACK) stack[(sp++) * stride] = far;
-        else if(sp < STACK_SIZE) spill[(sp++) - SMEM_STACK] = far;
+        stack[sp++ & (STACK_SIZE - 1)] = far;
         node = first0 ? N.child[0] : N.child[1];
       } else if(in0 || in1) {
         node = in0 ? N.child[0] : N.child[1];
@@ -729,7 +722,7 @@ __device__ bool trace_ray
         node = -1;
       } else {
         --sp;
-        node = sp < SMEM_STACK ? stack[sp * stride] : spill[sp - SMEM_STACK];
+        node = stack[sp];
       }
     }
     if(lc0 == 0) break;
@@ -758,8 +751,7 @@ __device__ bool trace_ray
 enum : int { PS_V0 = 0, PS_ABS = 6, PS_ATM = 7, PS_OTHER = 8, PS_COS = 9,
              PS_UV = 10 };
 /* Path sums a kernel variant keeps: PS_UV only with shading attributes
- * (without it three blocks of 256 threads of the plain kernel fit the SM's
- * 132 KB shared-memory configuration) */
+ */
 __host__ __device__ constexpr int ps_count(int feat)
 { return feat & FEAT_ATTRIBUTES ? 11 : 10; }
 
@@ -1646,8 +1638,8 @@ realisation_kernel
    const DControl ctl)
 {
   /* Shared memory: per-thread FP64 path sums [ps_count][blockDim], the
-   * warps' tally tiles [TILES][blockDim], the first traversal stack entries
-   * [SMEM_STACK][blockDim]; shared memory left unused goes to the L1 cache */
+   * warps' tally tiles [TILES][blockDim]; shared memory left unused goes to
+   * the L1 cache */
   extern __shared__ double2 smem[];
   __shared__ double red[MAX_BLOCK / 32][8];
   __shared__ WarpKeys keys[MAX_BLOCK / 32];
@@ -1656,8 +1648,6 @@ realisation_kernel
   const unsigned lane = tid & 31u;
   double2* tile = smem + tid;
   double* ps = reinterpret_cast<double*>(smem + TILES * bd) + tid;
-  int* stack = reinterpret_cast<int*>(reinterpret_cast<double*>(smem + TILES * bd)
-                                      + ps_count(FEAT) * bd) + tid;
   WarpKeys* wk = keys + (tid >> 5);
   for(int k = 0; k < TILES; ++k) tile[k * bd] = make_double2(0.0, 0.0);
   if(lane == 0) *wk = {0, 0, -1, -1};
@@ -1801,7 +1791,7 @@ realisation_kernel
       self.side = p.side;
       self.discard_virtual = shadow;
       self.reversed = shadow;
-      found = trace_ray<R, FEAT>(S, p.org, p.rd, p.tmin, self, shadow, h, cnt, stack, bd);
+      found = trace_ray<R, FEAT>(S, p.org, p.rd, p.tmin, self, shadow, h, cnt);
     }
 
     int end = END_NONE;
@@ -1927,8 +1917,6 @@ batch_kernel
   const unsigned lane = tid & 31u;
   double2* tile = smem + tid;
   double* ps = reinterpret_cast<double*>(smem + TILES * bd) + tid;
-  int* stack = reinterpret_cast<int*>(reinterpret_cast<double*>(smem + TILES * bd)
-                                      + ps_count(FEAT) * bd) + tid;
   WarpKeys* wk = keys + (tid >> 5);
   for(int k = 0; k < TILES; ++k) tile[k * bd] = make_double2(0.0, 0.0);
   if(lane == 0) *wk = {-1, -1, -1, -1};
@@ -1938,8 +1926,7 @@ batch_kernel
    * their scene from shared memory instead of device memory. Tags change
    * only where the warp is converged. */
   DScene<R>* wscene = reinterpret_cast<DScene<R>*>(
-    reinterpret_cast<int*>(reinterpret_cast<double*>(smem + TILES * bd) + ps_count(FEAT) * bd)
-    + SMEM_STACK * bd) + (size_t)(tid >> 5) * 2;
+    reinterpret_cast<double*>(smem + TILES * bd) + ps_count(FEAT) * bd) + (size_t)(tid >> 5) * 2;
   __syncwarp();
   int stag[2] = {-1, -1};
   int cur = 0;
@@ -2085,7 +2072,7 @@ batch_kernel
       self.side = p.side;
       self.discard_virtual = shadow;
       self.reversed = shadow;
-      found = trace_ray<R, FEAT>(S, p.org, p.rd, p.tmin, self, shadow, h, cnt, stack, bd);
+      found = trace_ray<R, FEAT>(S, p.org, p.rd, p.tmin, self, shadow, h, cnt);
     }
 
     int end = END_NONE;
@@ -2392,11 +2379,10 @@ template<class R, int MINB, bool TRACK, int FEAT> struct RealisationTag {};
 template<class R, int MINB, int FEAT> struct BatchTag {};
 
 /* Shared memory of a block of the realisation kernels: tally tiles, path
- * sums, traversal stack */
+ * sums */
 static size_t path_smem(int feat, int block)
 {
-  return (size_t)block * (TILES * sizeof(double2) + ps_count(feat) * sizeof(double)
-                          + SMEM_STACK * sizeof(int));
+  return (size_t)block * (TILES * sizeof(double2) + ps_count(feat) * sizeof(double));
 }
 
 /* Scratch and kernels of the coherent order of one chunk of a launch */

@@ -400,6 +400,7 @@ res_T render_device
     A.seed = job.seed;
     A.pixels = d_pixels;
     A.counters = (unsigned long long*)d_scratch;
+    A.features = snap.features;
     cudaEventCreate(&ev0);
     cudaEventCreate(&ev1);
     cudaEventRecord(ev0, s);

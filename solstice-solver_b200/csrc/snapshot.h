@@ -19,6 +19,7 @@ struct DeviceSnapshot {
   size_t alloc = 0; /* bytes of the device block */
   size_t bytes = 0; /* host -> device bytes */
   int precision = SSOL_B200_FP32;
+  int features = 0; /* FEAT_* bits the scene needs */
   ssolb::DScene<float> s32{};
   ssolb::DScene<double> s64{};
 };

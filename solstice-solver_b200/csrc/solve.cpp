@@ -691,6 +691,7 @@ res_T ssolb_snapshot_create
   }
   res = device_bind(scn->dev);
   if(res != RES_OK) return res;
+  out.features = f32 ? f32->meta.features : f64->meta.features;
   res = f32 ? snapshot_upload(scn->dev, *f32, out.s32, out)
             : snapshot_upload(scn->dev, *f64, out.s64, out);
   if(res != RES_OK) ssolb_snapshot_release(scn->dev, out);
