@@ -45,14 +45,17 @@ enum ssol_b200_precision {
  *    which do not know how many realisations they will trace, use the SAH
  *    builder.
  * Both trees find the same closest hits; only the time to build them and to
- * traverse them differs. Batches and the renderers always use the SAH
- * builder. */
+ * traverse them differs. Batches always use the SAH builder. The renderers
+ * use the device builder by default for images of at most
+ * SSOL_B200_BVH_AUTO_MAX_SAMPLES camera samples (with leaves of one
+ * primitive), the SAH builder above. */
 enum ssol_b200_bvh_builder {
   SSOL_B200_BVH_AUTO = 0,
   SSOL_B200_BVH_SAH = 1,
   SSOL_B200_BVH_LBVH = 2
 };
 #define SSOL_B200_BVH_AUTO_MAX_PATHS (1ull << 24)
+#define SSOL_B200_BVH_AUTO_MAX_SAMPLES (1ull << 27)
 
 struct ssol_b200_options {
   enum ssol_b200_precision precision;

@@ -5,8 +5,7 @@
  *
  * It replaces, on the device, the per-solve Star-3D view build of the
  * reference (src/ssol_scene.c:347-433, s3d_scene_view_create at :410-413).
- * Seven steps on one stream; the host reads the height histogram back once,
- * to size the per-height launches:
+ * Seven steps on one stream, without a read-back between them:
  *   1. centroid bounds of the primitive boxes (one block);
  *   2. 30-bit Morton code of each centroid in those bounds (10 bits per axis);
  *   3. stable LSD radix sort of (code, primitive) pairs, 4 passes of 8 bits,
@@ -25,12 +24,15 @@
  *      stops, so no thread waits on another. The same walk computes each
  *      node's SAH cost, height and internal-node count;
  *   6. treelet restructuring for a lower SAH cost (Karras and Aila, HPG
- *      2013): the nodes grouped by height, then one launch per height, lowest
- *      first, one warp per node, whose lanes share the dynamic program over
- *      the treelet's leaf subsets; the root's height is the tree depth, which
- *      the host reads back to check the traversal stack bound;
+ *      2013): the nodes grouped by height, lowest first, one warp per node,
+ *      whose lanes share the dynamic program over the treelet's leaf subsets;
+ *      one launch for each of the lower heights and one block for the rest;
+ *      the root's height is the tree depth, which the host reads back to check
+ *      the traversal stack bound;
  *   7. the internal nodes are renumbered depth first, slot 0 first, so that
  *      a node's first child follows it in memory.
+ * Scenes of at most SMALL_BUILD primitives go through all of them in one
+ * launch.
  */
 #include "kernels.h"
 
@@ -67,9 +69,11 @@ __device__ __forceinline__ R centroid(const R* box, int i, int c)
   return (R)0.5 * (box[6 * i + c] + box[6 * i + 3 + c]);
 }
 
-/* Step 1: bounds of the centroids, one block */
+/* Steps 1 to 3 run in one block of SORT_THREADS threads */
+
+/* Step 1: bounds of the centroids */
 template<class R>
-__global__ void __launch_bounds__(SORT_THREADS) lbvh_bounds(const R* box, int n, R* cb)
+__device__ __forceinline__ void lbvh_bounds(const R* box, int n, R* cb)
 {
   __shared__ R red[6][SORT_WARPS];
   R lo[3], hi[3];
@@ -106,27 +110,27 @@ __global__ void __launch_bounds__(SORT_THREADS) lbvh_bounds(const R* box, int n,
 
 /* Step 2: Morton codes; vals are the primitives' input positions */
 template<class R>
-__global__ void lbvh_morton(const R* box, int n, const R* cb, uint32_t* keys, uint32_t* vals)
+__device__ __forceinline__ void lbvh_morton(const R* box, int n, const R* cb, uint32_t* keys,
+                                            uint32_t* vals)
 {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if(i >= n) return;
-  uint32_t q[3];
-  for(int c = 0; c < 3; ++c) {
-    const R ext = cb[3 + c] - cb[c];
-    const R t = ext > (R)0 ? (centroid(box, i, c) - cb[c]) / ext : (R)0;
-    const R s = t * (R)1024;
-    q[c] = s <= (R)0 ? 0u : s >= (R)1023 ? 1023u : (uint32_t)s;
+  for(int i = threadIdx.x; i < n; i += SORT_THREADS) {
+    uint32_t q[3];
+    for(int c = 0; c < 3; ++c) {
+      const R ext = cb[3 + c] - cb[c];
+      const R t = ext > (R)0 ? (centroid(box, i, c) - cb[c]) / ext : (R)0;
+      const R s = t * (R)1024;
+      q[c] = s <= (R)0 ? 0u : s >= (R)1023 ? 1023u : (uint32_t)s;
+    }
+    keys[i] = (spread3(q[0]) << 2) | (spread3(q[1]) << 1) | spread3(q[2]);
+    vals[i] = (uint32_t)i;
   }
-  keys[i] = (spread3(q[0]) << 2) | (spread3(q[1]) << 1) | spread3(q[2]);
-  vals[i] = (uint32_t)i;
 }
 
-/* Step 3: stable radix sort in one block; (k0, v0) in and out, (k1, v1)
- * scratch */
-__global__ void __launch_bounds__(SORT_THREADS) lbvh_sort
-  (uint32_t* k0, uint32_t* v0, uint32_t* k1, uint32_t* v1, int n)
+/* Step 3: stable radix sort; (k0, v0) in and out, (k1, v1) scratch;
+ * wcnt: SORT_WARPS x 256 words of shared memory */
+__device__ __forceinline__ void lbvh_sort
+  (uint32_t (*wcnt)[256], uint32_t* k0, uint32_t* v0, uint32_t* k1, uint32_t* v1, int n)
 {
-  __shared__ uint32_t wcnt[SORT_WARPS][256];
   __shared__ uint32_t base[256];
   __shared__ uint32_t tile_total[256];
   const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
@@ -202,11 +206,10 @@ __device__ __forceinline__ int lcp(const uint32_t* k, int n, int i, int j)
 /* Step 4: internal node i of n - 1. parent[] holds (parent << 1) | slot:
  * entries [0, n - 1) for internal nodes, [n - 1, 2n - 1) for leaves. */
 template<class R>
-__global__ void lbvh_nodes(const uint32_t* keys, const uint32_t* vals, const uint32_t* ref,
-                           int n, DNode<R>* nodes, int32_t* parent)
+__device__ __forceinline__ void lbvh_node(const uint32_t* keys, const uint32_t* vals,
+                                          const uint32_t* ref, int n, int i, DNode<R>* nodes,
+                                          int32_t* parent)
 {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if(i >= n - 1) return;
   const int d = lcp(keys, n, i, i + 1) - lcp(keys, n, i, i - 1) > 0 ? 1 : -1;
   const int dmin = lcp(keys, n, i, i - d);
   int lmax = 2;
@@ -306,6 +309,30 @@ __device__ __forceinline__ void read_slot(const DNode<R>& N, int k, const Aux& A
   }
 }
 
+/* Both slots of a node by the warp, 8 lanes a slot: two loads one after the
+ * other (the slot, then what is known of its subtree) instead of 22 */
+template<class R>
+__device__ __forceinline__ void read_slots(const DNode<R>& N, const Aux& A, TLeaf<R>& L0,
+                                           TLeaf<R>& L1, int lane)
+{
+  const int k = lane >> 3, f = lane & 7;
+  TLeaf<R>& L = k ? L1 : L0;
+  if(lane < 16) {
+    if(f < 3) L.lo[f] = __ldcg(&N.lo[k][f]);
+    else if(f < 6) L.hi[f - 3] = __ldcg(&N.hi[k][f - 3]);
+    else if(f == 6) L.child = __ldcg(&N.child[k]);
+    else L.count = __ldcg(&N.count[k]);
+  }
+  __syncwarp();
+  if(lane < 16) {
+    const bool inner = L.count == 0;
+    if(f == 0) L.cost = inner ? __ldcg(&A.cost[L.child]) : C_PRIM * half_area(L.lo, L.hi);
+    else if(f == 1) L.height = inner ? __ldcg(&A.height[L.child]) : 0;
+    else if(f == 2) L.ninner = inner ? __ldcg(&A.ninner[L.child]) : 0;
+  }
+  __syncwarp();
+}
+
 template<class R>
 __device__ __forceinline__ void union_of(const TLeaf<R>* L, int S, R lo[3], R hi[3])
 {
@@ -318,59 +345,74 @@ __device__ __forceinline__ void union_of(const TLeaf<R>* L, int S, R lo[3], R hi
       }
 }
 
+/* The new internal nodes of a treelet: the leaf subset and node index of
+ * each, and its two children (another of them, or -1 - leaf) */
+struct Rebuilt {
+  int cnt, nset[TREELET - 1], nidx[TREELET - 1], kid[TREELET - 1][2];
+};
+
 /* Rewrite the internal nodes of a treelet (root first, then inner[1..]) to
  * the binary tree over its nl leaves that part[] describes (part[S]: the
  * subset holding S's lowest leaf), and set their parent links, costs (c[]),
  * heights and internal node counts. The root keeps its index and box; the
- * leaves' subtrees are untouched. */
+ * leaves' subtrees are untouched. Lane 0 lays the tree out, then one lane
+ * writes each slot. */
 template<class R>
-__device__ void rebuild_treelet(DNode<R>* nodes, const Aux& A, const TLeaf<R>* L, int nl,
-                                const int* inner, const float* c, const uint8_t* part)
+__device__ __forceinline__ void rebuild_treelet
+  (DNode<R>* nodes, const Aux& A, const TLeaf<R>* L, int nl, const int* inner, const float* c,
+   const uint8_t* part, Rebuilt& B, int lane)
 {
-  int nset[TREELET - 1], nidx[TREELET - 1], kid[TREELET - 1][2];
-  int hh[TREELET - 1], nn[TREELET - 1];
-  int cnt = 1, next = 1;
-  nset[0] = (1 << nl) - 1;
-  nidx[0] = inner[0];
-  for(int q = 0; q < cnt; ++q) {
-    const int nd = nidx[q];
-    DNode<R>& N = nodes[nd];
-    const int S = nset[q];
-    const int T[2] = {part[S], S ^ part[S]};
-    for(int k = 0; k < 2; ++k) {
-      R lo[3], hi[3];
-      if(__popc(T[k]) == 1) {
-        const int i = __ffs(T[k]) - 1;
-        put_slot(N, k, L[i].lo, L[i].hi);
-        N.child[k] = L[i].child;
-        N.count[k] = L[i].count;
-        if(L[i].count == 0) A.parent[L[i].child] = (nd << 1) | k;
-        kid[q][k] = -1 - i;
-      } else {
-        const int m = inner[next++];
-        union_of(L, T[k], lo, hi);
-        put_slot(N, k, lo, hi);
-        N.child[k] = m;
-        N.count[k] = 0;
-        A.parent[m] = (nd << 1) | k;
-        nset[cnt] = T[k];
-        nidx[cnt] = m;
-        kid[q][k] = cnt++;
+  if(lane == 0) {
+    int cnt = 1;
+    B.nset[0] = (1 << nl) - 1;
+    B.nidx[0] = inner[0];
+    for(int q = 0; q < cnt; ++q)
+      for(int k = 0; k < 2; ++k) {
+        const int S = B.nset[q], T = k ? S ^ part[S] : part[S];
+        if(__popc(T) == 1) {
+          B.kid[q][k] = -__ffs(T);
+        } else {
+          B.nset[cnt] = T;
+          B.nidx[cnt] = inner[cnt];
+          B.kid[q][k] = cnt++;
+        }
       }
+    B.cnt = cnt;
+  }
+  __syncwarp();
+  if(lane < 2 * B.cnt) {
+    const int q = lane >> 1, k = lane & 1, nd = B.nidx[q], e = B.kid[q][k];
+    DNode<R>& N = nodes[nd];
+    if(e < 0) {
+      const TLeaf<R>& leaf = L[-1 - e];
+      put_slot(N, k, leaf.lo, leaf.hi);
+      N.child[k] = leaf.child;
+      N.count[k] = leaf.count;
+      if(leaf.count == 0) A.parent[leaf.child] = (nd << 1) | k;
+    } else {
+      R lo[3], hi[3];
+      union_of(L, B.nset[e], lo, hi);
+      put_slot(N, k, lo, hi);
+      N.child[k] = B.nidx[e];
+      N.count[k] = 0;
+      A.parent[B.nidx[e]] = (nd << 1) | k;
     }
   }
-  for(int q = cnt - 1; q >= 0; --q) {
-    int hm = 0, sum = 1;
-    for(int k = 0; k < 2; ++k) {
-      const int e = kid[q][k];
-      hm = max(hm, e >= 0 ? hh[e] : L[-1 - e].height);
-      sum += e >= 0 ? nn[e] : L[-1 - e].ninner;
+  if(lane == 0) {
+    int hh[TREELET - 1], nn[TREELET - 1];
+    for(int q = B.cnt - 1; q >= 0; --q) {
+      int hm = 0, sum = 1;
+      for(int k = 0; k < 2; ++k) {
+        const int e = B.kid[q][k];
+        hm = max(hm, e >= 0 ? hh[e] : L[-1 - e].height);
+        sum += e >= 0 ? nn[e] : L[-1 - e].ninner;
+      }
+      hh[q] = 1 + hm;
+      nn[q] = sum;
+      A.cost[B.nidx[q]] = c[B.nset[q]];
+      A.height[B.nidx[q]] = hh[q];
+      A.ninner[B.nidx[q]] = nn[q];
     }
-    hh[q] = 1 + hm;
-    nn[q] = sum;
-    A.cost[nidx[q]] = c[nset[q]];
-    A.height[nidx[q]] = hh[q];
-    A.ninner[nidx[q]] = nn[q];
   }
 }
 
@@ -379,7 +421,7 @@ constexpr int MAX_LEVELS = 128;
 /* Internal nodes grouped by height (one block): level_first[h] .. [h + 1]
  * of level_nodes; *maxh the largest height present. Nodes of one height
  * are never ancestors of one another, so their treelets are disjoint. */
-__global__ void __launch_bounds__(SORT_THREADS) lbvh_levels
+__device__ __forceinline__ void lbvh_levels
   (const int32_t* height, int m, int32_t* level_first, int32_t* level_nodes, int32_t* maxh)
 {
   __shared__ uint32_t cnt[MAX_LEVELS], cur[MAX_LEVELS];
@@ -408,108 +450,175 @@ __global__ void __launch_bounds__(SORT_THREADS) lbvh_levels
 
 constexpr int TREELET_WARPS = 4;
 
+/* Shared memory of a warp's treelet */
+template<class R> struct TreeletScratch {
+  TLeaf<R> L[TREELET];
+  float c[1 << TREELET]; /* cost of the best tree over a leaf subset */
+  float area[1 << TREELET]; /* half area of its box */
+  uint8_t part[1 << TREELET];
+  int inner[TREELET - 1];
+  Rebuilt rebuilt;
+};
+
+/* The subsets of two to five of TREELET leaves, by size, and where each size
+ * starts */
+__constant__ uint8_t SUBSETS[] = {
+  3, 5, 6, 9, 10, 12, 17, 18, 20, 24, 33, 34, 36, 40, 48,
+  7, 11, 13, 14, 19, 21, 22, 25, 26, 28, 35, 37, 38, 41, 42, 44, 49, 50, 52, 56,
+  15, 23, 27, 29, 30, 39, 43, 45, 46, 51, 53, 54, 57, 58, 60,
+  31, 47, 55, 59, 61, 62};
+__constant__ uint8_t SUBSET_FIRST[] = {0, 15, 35, 50, 56};
+static_assert(TREELET == 6, "SUBSETS lists the subsets of six leaves");
+
 /* Treelet restructuring (Karras and Aila, "Fast Parallel Construction of
- * High-Quality Bounding Volume Hierarchies", HPG 2013) of the nodes of one
- * height, one warp per node, heights in increasing order (one launch each),
- * so that a node's subtree is final when its treelet is formed. Lane 0
- * refreshes the node's cost, height and node count from its slots (its
- * descendants may have changed), then grows a treelet of up to TREELET
- * leaves by opening the leaf of largest area that is a subtree; the lanes
- * then find the binary tree over those leaves of lowest SAH cost by dynamic
- * programming over their subsets, all subsets of one size at a time; lane 0
- * rewrites the treelet's internal nodes to it if it is cheaper. */
+ * High-Quality Bounding Volume Hierarchies", HPG 2013) of node `root` by one
+ * warp, once its subtree is final. The node's cost, height and node count are
+ * refreshed from its slots (its descendants may have changed), and a treelet
+ * of up to TREELET leaves grown by opening the leaf of largest area that is a
+ * subtree; the lanes then find the binary tree over those leaves of lowest
+ * SAH cost by dynamic programming over their subsets, all subsets of one size
+ * at a time, and rewrite the treelet's internal nodes to it if it is cheaper.
+ * Bound by the chain of loads and shared-memory steps of one warp, so the
+ * boxes of all subsets are formed first, the lanes of a step hold one subset
+ * each, and the partitions of the whole set are spread over the lanes: a
+ * height of few nodes takes 12 to 19 us, and took 30 with a lane going
+ * through its subsets one after the other. */
+template<class R>
+__device__ __forceinline__ void restructure
+  (DNode<R>* nodes, const Aux& A, int root, int32_t* depth, TreeletScratch<R>& M, int lane)
+{
+  TLeaf<R>* L = M.L;
+  float* c = M.c;
+  uint8_t* part = M.part;
+  read_slots(nodes[root], A, L[0], L[1], lane);
+  R lo[3], hi[3];
+  union_of(L, 3, lo, hi);
+  const float cur = C_NODE * half_area(lo, hi) + L[0].cost + L[1].cost;
+  if(lane == 0) {
+    const int h = 1 + max(L[0].height, L[1].height);
+    A.cost[root] = cur;
+    A.height[root] = h;
+    A.ninner[root] = 1 + L[0].ninner + L[1].ninner;
+    if(root == 0) *depth = h;
+    M.inner[0] = root;
+  }
+  int nl = 2, ni = 1;
+  while(nl < TREELET) {
+    /* the subtree of largest area, the first of equal ones */
+    unsigned key = 0;
+    if(lane < nl && L[lane].count == 0)
+      key = __float_as_uint(half_area(L[lane].lo, L[lane].hi)) + 1u;
+    const unsigned top = __reduce_max_sync(0xffffffffu, key);
+    if(top == 0u) break;
+    const int best = __ffs(__ballot_sync(0xffffffffu, key == top)) - 1;
+    const int nd = L[best].child;
+    if(lane == 0) M.inner[ni] = nd;
+    ++ni;
+    __syncwarp();
+    read_slots(nodes[nd], A, L[best], L[nl], lane);
+    ++nl;
+  }
+  __syncwarp();
+  if(nl >= 3) {
+    const int full = (1 << nl) - 1;
+    for(int S = lane + 1; S <= full; S += 32) {
+      for(int k = 0; k < 3; ++k) { lo[k] = rmax<R>(); hi[k] = -rmax<R>(); }
+#pragma unroll
+      for(int i = 0; i < TREELET; ++i)
+        if((S >> i) & 1)
+          for(int k = 0; k < 3; ++k) {
+            lo[k] = fmin(lo[k], L[i].lo[k]);
+            hi[k] = fmax(hi[k], L[i].hi[k]);
+          }
+      M.area[S] = half_area(lo, hi);
+      if((S & (S - 1)) == 0) c[S] = L[__ffs(S) - 1].cost;
+    }
+    __syncwarp();
+    for(int k = 0; k < 4; ++k) {
+      const int i = SUBSET_FIRST[k] + lane;
+      const int S = i < SUBSET_FIRST[k + 1] ? SUBSETS[i] : full;
+      if(S < full) {
+        /* each partition once: the part holding S's lowest leaf */
+        const int low = S & -S, others = S ^ low;
+        float bc = 3.4e38f;
+        int bp = low;
+        for(int Q = others;;) {
+          Q = (Q - 1) & others;
+          const int P = Q | low;
+          const float v = c[P] + c[S ^ P];
+          if(v < bc) { bc = v; bp = P; }
+          if(Q == 0) break;
+        }
+        c[S] = C_NODE * M.area[S] + bc;
+        part[S] = (uint8_t)bp;
+      }
+      __syncwarp();
+    }
+    /* The whole set: one of its partitions per lane */
+    {
+      const int P = 2 * lane + 1;
+      float v = P < full ? c[P] + c[full ^ P] : 3.4e38f;
+      int bp = P;
+      for(int o = 16; o > 0; o >>= 1) {
+        const float u = __shfl_xor_sync(0xffffffffu, v, o);
+        const int q = __shfl_xor_sync(0xffffffffu, bp, o);
+        if(u < v || (u == v && q > bp)) { v = u; bp = q; }
+      }
+      if(lane == 0) {
+        c[full] = C_NODE * M.area[full] + v;
+        part[full] = (uint8_t)bp;
+      }
+      __syncwarp();
+    }
+    if(c[full] < cur * (1.f - 1e-5f)) {
+      rebuild_treelet(nodes, A, L, nl, M.inner, c, part, M.rebuilt, lane);
+      if(lane == 0 && root == 0) *depth = A.height[0];
+    }
+  }
+  __syncwarp();
+}
+
+/* The nodes of one height, one warp per node: heights in increasing order,
+ * so that a node's subtree is final when its treelet is formed. Trees of
+ * MAX_LEVELS heights or more are left as they are. */
 template<class R>
 __global__ void __launch_bounds__(32 * TREELET_WARPS) lbvh_treelets
   (DNode<R>* nodes, const Aux A, const int32_t* level_first, const int32_t* level_nodes,
    int level, int32_t* depth)
 {
-  __shared__ TLeaf<R> Ls[TREELET_WARPS][TREELET];
-  __shared__ float cs[TREELET_WARPS][1 << TREELET];
-  __shared__ uint8_t ps[TREELET_WARPS][1 << TREELET];
-  __shared__ int inner_s[TREELET_WARPS][TREELET - 1];
-  __shared__ int nl_s[TREELET_WARPS];
-  __shared__ float cur_s[TREELET_WARPS];
+  __shared__ TreeletScratch<R> scratch[TREELET_WARPS];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int maxh = level_first[MAX_LEVELS + 1];
+  if(level > maxh || maxh >= MAX_LEVELS - 1) return;
   const int first = level_first[level], count = level_first[level + 1] - first;
-  TLeaf<R>* L = Ls[w];
-  float* c = cs[w];
-  uint8_t* part = ps[w];
-  for(int t = blockIdx.x * TREELET_WARPS + w; t < count; t += gridDim.x * TREELET_WARPS) {
-    const int root = level_nodes[first + t];
-    if(lane == 0) {
-      read_slot(nodes[root], 0, A, L[0]);
-      read_slot(nodes[root], 1, A, L[1]);
-      R lo[3], hi[3];
-      union_of(L, 3, lo, hi);
-      const float cur = C_NODE * half_area(lo, hi) + L[0].cost + L[1].cost;
-      const int h = 1 + max(L[0].height, L[1].height);
-      A.cost[root] = cur;
-      A.height[root] = h;
-      A.ninner[root] = 1 + L[0].ninner + L[1].ninner;
-      if(root == 0) *depth = h;
-      int nl = 2, ni = 1;
-      inner_s[w][0] = root;
-      while(nl < TREELET) {
-        int best = -1;
-        float ba = -1.f;
-        for(int i = 0; i < nl; ++i)
-          if(L[i].count == 0) {
-            const float a = half_area(L[i].lo, L[i].hi);
-            if(a > ba) { ba = a; best = i; }
-          }
-        if(best < 0) break;
-        const int nd = L[best].child;
-        inner_s[w][ni++] = nd;
-        read_slot(nodes[nd], 1, A, L[nl]);
-        read_slot(nodes[nd], 0, A, L[best]);
-        ++nl;
-      }
-      nl_s[w] = nl;
-      cur_s[w] = cur;
-    }
-    __syncwarp();
-    const int nl = nl_s[w];
-    if(nl >= 3) {
-      const int full = (1 << nl) - 1;
-      for(int S = lane + 1; S <= full; S += 32)
-        if(__popc(S) == 1) c[S] = L[__ffs(S) - 1].cost;
-      __syncwarp();
-      for(int k = 2; k <= nl; ++k) {
-        for(int S = lane + 1; S <= full; S += 32) {
-          if(__popc(S) != k) continue;
-          R lo[3], hi[3];
-          union_of(L, S, lo, hi);
-          /* each partition once: the part holding S's lowest leaf */
-          const int low = S & -S;
-          float bc = 3.4e38f;
-          int bp = low;
-          for(int P = (S - 1) & S; P; P = (P - 1) & S) {
-            if(!(P & low)) continue;
-            const float v = c[P] + c[S ^ P];
-            if(v < bc) { bc = v; bp = P; }
-          }
-          c[S] = C_NODE * half_area(lo, hi) + bc;
-          part[S] = (uint8_t)bp;
-        }
-        __syncwarp();
-      }
-      if(lane == 0 && c[full] < cur_s[w] * (1.f - 1e-5f)) {
-        rebuild_treelet(nodes, A, L, nl, inner_s[w], c, part);
-        if(root == 0) *depth = A.height[0];
-      }
-    }
-    __syncwarp();
+  for(int t = blockIdx.x * TREELET_WARPS + w; t < count; t += gridDim.x * TREELET_WARPS)
+    restructure(nodes, A, level_nodes[first + t], depth, scratch[w], lane);
+}
+
+/* The remaining heights, whose nodes are few, in one block of `warps` warps */
+template<class R>
+__device__ __forceinline__ void treelets_from
+  (DNode<R>* nodes, const Aux& A, const int32_t* level_first, const int32_t* level_nodes,
+   int level, int32_t* depth, TreeletScratch<R>* scratch)
+{
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+  const int maxh = level_first[MAX_LEVELS + 1];
+  if(maxh >= MAX_LEVELS - 1) return;
+  for(; level <= maxh; ++level) {
+    const int first = level_first[level], count = level_first[level + 1] - first;
+    for(int t = w; t < count; t += warps)
+      restructure(nodes, A, level_nodes[first + t], depth, scratch[w], lane);
+    __syncthreads();
   }
 }
 
 /* Step 5: boxes, SAH costs, heights and internal node counts, one thread
  * per leaf; flags start at zero */
 template<class R>
-__global__ void lbvh_boxes(const R* box, const uint32_t* vals, int n, DNode<R>* nodes,
-                           const Aux A, uint32_t* flags, int32_t* depth)
+__device__ __forceinline__ void lbvh_box(const R* box, const uint32_t* vals, int n, int j,
+                                         DNode<R>* nodes, const Aux& A, uint32_t* flags,
+                                         int32_t* depth)
 {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if(j >= n) return;
   const int src = (int)vals[j];
   R lo[3], hi[3];
   for(int c = 0; c < 3; ++c) {
@@ -557,11 +666,9 @@ __global__ void lbvh_boxes(const R* box, const uint32_t* vals, int n, DNode<R>* 
  * per step plus, where the path takes slot 1, the internal nodes of the
  * slot-0 subtree it passes by */
 template<class R>
-__global__ void lbvh_order(const DNode<R>* nodes, const int32_t* parent, const int32_t* ninner,
-                           int n, int32_t* newidx)
+__device__ __forceinline__ int lbvh_index(const DNode<R>* nodes, const int32_t* parent,
+                                          const int32_t* ninner, int i)
 {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if(i >= n - 1) return;
   int x = 0, node = i;
   while(node != 0) {
     const int p = parent[node];
@@ -573,18 +680,131 @@ __global__ void lbvh_order(const DNode<R>* nodes, const int32_t* parent, const i
     }
     node = par;
   }
-  newidx[i] = x;
+  return x;
 }
 
 template<class R>
-__global__ void lbvh_permute(const DNode<R>* src, DNode<R>* dst, const int32_t* newidx, int n)
+__device__ __forceinline__ void lbvh_permute(const DNode<R>* src, DNode<R>* dst,
+                                             const int32_t* newidx, int i)
 {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if(i >= n - 1) return;
   DNode<R> N = src[i];
   for(int k = 0; k < 2; ++k)
     if(N.count[k] == 0) N.child[k] = newidx[N.child[k]];
   dst[newidx[i]] = N;
+}
+
+/* The arguments of a build, typed: the tree is built in `work` and written
+ * depth first to `nodes` */
+template<class R> struct Build {
+  int n;
+  const R* box;
+  const uint32_t* ref;
+  R* cb;
+  DNode<R>* work;
+  DNode<R>* nodes;
+  uint32_t *k0, *k1, *v0, *v1, *flags;
+  int32_t *depth, *newidx, *level_first, *level_nodes;
+  Aux aux;
+};
+
+template<class R>
+__global__ void __launch_bounds__(SORT_THREADS) lbvh_sorted(const Build<R> B)
+{
+  __shared__ uint32_t wcnt[SORT_WARPS][256];
+  lbvh_bounds(B.box, B.n, B.cb);
+  __syncthreads();
+  lbvh_morton(B.box, B.n, B.cb, B.k0, B.v0);
+  __syncthreads();
+  lbvh_sort(wcnt, B.k0, B.v0, B.k1, B.v1, B.n);
+}
+template<class R>
+__global__ void lbvh_hierarchy(const Build<R> B)
+{
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if(i >= B.n - 1) return;
+  B.flags[i] = 0;
+  lbvh_node(B.k0, B.v0, B.ref, B.n, i, B.work, B.aux.parent);
+}
+template<class R>
+__global__ void lbvh_boxes(const Build<R> B)
+{
+  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  if(j < B.n) lbvh_box(B.box, B.v0, B.n, j, B.work, B.aux, B.flags, B.depth);
+}
+template<class R>
+__global__ void __launch_bounds__(SORT_THREADS) lbvh_heights(const Build<R> B)
+{
+  lbvh_levels(B.aux.height, B.n - 1, B.level_first, B.level_nodes,
+              B.level_first + MAX_LEVELS + 1);
+}
+template<class R>
+__global__ void __launch_bounds__(SORT_THREADS) lbvh_treelets_top(const Build<R> B, int level)
+{
+  __shared__ TreeletScratch<R> scratch[SORT_WARPS];
+  treelets_from(B.work, B.aux, B.level_first, B.level_nodes, level, B.depth, scratch);
+}
+template<class R>
+__global__ void lbvh_order(const Build<R> B)
+{
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if(i < B.n - 1) B.newidx[i] = lbvh_index(B.work, B.aux.parent, B.aux.ninner, i);
+}
+template<class R>
+__global__ void lbvh_write(const Build<R> B)
+{
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if(i < B.n - 1) lbvh_permute(B.work, B.nodes, B.newidx, i);
+}
+
+/* Every step in one block, for scenes so small that the launches and the gaps
+ * between them are the build: four triangles take 112 us of plan creation
+ * with a launch per step, and 65 so; the block keeps up with the
+ * launches up to a few hundred primitives */
+constexpr int SMALL_BUILD = 512;
+template<class R>
+__global__ void __launch_bounds__(SORT_THREADS) lbvh_small(const Build<R> B, int optimize)
+{
+  /* the sort's counts, then the treelets */
+  __shared__ union Shared {
+    uint32_t wcnt[SORT_WARPS][256];
+    TreeletScratch<R> treelets[SORT_WARPS];
+  } shared;
+  const int tid = threadIdx.x, n = B.n;
+  lbvh_bounds(B.box, n, B.cb);
+  __syncthreads();
+  lbvh_morton(B.box, n, B.cb, B.k0, B.v0);
+  __syncthreads();
+  lbvh_sort(shared.wcnt, B.k0, B.v0, B.k1, B.v1, n);
+  __syncthreads();
+  if(tid < n - 1) {
+    B.flags[tid] = 0;
+    lbvh_node(B.k0, B.v0, B.ref, n, tid, B.work, B.aux.parent);
+  }
+  __syncthreads();
+  if(tid < n) lbvh_box(B.box, B.v0, n, tid, B.work, B.aux, B.flags, B.depth);
+  __syncthreads();
+  if(optimize) {
+    lbvh_levels(B.aux.height, n - 1, B.level_first, B.level_nodes,
+                B.level_first + MAX_LEVELS + 1);
+    __syncthreads();
+    treelets_from(B.work, B.aux, B.level_first, B.level_nodes, 2, B.depth,
+                  shared.treelets);
+    __syncthreads();
+  }
+  if(tid < n - 1) B.newidx[tid] = lbvh_index(B.work, B.aux.parent, B.aux.ninner, tid);
+  __syncthreads();
+  if(tid < n - 1) lbvh_permute(B.work, B.nodes, B.newidx, tid);
+}
+
+/* Heights whose nodes get a launch of their own, lowest first; a few dozen
+ * nodes are left above them (3152 primitives have 664, 368, 240, 196 and 116
+ * nodes of heights 2 to 6, and 64 of height 7). The counts stay on the
+ * device: each launch is sized by a bound and strides over what there is. */
+static int wide_levels(int n)
+{
+  int last = 6;
+  for(long long m = 3000; m < n; m *= 2) last += (last & 1) ? 2 : 1;
+  return std::min(last, MAX_LEVELS - 1);
 }
 
 template<class R>
@@ -593,47 +813,44 @@ int launch_lbvh(const LbvhArgs& A, void* stream)
   const cudaStream_t s = (cudaStream_t)stream;
   const int n = A.n;
   if(n < 2) return (int)cudaErrorInvalidValue;
-  const R* box = (const R*)A.box;
-  R* cb = (R*)A.cbounds;
-  DNode<R>* nodes = (DNode<R>*)A.nodes;
-  uint32_t* k0 = A.keys;
-  uint32_t* k1 = A.keys + n;
-  uint32_t* v0 = A.vals;
-  uint32_t* v1 = A.vals + n;
-  if(cudaMemsetAsync(A.flags, 0, sizeof(uint32_t) * (size_t)(n - 1), s) != cudaSuccess)
+  Build<R> B;
+  B.n = n;
+  B.box = (const R*)A.box;
+  B.ref = A.ref;
+  B.cb = (R*)A.cbounds;
+  B.work = (DNode<R>*)A.tmp_nodes;
+  B.nodes = (DNode<R>*)A.nodes;
+  B.k0 = A.keys;
+  B.k1 = A.keys + n;
+  B.v0 = A.vals;
+  B.v1 = A.vals + n;
+  B.flags = A.flags;
+  B.depth = A.depth;
+  B.newidx = A.newidx;
+  B.level_first = A.level_first;
+  B.level_nodes = A.level_nodes;
+  B.aux = {A.cost, A.height, A.ninner, A.parent};
+  const bool optimize = A.optimize && n >= 3;
+  if(n <= SMALL_BUILD) {
+    lbvh_small<R><<<1, SORT_THREADS, 0, s>>>(B, optimize ? 1 : 0);
     return (int)cudaGetLastError();
-  lbvh_bounds<R><<<1, SORT_THREADS, 0, s>>>(box, n, cb);
-  const unsigned g = (unsigned)((n + 255) / 256);
-  lbvh_morton<R><<<g, 256, 0, s>>>(box, n, cb, k0, v0);
-  lbvh_sort<<<1, SORT_THREADS, 0, s>>>(k0, v0, k1, v1, n);
-  lbvh_nodes<R><<<g, 256, 0, s>>>(k0, v0, A.ref, n, nodes, A.parent);
-  const Aux aux = {A.cost, A.height, A.ninner, A.parent};
-  lbvh_boxes<R><<<g, 256, 0, s>>>(box, v0, n, nodes, aux, A.flags, A.depth);
-  if(A.optimize && n >= 3) {
-    /* the heights decide how many levels to launch and how wide */
-    lbvh_levels<<<1, SORT_THREADS, 0, s>>>(A.height, n - 1, A.level_first, A.level_nodes,
-                                           A.level_first + MAX_LEVELS + 1);
-    int32_t lf[MAX_LEVELS + 2];
-    if(cudaMemcpyAsync(lf, A.level_first, sizeof(lf), cudaMemcpyDeviceToHost, s) != cudaSuccess
-    || cudaStreamSynchronize(s) != cudaSuccess)
-      return (int)cudaGetLastError();
-    const int maxh = lf[MAX_LEVELS + 1];
-    if(maxh < MAX_LEVELS - 1)
-      for(int h = 2; h <= maxh; ++h) {
-        const int cnt = lf[h + 1] - lf[h];
-        if(cnt <= 0) continue;
-        const unsigned blocks = (unsigned)std::min(
-          (cnt + TREELET_WARPS - 1) / TREELET_WARPS, 148 * 8);
-        lbvh_treelets<R><<<blocks, 32 * TREELET_WARPS, 0, s>>>(nodes, aux, A.level_first,
-                                                               A.level_nodes, h, A.depth);
-      }
   }
-  DNode<R>* tmp = (DNode<R>*)A.tmp_nodes;
-  lbvh_order<R><<<g, 256, 0, s>>>(nodes, A.parent, A.ninner, n, A.newidx);
-  lbvh_permute<R><<<g, 256, 0, s>>>(nodes, tmp, A.newidx, n);
-  if(cudaMemcpyAsync(nodes, tmp, sizeof(DNode<R>) * (size_t)(n - 1), cudaMemcpyDeviceToDevice,
-                     s) != cudaSuccess)
-    return (int)cudaGetLastError();
+  const unsigned g = (unsigned)((n + 255) / 256);
+  lbvh_sorted<R><<<1, SORT_THREADS, 0, s>>>(B);
+  lbvh_hierarchy<R><<<g, 256, 0, s>>>(B);
+  lbvh_boxes<R><<<g, 256, 0, s>>>(B);
+  if(optimize) {
+    lbvh_heights<R><<<1, SORT_THREADS, 0, s>>>(B);
+    const int wide = wide_levels(n);
+    for(int h = 2; h <= wide; ++h) {
+      const unsigned blocks = (unsigned)std::min(n / (2 * h * TREELET_WARPS) + 1, 148 * 8);
+      lbvh_treelets<R><<<blocks, 32 * TREELET_WARPS, 0, s>>>(B.work, B.aux, B.level_first,
+                                                             B.level_nodes, h, B.depth);
+    }
+    lbvh_treelets_top<R><<<1, SORT_THREADS, 0, s>>>(B, wide + 1);
+  }
+  lbvh_order<R><<<g, 256, 0, s>>>(B);
+  lbvh_write<R><<<g, 256, 0, s>>>(B);
   return (int)cudaGetLastError();
 }
 

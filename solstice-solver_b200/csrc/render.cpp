@@ -355,7 +355,8 @@ res_T render_device
     return RES_BAD_ARG;
   const size_t img_bytes = npix * 3 * sizeof(double);
   DeviceSnapshot snap;
-  res_T res = ssolb_snapshot_create(scn, options, snap);
+  const uint64_t samples = job.spp > UINT64_MAX / npix ? UINT64_MAX : (uint64_t)npix * job.spp;
+  res_T res = ssolb_snapshot_create(scn, options, samples, snap);
   if(res != RES_OK) return res;
   ssol_device* dev = scn->dev;
   const cudaStream_t s = (cudaStream_t)dev->stream;

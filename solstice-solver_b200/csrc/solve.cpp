@@ -590,11 +590,20 @@ static void add_scene(Blob& b, const FlatScene<R>& f)
 static int launch_lbvh_r(const LbvhArgs& A, void* s, float) { return launch_lbvh_f32(A, s); }
 static int launch_lbvh_r(const LbvhArgs& A, void* s, double) { return launch_lbvh_f64(A, s); }
 
+/* A snapshot in device memory */
+struct SceneBlock {
+  void* mem = nullptr;
+  size_t alloc = 0; /* bytes of the device block */
+  size_t bytes = 0; /* host -> device bytes */
+  int depth = 0; /* of a device-built BVH */
+};
+
 /* Snapshot upload; a device-built BVH is built here, after the copy, on the
  * device's stream, and its depth read back. RES_BAD_OP: the tree is deeper
- * than the traversal stack allows (the caller rebuilds on the host). */
+ * than the traversal stack allows (the caller rebuilds on the host). The
+ * block is the caller's to free, whatever the result. */
 template<class R>
-static res_T upload(ssol_b200_plan* p, const FlatScene<R>& f, DScene<R>& S)
+static res_T upload(ssol_device* dev, const FlatScene<R>& f, DScene<R>& S, SceneBlock& out)
 {
   Blob b;
   add_scene(b, f);
@@ -606,16 +615,19 @@ static res_T upload(ssol_b200_plan* p, const FlatScene<R>& f, DScene<R>& S)
     o_scratch = (b.host.size() + 255) & ~size_t(255);
     bytes = o_scratch + lbvh_scratch_bytes(nprims) + 256;
   }
-  const cudaStream_t st = (cudaStream_t)p->dev->stream;
-  if(dev_alloc(p->dev, &p->d_scene, bytes) != cudaSuccess) return RES_MEM_ERR;
-  p->scene_alloc = bytes;
-  if(cudaMemcpyAsync(p->d_scene, b.host.data(), b.host.size(),
-                     cudaMemcpyHostToDevice, st) != cudaSuccess)
+  const cudaStream_t st = (cudaStream_t)dev->stream;
+  if(dev_alloc(dev, &out.mem, bytes) != cudaSuccess) {
+    out.mem = nullptr;
+    return RES_MEM_ERR;
+  }
+  out.alloc = bytes;
+  if(cudaMemcpyAsync(out.mem, b.host.data(), b.host.size(), cudaMemcpyHostToDevice, st)
+     != cudaSuccess)
     return RES_UNKNOWN_ERR;
-  p->scene_bytes = b.host.size();
-  bind_scene(S, f, b, (unsigned char*)p->d_scene);
+  out.bytes = b.host.size();
+  bind_scene(S, f, b, (unsigned char*)out.mem);
   if(f.device_bvh) {
-    unsigned char* base = (unsigned char*)p->d_scene;
+    unsigned char* base = (unsigned char*)out.mem;
     LbvhArgs A = {};
     A.n = nprims;
     A.box = base + o_box;
@@ -628,7 +640,7 @@ static res_T upload(ssol_b200_plan* p, const FlatScene<R>& f, DScene<R>& S)
     if(cudaMemcpyAsync(&depth, A.depth, sizeof(depth), cudaMemcpyDeviceToHost, st)
        != cudaSuccess || cudaStreamSynchronize(st) != cudaSuccess)
       return RES_UNKNOWN_ERR;
-    p->bvh_depth = depth;
+    out.depth = depth;
     if(depth < 1 || depth > 30) return RES_BAD_OP;
   }
   return RES_OK;
@@ -643,27 +655,8 @@ cudaError_t ssolb_dev_alloc(ssol_device* dev, void** p, size_t bytes)
 void ssolb_dev_free(ssol_device* dev, void* p, size_t bytes)
 { dev_free(dev, p, bytes); }
 
-template<class R>
-static res_T snapshot_upload(ssol_device* dev, const FlatScene<R>& f, DScene<R>& S,
-                             DeviceSnapshot& out)
-{
-  Blob b;
-  add_scene(b, f);
-  out.alloc = b.host.size() + 256;
-  if(dev_alloc(dev, &out.d_scene, out.alloc) != cudaSuccess) {
-    out.d_scene = nullptr;
-    return RES_MEM_ERR;
-  }
-  if(cudaMemcpyAsync(out.d_scene, b.host.data(), b.host.size(), cudaMemcpyHostToDevice,
-                     (cudaStream_t)dev->stream) != cudaSuccess)
-    return RES_UNKNOWN_ERR;
-  out.bytes = b.host.size();
-  bind_scene(S, f, b, (unsigned char*)out.d_scene);
-  return RES_OK;
-}
-
 res_T ssolb_snapshot_create
-  (ssol_scene* scn, const ssol_b200_options* options, DeviceSnapshot& out)
+  (ssol_scene* scn, const ssol_b200_options* options, uint64_t samples, DeviceSnapshot& out)
 {
   out = DeviceSnapshot();
   const ssol_b200_options opt = options ? *options : SSOL_B200_OPTIONS_DEFAULT;
@@ -673,29 +666,41 @@ res_T ssolb_snapshot_create
   BvhBuildParams bp;
   bp.max_leaf = opt.bvh_leaf_size ? opt.bvh_leaf_size : 1;
   bp.threads = host_threads();
+  /* The device's tree has one primitive per leaf */
+  bp.device = opt.bvh_builder == SSOL_B200_BVH_LBVH
+    || (opt.bvh_builder == SSOL_B200_BVH_AUTO && bp.max_leaf == 1
+        && samples <= SSOL_B200_BVH_AUTO_MAX_SAMPLES);
   out.precision = opt.precision;
   std::unique_ptr<FlatScene<float>> f32;
   std::unique_ptr<FlatScene<double>> f64;
   res_T res;
-  if(opt.precision == SSOL_B200_FP32) {
-    f32.reset(new FlatScene<float>());
-    res = flatten_scene(scn, bp, *f32, true);
-  } else {
-    f64.reset(new FlatScene<double>());
-    res = flatten_scene(scn, bp, *f64, true);
+  for(;;) {
+    if(opt.precision == SSOL_B200_FP32) {
+      f32.reset(new FlatScene<float>());
+      res = flatten_scene(scn, bp, *f32, true);
+    } else {
+      f64.reset(new FlatScene<double>());
+      res = flatten_scene(scn, bp, *f64, true);
+    }
+    if(res != RES_OK) return res;
+    if(f32 ? !validate(*f32, false) : !validate(*f64, false)) {
+      scn->dev->log_error("inconsistent device scene snapshot.\n");
+      return RES_UNKNOWN_ERR;
+    }
+    res = device_bind(scn->dev);
+    if(res != RES_OK) return res;
+    out.features = f32 ? f32->meta.features : f64->meta.features;
+    SceneBlock block;
+    res = f32 ? upload(scn->dev, *f32, out.s32, block) : upload(scn->dev, *f64, out.s64, block);
+    out.d_scene = block.mem;
+    out.alloc = block.alloc;
+    out.bytes = block.bytes;
+    if(res == RES_OK) return res;
+    ssolb_snapshot_release(scn->dev, out);
+    if(res != RES_BAD_OP || !bp.device) return res;
+    scn->dev->log_warning("device BVH deeper than 30 levels; built on the host instead.\n");
+    bp.device = false;
   }
-  if(res != RES_OK) return res;
-  if(f32 ? !validate(*f32, false) : !validate(*f64, false)) {
-    scn->dev->log_error("inconsistent device scene snapshot.\n");
-    return RES_UNKNOWN_ERR;
-  }
-  res = device_bind(scn->dev);
-  if(res != RES_OK) return res;
-  out.features = f32 ? f32->meta.features : f64->meta.features;
-  res = f32 ? snapshot_upload(scn->dev, *f32, out.s32, out)
-            : snapshot_upload(scn->dev, *f64, out.s64, out);
-  if(res != RES_OK) ssolb_snapshot_release(scn->dev, out);
-  return res;
 }
 
 void ssolb_snapshot_release(ssol_device* dev, DeviceSnapshot& s)
@@ -791,13 +796,13 @@ static res_T plan_create_impl
   p->bvh_device = f32 ? f32->device_bvh : f64->device_bvh;
   p->bvh_depth = f32 ? f32->bvh.depth : f64->bvh.depth;
   p->bvh_nodes = f32 ? f32->nodes.size() : f64->nodes.size();
-  if(f32) {
-    p->meta = f32->meta;
-    res = upload(p, *f32, p->s32);
-  } else {
-    p->meta = f64->meta;
-    res = upload(p, *f64, p->s64);
-  }
+  p->meta = f32 ? f32->meta : f64->meta;
+  SceneBlock block;
+  res = f32 ? upload(p->dev, *f32, p->s32, block) : upload(p->dev, *f64, p->s64, block);
+  p->d_scene = block.mem;
+  p->scene_alloc = block.alloc;
+  p->scene_bytes = block.bytes;
+  if(p->bvh_device) p->bvh_depth = block.depth;
   if(res == RES_BAD_OP) {
     /* A device-built tree too deep for the traversal stack: the host SAH
      * builder bounds its depth */
