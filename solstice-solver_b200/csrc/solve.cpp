@@ -210,17 +210,39 @@ void ssolb_device_release_gpu(ssol_device* dev)
  ******************************************************************************/
 namespace {
 
-/* One contiguous device allocation holding several arrays */
+/* Bytes that are written before they are read: a vector would clear them
+ * first, and grow by copies, each on fresh pages */
+struct RawBytes {
+  std::unique_ptr<unsigned char[]> mem;
+  size_t bytes = 0;
+  bool alloc(size_t n)
+  {
+    mem.reset(new (std::nothrow) unsigned char[n ? n : 1]);
+    bytes = n;
+    return mem != nullptr;
+  }
+  unsigned char* data() const { return mem.get(); }
+};
+
+/* One contiguous device allocation holding several arrays, in 256-byte
+ * steps: the arrays' places first, then one copy of each into a buffer of
+ * their size. The vectors added must outlive write(). */
 struct Blob {
-  std::vector<unsigned char> host;
+  struct Part { size_t off; const void* src; size_t bytes; };
+  std::vector<Part> parts;
   std::vector<size_t> offsets;
+  size_t size = 0;
   template<class T> size_t add(const std::vector<T>& v)
   {
-    size_t off = (host.size() + 255) & ~size_t(255);
-    host.resize(off + v.size() * sizeof(T));
-    if(!v.empty()) std::memcpy(host.data() + off, v.data(), v.size() * sizeof(T));
+    const size_t off = (size + 255) & ~size_t(255);
+    size = off + v.size() * sizeof(T);
+    if(!v.empty()) parts.push_back({off, v.data(), v.size() * sizeof(T)});
     offsets.push_back(off);
     return off;
+  }
+  void write(unsigned char* dst) const
+  {
+    for(const Part& p : parts) std::memcpy(dst + p.off, p.src, p.bytes);
   }
 };
 
@@ -560,10 +582,13 @@ static bool validate(const FlatScene<R>& f, bool need_samp = true)
   return true;
 }
 
+/* (A device-built tree's nodes have no contents to copy: an empty array
+ * holds their place in the order, and the upload points it elsewhere) */
 template<class R>
 static void add_scene(Blob& b, const FlatScene<R>& f)
 {
-  b.add(f.nodes);
+  static const std::vector<DNode<R>> none;
+  b.add(f.device_bvh ? none : f.nodes);
   b.add(f.bvh.primrefs);
   b.add(f.tris);
   b.add(f.quads);
@@ -607,24 +632,27 @@ static res_T upload(ssol_device* dev, const FlatScene<R>& f, DScene<R>& S, Scene
 {
   Blob b;
   add_scene(b, f);
-  size_t o_box = 0, o_ref = 0, o_scratch = 0, bytes = b.host.size() + 256;
+  size_t o_box = 0, o_ref = 0, o_scratch = 0, bytes = b.size + 256;
   const int nprims = (int)f.prim_ref.size();
   if(f.device_bvh) {
     o_box = b.add(f.prim_box);
     o_ref = b.add(f.prim_ref);
-    o_scratch = (b.host.size() + 255) & ~size_t(255);
+    b.offsets[0] = (b.size + 255) & ~size_t(255);
+    o_scratch = (b.offsets[0] + f.nodes.size() * sizeof(DNode<R>) + 255) & ~size_t(255);
     bytes = o_scratch + lbvh_scratch_bytes(nprims) + 256;
   }
+  RawBytes host;
+  if(!host.alloc(b.size)) return RES_MEM_ERR;
+  b.write(host.data());
   const cudaStream_t st = (cudaStream_t)dev->stream;
   if(dev_alloc(dev, &out.mem, bytes) != cudaSuccess) {
     out.mem = nullptr;
     return RES_MEM_ERR;
   }
   out.alloc = bytes;
-  if(cudaMemcpyAsync(out.mem, b.host.data(), b.host.size(), cudaMemcpyHostToDevice, st)
-     != cudaSuccess)
+  if(cudaMemcpyAsync(out.mem, host.data(), b.size, cudaMemcpyHostToDevice, st) != cudaSuccess)
     return RES_UNKNOWN_ERR;
-  out.bytes = b.host.size();
+  out.bytes = b.size;
   bind_scene(S, f, b, (unsigned char*)out.mem);
   if(f.device_bvh) {
     unsigned char* base = (unsigned char*)out.mem;
@@ -977,13 +1005,16 @@ static res_T swap_sah(ssol_b200_plan* p, const FlatScene<R>& f, DScene<R>& S)
   Blob b;
   const size_t o_nodes = b.add(nodes);
   const size_t o_refs = b.add(r.primrefs);
-  const size_t bytes = b.host.size() + 256;
+  const size_t bytes = b.size + 256;
+  RawBytes host;
+  if(!host.alloc(b.size)) return RES_OK;
+  b.write(host.data());
   if(dev_alloc(p->dev, &p->d_bvh2, bytes) != cudaSuccess) {
     p->d_bvh2 = nullptr;
     return RES_OK; /* keep tracing on the device's tree */
   }
   p->bvh2_alloc = bytes;
-  if(cudaMemcpyAsync(p->d_bvh2, b.host.data(), b.host.size(), cudaMemcpyHostToDevice,
+  if(cudaMemcpyAsync(p->d_bvh2, host.data(), b.size, cudaMemcpyHostToDevice,
                      (cudaStream_t)p->dev->stream) != cudaSuccess)
     return RES_UNKNOWN_ERR;
   unsigned char* base = (unsigned char*)p->d_bvh2;
@@ -1019,7 +1050,8 @@ extern "C" res_T ssol_b200_plan_finish
 {
   if(!p || !rng || !out) return RES_BAD_ARG;
   const cudaStream_t s = plan_stream(p, stream);
-  std::vector<unsigned char> h(p->tl.total);
+  RawBytes h;
+  if(!h.alloc(p->tl.total)) return RES_MEM_ERR;
   if(cudaMemcpyAsync(h.data(), p->d_tally, p->tl.total,
                      cudaMemcpyDeviceToHost, s) != cudaSuccess)
     return RES_UNKNOWN_ERR;
@@ -1461,12 +1493,19 @@ static res_T batch_upload(ssol_b200_batch* b, std::vector<FlatScene<R>>& f)
    * device block, followed by the DScene array */
   const size_t n = f.size();
   std::vector<Blob> blobs(n);
-  parallel_for(n, [&](size_t i) { add_scene(blobs[i], f[i]); });
+  std::vector<RawBytes> host(n);
+  std::atomic<bool> room{true};
+  parallel_for(n, [&](size_t i) {
+    add_scene(blobs[i], f[i]);
+    if(host[i].alloc(blobs[i].size)) blobs[i].write(host[i].data());
+    else room = false;
+  });
+  if(!room) return RES_MEM_ERR;
   std::vector<size_t> base_off(n);
   size_t total = 0;
   for(size_t i = 0; i < n; ++i) {
     base_off[i] = total;
-    total = (total + blobs[i].host.size() + 255) & ~size_t(255);
+    total = (total + blobs[i].size + 255) & ~size_t(255);
   }
   const size_t s_off = total;
   total += n * sizeof(DScene<R>);
@@ -1480,8 +1519,8 @@ static res_T batch_upload(ssol_b200_batch* b, std::vector<FlatScene<R>>& f)
   const cudaStream_t st = (cudaStream_t)b->dev->stream;
   for(size_t i = 0; i < n; ++i) {
     bind_scene(S[i], f[i], blobs[i], base + base_off[i]);
-    if(!blobs[i].host.empty()
-    && cudaMemcpyAsync(base + base_off[i], blobs[i].host.data(), blobs[i].host.size(),
+    if(blobs[i].size
+    && cudaMemcpyAsync(base + base_off[i], host[i].data(), blobs[i].size,
                        cudaMemcpyHostToDevice, st) != cudaSuccess)
       return RES_UNKNOWN_ERR;
   }
@@ -1705,7 +1744,10 @@ static res_T tracking_upload
   Blob blob;
   add_scene(blob, f);
   const size_t ntri = f.tris.size(), nsamp = f.samp.size();
-  size_t total = (blob.host.size() + 255) & ~size_t(255);
+  RawBytes host;
+  if(!host.alloc(blob.size)) return RES_MEM_ERR;
+  blob.write(host.data());
+  size_t total = (blob.size + 255) & ~size_t(255);
   auto take = [&](size_t bytes) { const size_t o = total; total = (total + bytes + 255) & ~size_t(255); return o; };
   const size_t o_tris = take(nitems * ntri * sizeof(DTri<R>));
   const size_t o_samp = take(nitems * nsamp * sizeof(DSampTri<R>));
@@ -1733,7 +1775,7 @@ static res_T tracking_upload
     return !bytes || cudaMemcpyAsync(base + off, src, bytes, cudaMemcpyHostToDevice, st)
                        == cudaSuccess;
   };
-  bool ok = up(0, blob.host.data(), blob.host.size())
+  bool ok = up(0, host.data(), blob.size)
     && up(o_helio, helio_data.data(), helio_data.size() * sizeof(double))
     && up(o_sun, to_sun.data(), to_sun.size() * sizeof(double))
     && up(o_th, tri_helio.data(), tri_helio.size() * sizeof(int32_t))
@@ -1792,7 +1834,7 @@ static res_T tracking_upload
   if(!up(o_scenes, S.data(), nitems * sizeof(DScene<R>))
   || cudaStreamSynchronize(st) != cudaSuccess)
     return RES_UNKNOWN_ERR;
-  b->scene_bytes = blob.host.size() + local.size() * sizeof(double);
+  b->scene_bytes = blob.size + local.size() * sizeof(double);
   b->d_scenes = base + o_scenes;
   return RES_OK;
 }
