@@ -37,9 +37,10 @@ enum ssol_b200_precision {
  *    order), one primitive per leaf (bvh_leaf_size is ignored); the fastest
  *    to build. A tree deeper than the traversal stack allows (more than 30
  *    levels) is rebuilt on the host with the SAH builder, with a warning;
- *  - SSOL_B200_BVH_AUTO (the default): ssol_solve and ssol_solve_ex use the
- *    device builder for solves of at most SSOL_B200_BVH_AUTO_MAX_PATHS
- *    realisations, where building is a large part of the call. Larger solves
+ *  - SSOL_B200_BVH_AUTO (the default): ssol_solve, ssol_solve_ex and (with
+ *    leaves of one primitive) ssol_solve_adjoint use the device builder for
+ *    at most SSOL_B200_BVH_AUTO_MAX_PATHS realisations, where building is a
+ *    large part of the call. Larger solves
  *    start on the device's tree and, after their first 6e6 realisations,
  *    trace on the SAH tree that the host threads built meanwhile. Plans,
  *    which do not know how many realisations they will trace, use the SAH
