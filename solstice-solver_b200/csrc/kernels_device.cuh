@@ -231,7 +231,15 @@ __device__ __forceinline__ V3<R> sun_local_to_world(const DScene<R>& S, V3<R> p)
 }
 
 /* Buie zenith angle by rejection (src/ssol_ranst_sun_dir.c:177-195); the
- * draws of attempt k come from event 2 + k of the primary domain */
+ * draws of attempt k come from event 2 + k of the primary domain.
+ *
+ * The warp repeats the loop until its last lane accepts, and an attempt's FP64
+ * cosines, power, sine and division were a fifth of the kernel. The density
+ * in FP32 decides all but the closest attempts: its relative error is below
+ * 1e-5 (the cosines' arguments reach 1.52, where a cosine of 0.055 takes 18
+ * times the 1.2e-7 of its argument), so outside a margin of 1e-3 the FP64
+ * comparison has the same outcome, and inside it is made. Field of 317, 5.1e6
+ * paths under CSR 0.05: kernel 4.46 -> 4.10 ms. */
 static __device__ __noinline__ double buie_theta
   (double thetaSD, double dCSSD, double gamma, double ek1000g, double alpha, double h1,
    double h2, double p1, const Rng rng)
@@ -246,6 +254,16 @@ static __device__ __noinline__ double buie_theta
     } else {
       theta = thetaSD + u01d(r.v[1]) * dCSSD;
       value = u01d(r.v[2]) * h2;
+    }
+    {
+      const float t = (float)theta, v = (float)value;
+      const float phi = theta < thetaSD ? cosf(326.f * t) / cosf(308.f * t)
+                                        : (float)ek1000g * powf(t, (float)gamma);
+      const float p = (float)alpha * phi * sinf(t);
+      if(p > 1e-30f && p < 1e30f) {
+        if(v < p * 0.999f) break;
+        if(v > p * 1.001f) continue;
+      }
     }
     const double phi = theta < thetaSD
       ? cos(326 * theta) / cos(308 * theta)
