@@ -2247,16 +2247,14 @@ extern "C" res_T ssol_solve_ex
   *out = nullptr;
   if(n > (size_t)INT64_MAX || max_failed > (size_t)INT64_MAX)
     return RES_BAD_ARG;
-  /* The default builder by solve size: below the threshold, building the
-   * tree on the device saves more (2 ms on the 1000-heliostat field) than
-   * its slightly slower traversal costs */
   ssol_b200_options opt = options ? *options : SSOL_B200_OPTIONS_DEFAULT;
-  /* The default builder by solve size. Larger solves start on the device's
+  /* The default builder by solve size: below the threshold, building the
+   * tree on the device saves more (2 ms on the 1000-heliostat field) than its
+   * slightly slower traversal costs. Larger solves start on the device's
    * tree and switch to the host SAH tree, built meanwhile on the host
-   * threads, after their first 6e6 realisations (the smallest launch that
-   * runs in the coherent order, 8.5 ms on the 1000-heliostat field): the
-   * host build (2-3 ms there) no longer delays the first launch, and only
-   * that first part traces on the slower tree */
+   * threads, after their first 6e6 realisations (4 ms on that field): the
+   * host build (2-3 ms there) does not delay the first launch, and only that
+   * first part traces on the slower tree */
   const bool hybrid = opt.bvh_builder == SSOL_B200_BVH_AUTO && !tracker
     && (unsigned long long)n > SSOL_B200_BVH_AUTO_MAX_PATHS;
   if(opt.bvh_builder == SSOL_B200_BVH_AUTO)
