@@ -63,7 +63,8 @@ struct ssol_b200_options {
   int block_size; /* threads per block, <= 256; 0 => 256 */
   int grid_blocks; /* 0 => one persistent wave sized from occupancy */
   int waves; /* persistent grid multiplier when grid_blocks == 0 */
-  int bvh_leaf_size; /* primitives per BVH leaf; 0 => 1 */
+  int bvh_leaf_size; /* primitives per BVH leaf; 0 => by the scene: 2 for meshes,
+                      * 1 with punched surfaces */
   unsigned long long max_segments; /* path segment budget; 0 => 1e6 */
   int min_blocks_per_sm; /* register budget of the kernel variant: 1, 2, 3;
                           * 0 => 3 in FP32, 2 in FP64 */

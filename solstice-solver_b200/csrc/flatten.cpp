@@ -989,7 +989,9 @@ static res_T flatten_impl
     out.nodes.assign(n - 1, DNode<R>());
     return RES_OK;
   }
-  build_bvh(boxes, bvh_params, out.bvh);
+  BvhBuildParams prm = bvh_params;
+  if(prm.max_leaf == 0) prm.max_leaf = default_leaf(out);
+  build_bvh(boxes, prm, out.bvh);
   out.nodes = bvh_nodes<R>(out.bvh);
   return RES_OK;
 }

@@ -92,6 +92,17 @@ template<class R> struct FlatScene {
   int32_t air_medium = 0;
 };
 
+/* Primitives per leaf of the host's tree where the caller leaves the choice.
+ * Two for meshes: a rectangle's two triangles are one leaf, so a ray makes
+ * fewer node visits (field 40.4 for 44.3 a path) for a few more triangle
+ * tests (7.7 for 7.2), which a warp makes together. One with punched
+ * surfaces, whose test costs more than a node visit. Plan launches, leaves of
+ * 1 / 2 / 3 / 4: field of 1000, 5e7 paths, 30.8 / 29.1 / 29.1 / 30.4 ms; of
+ * 317, 2e7, 11.0 / 10.4 / 10.4 / 10.9; FP64, 5e6, 7.1 / 6.5 / 6.5 / 6.6; one
+ * mirror, 5e6, 1.36 / 1.28 / 1.28 / 1.31; beam-down, 1e7, 13.8 / 14.4 / 14.9 /
+ * 15.6. */
+template<class R> int default_leaf(const FlatScene<R>& f) { return f.quads.empty() ? 2 : 1; }
+
 /* for_draw: snapshot for the renderers, which sample no instance (no
  * "nothing to sample" error, no receiver warning) */
 res_T flatten_scene

@@ -692,11 +692,11 @@ res_T ssolb_snapshot_create
     return RES_BAD_ARG;
   if(opt.bvh_leaf_size < 0 || !builder_ok(opt.bvh_builder)) return RES_BAD_ARG;
   BvhBuildParams bp;
-  bp.max_leaf = opt.bvh_leaf_size ? opt.bvh_leaf_size : 1;
+  bp.max_leaf = opt.bvh_leaf_size;
   bp.threads = host_threads();
   /* The device's tree has one primitive per leaf */
   bp.device = opt.bvh_builder == SSOL_B200_BVH_LBVH
-    || (opt.bvh_builder == SSOL_B200_BVH_AUTO && bp.max_leaf == 1
+    || (opt.bvh_builder == SSOL_B200_BVH_AUTO && bp.max_leaf <= 1
         && samples <= SSOL_B200_BVH_AUTO_MAX_SAMPLES);
   out.precision = opt.precision;
   std::unique_ptr<FlatScene<float>> f32;
@@ -780,7 +780,6 @@ static res_T plan_create_impl
     return RES_BAD_ARG;
   if(opt.block_size == 0) opt.block_size = 256;
   if(opt.block_size % 32) return RES_BAD_ARG;
-  if(opt.bvh_leaf_size == 0) opt.bvh_leaf_size = 1;
   if(opt.max_segments == 0) opt.max_segments = 1000000ull;
   if(opt.min_blocks_per_sm < 0 || opt.min_blocks_per_sm > 3) return RES_BAD_ARG;
   if(opt.min_blocks_per_sm == 0) opt.min_blocks_per_sm = default_min_blocks(opt.precision);
@@ -996,7 +995,7 @@ static res_T swap_sah(ssol_b200_plan* p, const FlatScene<R>& f, DScene<R>& S)
     boxes[i].ref = f.prim_ref[i];
   }
   BvhBuildParams bp;
-  bp.max_leaf = 1;
+  bp.max_leaf = default_leaf(f);
   bp.threads = host_threads();
   BvhResult r;
   build_bvh(std::move(boxes), bp, r);
@@ -1558,7 +1557,6 @@ extern "C" res_T ssol_b200_batch_create
     return RES_BAD_ARG;
   if(opt.block_size == 0) opt.block_size = 256;
   if(opt.block_size % 32) return RES_BAD_ARG;
-  if(opt.bvh_leaf_size == 0) opt.bvh_leaf_size = 1;
   if(opt.max_segments == 0) opt.max_segments = 1000000ull;
   if(opt.min_blocks_per_sm == 0) opt.min_blocks_per_sm = default_min_blocks(opt.precision);
 
@@ -1863,7 +1861,6 @@ extern "C" res_T ssol_b200_batch_create_tracking
     return RES_BAD_ARG;
   if(opt.block_size == 0) opt.block_size = 256;
   if(opt.block_size % 32) return RES_BAD_ARG;
-  if(opt.bvh_leaf_size == 0) opt.bvh_leaf_size = 1;
   if(opt.max_segments == 0) opt.max_segments = 1000000ull;
   if(opt.min_blocks_per_sm == 0) opt.min_blocks_per_sm = default_min_blocks(opt.precision);
   /* Sun directions normalised as ssol_sun_set_direction does */
