@@ -39,26 +39,31 @@ WORKLOAD = ("1000 flat 10x10 heliostats (radial staggered, r 100-600 m, Beckmann
 
 
 # DRAM bytes per path of the realisation kernel, from ncu captures of launches
-# of the same scenes, the variants without work counters (field: one sorted
-# chunk of 2^24 paths at 3 blocks per SM; beam-down: 4e6 paths)
+# of the same scenes, the variants without work counters (one sorted chunk
+# of 2^24 paths each)
 # (dram__bytes_read.sum + dram__bytes_write.sum);
 # the traffic scales with the paths traced (per-thread frames written back)
-DRAM_BYTES_PER_PATH = {"field": (2202.1e6 + 15599.4e6) / 16777216,
-                       "beamdown": (892.0e6 + 3562.1e6) / 4e6}  # beam-down: id order
+DRAM_BYTES_PER_PATH = {"field": (121.6e6 + 2698.4e6) / 16777216,
+                       "beamdown": (447.9e6 + 4585.7e6) / 16777216}
 
-# Kernels of one plain launch of n realisations: below 6e6 the realisation
-# kernel alone; from 6e6 on, per chunk of at most 2^24 realisations, the
-# coherent order's presort (count, scan, scatter) and the realisation kernel
-# (every bench scene samples more than one and fewer than 12288 primitives)
-SORT_MIN, SORT_CHUNK = 6_000_000, 1 << 24
+# Kernels of one plain launch of n realisations: the realisation kernel, with
+# the coherent order's presort (count, scan, scatter) before it from SORT_MIN
+# realisations on (more with quadrics, never with one sampled mirror), per
+# chunk of at most 2^24; and the sums that follow from others, once
+SORT_MIN = {"field": 200_000, "beamdown": 1_000_000}
+SORT_CHUNK = 1 << 24
 
 
-def launches_per_plain_launch(n):
-    return 1 if n < SORT_MIN else 4 * ((n + SORT_CHUNK - 1) // SORT_CHUNK)
+def launches_per_plain_launch(n, config):
+    if n < SORT_MIN.get(config, n + 1):
+        return 2
+    return 4 * ((n + SORT_CHUNK - 1) // SORT_CHUNK) + 1
+
+
 # Both passes of the adjoint kernel on the field, from a capture of 4e6 paths
-ADJOINT_DRAM_BYTES_PER_PATH = (2.76e6 + 26.97e6 + 5.95e6 + 52.99e6) / 4e6
-# Same for the batched kernel, from a capture of 32 suns (32245124 paths)
-BATCH_DRAM_BYTES_PER_PATH = (4571.5e6 + 19782.1e6) / 32245124
+ADJOINT_DRAM_BYTES_PER_PATH = (24.6e6 + 61.1e6 + 152.2e6 + 1395.3e6) / 4e6
+# Same for the batched kernel, from a capture of 32 suns (18907863 paths)
+BATCH_DRAM_BYTES_PER_PATH = (208.5e6 + 4448.8e6) / 18907863
 
 
 def flops_per_run(st):
@@ -445,7 +450,7 @@ def run_b200(args):
         "e2e": {"value": e2e_value, "unit": METRIC, "h2d_bytes_per_step": h2d,
                 "d2h_bytes_per_step": d2h,
                 "timing": "wall clock around synchronous ssol_solve"},
-        "gpu_launches": args.steps * launches_per_plain_launch(n),
+        "gpu_launches": args.steps * launches_per_plain_launch(n, args.config),
         "roofline": {"bound": "fp32", "achieved": achieved, "peak": fp32_peak,
                      "unit": "TFLOP/s", "frac": achieved / fp32_peak if fp32_peak else None,
                      "traffic": (DRAM_BYTES_PER_PATH[args.config] * n
@@ -454,7 +459,7 @@ def run_b200(args):
                                        "realisation kernel, scaled to paths_per_step "
                                        "(bytes per step: its chunks' launches together)",
                      "timing": "CUDA events around each step: the realisation kernel and "
-                               "the coherent order's presort (2.3 % of the step)",
+                               "the coherent order's presort (1.9 % of the step)",
                      "peak_source": "SMs x 128 FP32 lanes x 2 x measured max SM clock "
                                     "(MEASURED_PEAKS.json sm_max_mhz)",
                      "work_model": "20/slab x2 per node + 55/triangle + 90/quadric + "
@@ -966,9 +971,10 @@ def run_suns(args):
         "e2e": {"value": r["paths"] / r["e2e_s"] / 1e6, "unit": METRIC,
                 "h2d_bytes_per_step": r["h2d"], "d2h_bytes_per_step": r["d2h"],
                 "timing": "wall clock: batch create + launch + finish per step"},
-        # batched launches of 2^22 to 2^29 realisations run the coherent
-        # order's presort (count, scan, scatter) before the batched kernel
-        "gpu_launches": args.steps * (4 if (1 << 22) <= r["n_total_rank"] <= (1 << 29) else 1),
+        # batched launches of 2^20 to 2^29 realisations run the coherent
+        # order's presort (count, scan, scatter) before the batched kernel,
+        # and every one the sums that follow from others after it
+        "gpu_launches": args.steps * (5 if (1 << 20) <= r["n_total_rank"] <= (1 << 29) else 2),
         "roofline": {"bound": "fp32", "achieved": achieved, "peak": fp32_peak,
                      "unit": "TFLOP/s", "frac": achieved / fp32_peak,
                      "traffic": BATCH_DRAM_BYTES_PER_PATH * r["n_total_rank"],
@@ -1093,7 +1099,8 @@ def run_adjoint(args):
         "e2e": {"value": e2e, "unit": METRIC, "h2d_bytes_per_step": None,
                 "d2h_bytes_per_step": (nx * ny + 4 * len(h["heliostats"])) * 8,
                 "timing": "wall clock around the synchronous ssol_solve_adjoint"},
-        "gpu_launches": 2 * args.steps,
+        # per pass: the presort of every chunk and the pass itself
+        "gpu_launches": 2 * args.steps * 4 * ((n + SORT_CHUNK - 1) // SORT_CHUNK),
         "roofline": {"bound": "fp32", "achieved": achieved, "peak": fp32_peak,
                      "unit": "TFLOP/s", "frac": achieved / fp32_peak,
                      "traffic": ADJOINT_DRAM_BYTES_PER_PATH * n / passes,
