@@ -34,9 +34,10 @@ enum ssol_b200_precision {
  *  - SSOL_B200_BVH_LBVH: linear BVH built on the device from the uploaded
  *    primitive boxes (Morton codes, radix sort, Karras' hierarchy, bottom-up
  *    boxes, treelet restructuring for a lower SAH cost, depth-first node
- *    order), one primitive per leaf (bvh_leaf_size is ignored); the fastest
- *    to build. A tree deeper than the traversal stack allows (more than 30
- *    levels) is rebuilt on the host with the SAH builder, with a warning;
+ *    order), one primitive per leaf, or up to two in scenes of meshes
+ *    (bvh_leaf_size is ignored); the fastest to build. A tree deeper than the
+ *    traversal stack allows (more than 30 levels) is rebuilt on the host with
+ *    the SAH builder, with a warning;
  *  - SSOL_B200_BVH_AUTO (the default): ssol_solve, ssol_solve_ex and (with
  *    leaves of one primitive) ssol_solve_adjoint use the device builder for
  *    at most SSOL_B200_BVH_AUTO_MAX_PATHS realisations, where building is a

@@ -92,7 +92,8 @@ template<class R> struct FlatScene {
   int32_t air_medium = 0;
 };
 
-/* Primitives per leaf of the host's tree where the caller leaves the choice.
+/* Primitives per leaf of the host's tree where the caller leaves the choice,
+ * and at most so many of the device's.
  * Two for meshes: a rectangle's two triangles are one leaf, so a ray makes
  * fewer node visits (field 40.4 for 44.3 a path) for a few more triangle
  * tests (7.7 for 7.2), which a warp makes together. One with punched

@@ -30,7 +30,8 @@
  *      the root's height is the tree depth, which the host reads back to check
  *      the traversal stack bound;
  *   7. the internal nodes are renumbered depth first, slot 0 first, so that
- *      a node's first child follows it in memory.
+ *      a node's first child follows it in memory; in scenes of meshes a node of
+ *      two primitives becomes a leaf of two.
  * Scenes of at most SMALL_BUILD primitives go through all of them in one
  * launch.
  */
@@ -683,13 +684,30 @@ __device__ __forceinline__ int lbvh_index(const DNode<R>* nodes, const int32_t* 
   return x;
 }
 
+/* With `pairs`, a node of two primitives becomes a leaf of two in its parent,
+ * whose references are listed at its own index (the node's place stays, unread):
+ * fewer node visits for a few more tests, which a warp makes together, as in
+ * the host's tree of mesh scenes (default_leaf). Adjoint, 1e7 paths, 13.1 ->
+ * 11.2 ms; field of 317 under Buie's sun, 5.1e6, 5.96 -> 5.79; FP64 field, 2e6,
+ * 3.73 -> 3.53; one mirror, 1e6, 0.405 -> 0.389; path-traced view 8.2 -> 7.8. */
 template<class R>
 __device__ __forceinline__ void lbvh_permute(const DNode<R>* src, DNode<R>* dst,
-                                             const int32_t* newidx, int i)
+                                             const int32_t* newidx, uint32_t* pairs, int i)
 {
   DNode<R> N = src[i];
-  for(int k = 0; k < 2; ++k)
-    if(N.count[k] == 0) N.child[k] = newidx[N.child[k]];
+  for(int k = 0; k < 2; ++k) {
+    if(N.count[k] != 0) continue;
+    const DNode<R>& C = src[N.child[k]];
+    const int at = newidx[N.child[k]];
+    if(pairs && C.count[0] == 1 && C.count[1] == 1) {
+      pairs[2 * at] = (uint32_t)C.child[0];
+      pairs[2 * at + 1] = (uint32_t)C.child[1];
+      N.count[k] = 2;
+      N.child[k] = 2 * at;
+    } else {
+      N.child[k] = at;
+    }
+  }
   dst[newidx[i]] = N;
 }
 
@@ -702,6 +720,7 @@ template<class R> struct Build {
   R* cb;
   DNode<R>* work;
   DNode<R>* nodes;
+  uint32_t* pairs;
   uint32_t *k0, *k1, *v0, *v1, *flags;
   int32_t *depth, *newidx, *level_first, *level_nodes;
   Aux aux;
@@ -753,7 +772,7 @@ template<class R>
 __global__ void lbvh_write(const Build<R> B)
 {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if(i < B.n - 1) lbvh_permute(B.work, B.nodes, B.newidx, i);
+  if(i < B.n - 1) lbvh_permute(B.work, B.nodes, B.newidx, B.pairs, i);
 }
 
 /* Every step in one block, for scenes so small that the launches and the gaps
@@ -793,7 +812,7 @@ __global__ void __launch_bounds__(SORT_THREADS) lbvh_small(const Build<R> B, int
   }
   if(tid < n - 1) B.newidx[tid] = lbvh_index(B.work, B.aux.parent, B.aux.ninner, tid);
   __syncthreads();
-  if(tid < n - 1) lbvh_permute(B.work, B.nodes, B.newidx, tid);
+  if(tid < n - 1) lbvh_permute(B.work, B.nodes, B.newidx, B.pairs, tid);
 }
 
 /* Heights whose nodes get a launch of their own, lowest first; a few dozen
@@ -820,6 +839,7 @@ int launch_lbvh(const LbvhArgs& A, void* stream)
   B.cb = (R*)A.cbounds;
   B.work = (DNode<R>*)A.tmp_nodes;
   B.nodes = (DNode<R>*)A.nodes;
+  B.pairs = A.pairs;
   B.k0 = A.keys;
   B.k1 = A.keys + n;
   B.v0 = A.vals;

@@ -632,13 +632,16 @@ static res_T upload(ssol_device* dev, const FlatScene<R>& f, DScene<R>& S, Scene
 {
   Blob b;
   add_scene(b, f);
-  size_t o_box = 0, o_ref = 0, o_scratch = 0, bytes = b.size + 256;
+  size_t o_box = 0, o_ref = 0, o_pairs = 0, o_scratch = 0, bytes = b.size + 256;
   const int nprims = (int)f.prim_ref.size();
   if(f.device_bvh) {
     o_box = b.add(f.prim_box);
     o_ref = b.add(f.prim_ref);
     b.offsets[0] = (b.size + 255) & ~size_t(255);
-    o_scratch = (b.offsets[0] + f.nodes.size() * sizeof(DNode<R>) + 255) & ~size_t(255);
+    o_pairs = (b.offsets[0] + f.nodes.size() * sizeof(DNode<R>) + 255) & ~size_t(255);
+    o_scratch = o_pairs;
+    if(default_leaf(f) == 2)
+      o_scratch = (o_pairs + 2 * f.nodes.size() * sizeof(uint32_t) + 255) & ~size_t(255);
     bytes = o_scratch + lbvh_scratch_bytes(nprims) + 256;
   }
   RawBytes host;
@@ -662,6 +665,10 @@ static res_T upload(ssol_device* dev, const FlatScene<R>& f, DScene<R>& S, Scene
     A.ref = (const uint32_t*)(base + o_ref);
     A.nodes = base + b.offsets[0];
     A.optimize = 1;
+    if(o_scratch != o_pairs) {
+      A.pairs = (uint32_t*)(base + o_pairs);
+      S.primrefs = A.pairs;
+    }
     lbvh_bind_scratch(A, base + o_scratch);
     if(launch_lbvh_r(A, st, R()) != 0) return RES_UNKNOWN_ERR;
     int32_t depth = 0;
@@ -694,7 +701,7 @@ res_T ssolb_snapshot_create
   BvhBuildParams bp;
   bp.max_leaf = opt.bvh_leaf_size;
   bp.threads = host_threads();
-  /* The device's tree has one primitive per leaf */
+  /* The device's tree does not take the caller's leaf size */
   bp.device = opt.bvh_builder == SSOL_B200_BVH_LBVH
     || (opt.bvh_builder == SSOL_B200_BVH_AUTO && bp.max_leaf <= 1
         && samples <= SSOL_B200_BVH_AUTO_MAX_SAMPLES);
@@ -1096,7 +1103,7 @@ extern "C" res_T ssol_b200_autotune
   ssol_b200_options best_opt = base;
   double best = DBL_MAX;
   for(const int leaf : leaves) {
-    /* a device-built tree has one primitive per leaf */
+    /* a device-built tree does not take the leaf size */
     if(base.bvh_builder == SSOL_B200_BVH_LBVH && leaf != 1) continue;
     ssol_b200_options o = base;
     o.bvh_leaf_size = leaf;
