@@ -207,6 +207,13 @@ enum : int32_t {
   FEAT_NOCOUNT = 8
 };
 
+/* Kernel variants that keep to DScene::own_boxes: FP32 without quadrics or
+ * dielectrics, and FP32 with everything */
+template<class R, int FEAT> struct OwnBoxes {
+  static constexpr bool value = sizeof(R) == sizeof(float)
+    && (!(FEAT & (FEAT_QUADRIC | FEAT_DIELECTRIC)) || (FEAT & FEAT_ATTRIBUTES));
+};
+
 /* Counters for the roofline model (see kernels_device.cuh) */
 struct DStats {
   unsigned long long rays;
@@ -237,6 +244,9 @@ template<typename R> struct DScene {
   /* Some material, medium or baked shader depends on the wavelength; the
    * paths of a scene without any need not sample theirs */
   int32_t spectral;
+  /* A triangle in a leaf of several counts as hit only where its own box is
+   * hit too (trace_ray) */
+  int32_t own_boxes;
 
   const DSampTri<R>* samp;
   const float* alias_prob;

@@ -466,6 +466,7 @@ static void bind_scene(DScene<R>& S, const FlatScene<R>& f, const Blob& b,
   for(const DMaterial& m : f.mtls) S.spectral |= m.uniform != 3;
   for(const DMedium& m : f.media)
     S.spectral |= m.extinction.spectrum >= 0 || m.refractive_index.spectrum >= 0;
+  S.own_boxes = f.own_boxes;
   S.nsamp = (int32_t)f.samp.size();
   S.sun_type = f.sun_type;
   for(int c = 0; c < 3; ++c) S.sun_dir[c] = f.sun_dir[c];
@@ -640,7 +641,7 @@ static res_T upload(ssol_device* dev, const FlatScene<R>& f, DScene<R>& S, Scene
     b.offsets[0] = (b.size + 255) & ~size_t(255);
     o_pairs = (b.offsets[0] + f.nodes.size() * sizeof(DNode<R>) + 255) & ~size_t(255);
     o_scratch = o_pairs;
-    if(default_leaf(f) == 2)
+    if(f.pairs)
       o_scratch = (o_pairs + 2 * f.nodes.size() * sizeof(uint32_t) + 255) & ~size_t(255);
     bytes = o_scratch + lbvh_scratch_bytes(nprims) + 256;
   }
@@ -984,8 +985,8 @@ extern "C" res_T ssol_b200_plan_launch
 
 /* Replace a plan's device-built tree by the host SAH tree of the same
  * primitive boxes, built on the calling thread while the plan's launches
- * already queued run on the device's tree. Both trees give the same closest
- * hits, so later launches only trace faster. The new nodes go to a buffer
+ * already queued run on the device's tree. Rays meet the same triangles in
+ * both, so later launches only trace faster. The new nodes go to a buffer
  * of their own; launches take the scene by value, so the queued ones keep
  * the old tree. No-op for a plan without a kept snapshot, or when the host
  * tree would be too deep. */
@@ -1026,6 +1027,7 @@ static res_T swap_sah(ssol_b200_plan* p, const FlatScene<R>& f, DScene<R>& S)
   unsigned char* base = (unsigned char*)p->d_bvh2;
   S.nodes = (const DNode<R>*)(base + o_nodes);
   S.primrefs = (const uint32_t*)(base + o_refs);
+  S.own_boxes = bp.max_leaf > 1;
   p->bvh_device = false;
   p->bvh_depth = r.depth;
   p->bvh_nodes = nodes.size();
@@ -1586,17 +1588,27 @@ extern "C" res_T ssol_b200_batch_create
   std::vector<FlatScene<double>> f64;
   /* Snapshots of the items in parallel on the host threads */
   std::vector<res_T> item_res(nscenes, RES_OK);
-  if(opt.precision == SSOL_B200_FP32) {
-    f32.resize(nscenes);
-    parallel_for(nscenes, [&](size_t i) {
+  auto snapshot = [&](size_t i) {
+    if(opt.precision == SSOL_B200_FP32) {
+      f32[i] = FlatScene<float>();
       item_res[i] = flatten_scene(scenes[i], bp, f32[i]);
       if(item_res[i] == RES_OK && !validate(f32[i])) item_res[i] = RES_UNKNOWN_ERR;
-    });
-  } else {
-    f64.resize(nscenes);
-    parallel_for(nscenes, [&](size_t i) {
+    } else {
       item_res[i] = flatten_scene(scenes[i], bp, f64[i]);
       if(item_res[i] == RES_OK && !validate(f64[i])) item_res[i] = RES_UNKNOWN_ERR;
+    }
+  };
+  if(opt.precision == SSOL_B200_FP32) f32.resize(nscenes);
+  else f64.resize(nscenes);
+  parallel_for(nscenes, snapshot);
+  /* One kernel variant traces every item: where it does not keep to own boxes
+   * (OwnBoxes), the items that count on them get leaves of one */
+  int features = 0;
+  for(const FlatScene<float>& f : f32) features |= f.meta.features;
+  if((features & (FEAT_QUADRIC | FEAT_DIELECTRIC)) && !(features & FEAT_ATTRIBUTES)) {
+    bp.max_leaf = bp.max_leaf ? bp.max_leaf : 1;
+    parallel_for(nscenes, [&](size_t i) {
+      if(item_res[i] == RES_OK && f32[i].own_boxes) snapshot(i);
     });
   }
   for(size_t i = 0; i < nscenes; ++i) {
