@@ -555,11 +555,13 @@ __device__ __forceinline__ void restructure
       }
       __syncwarp();
     }
-    /* The whole set: one of its partitions per lane */
+    /* The whole set: one of its partitions per lane. A lane without one must
+     * not win, also where the costs of all partitions overflow: it stands for
+     * the first partition, at an infinite cost. */
     {
       const int P = 2 * lane + 1;
-      float v = P < full ? c[P] + c[full ^ P] : 3.4e38f;
-      int bp = P;
+      float v = P < full ? c[P] + c[full ^ P] : INFINITY;
+      int bp = P < full ? P : 1;
       for(int o = 16; o > 0; o >>= 1) {
         const float u = __shfl_xor_sync(0xffffffffu, v, o);
         const int q = __shfl_xor_sync(0xffffffffu, bp, o);
