@@ -19,7 +19,8 @@ struct LaunchConfig {
   unsigned long long max_segments; /* per path segment budget */
   int min_blocks; /* register budget: 1 (255 regs), 2 (128) or 3 (64 in FP32,
                    * four blocks of 256 threads per SM; 80 in FP64) */
-  int max_nrcv = 0; /* batched launches: the most receiver sides of an item */
+  int max_nrcv = 0; /* batched launches: the most receiver sides of an item, */
+  int max_nsampled = 0; /* and the most sampled instances */
   bool coherent = true; /* larger plain launches run in the order of their
                          * sampled primitives */
   /* Plain launches: stop handing out realisations once this many paths

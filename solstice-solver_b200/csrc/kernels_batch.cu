@@ -100,7 +100,7 @@ static int launch_batch_noalloc_variant
      seed, cfg.max_segments, scratch + NOALLOC_NEXT,
      reinterpret_cast<DStats*>(scratch + NOALLOC_STATS), regen_lanes(cfg.features),
      nullptr, nullptr); /* id order: the coherent order needs scratch */
-  finish_batch<R>(scenes, tallies, nitems, cfg.max_nrcv, s);
+  launch_finish<R>(scenes, tallies, {}, nitems, cfg.max_nrcv, cfg.max_nsampled, s);
   return (int)cudaGetLastError();
 }
 

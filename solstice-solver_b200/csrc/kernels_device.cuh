@@ -1574,7 +1574,8 @@ static __device__ __forceinline__ void commit_warp
 /* The sums that follow from others, once a launch (block y: the item): a
  * receiver side's from its samp_rcv slots, the global cosine and shadowed
  * from the samp slots. Block x < nrcv: that receiver side; the last one: the
- * globals. */
+ * globals. Block z: its slice of the sampled instances; slices add up in what
+ * finish_clear has zeroed, a single one stores. */
 constexpr int FINISH_LANES = 48; /* sampled instances in flight per quantity */
 template<class R>
 __global__ void __launch_bounds__(FINISH_LANES * NRCV_Q * 2) finish_tallies
@@ -1591,16 +1592,53 @@ __global__ void __launch_bounds__(FINISH_LANES * NRCV_Q * 2) finish_tallies
   const double* src = glob ? T.samp + q : T.samp_rcv + (size_t)r * NRCV_Q * 2 + q;
   const size_t step = glob ? 4 : (size_t)nrcv * NRCV_Q * 2;
   double v = 0;
+  const int per = (nsampled + (int)gridDim.z - 1) / (int)gridDim.z;
+  const int last = min(nsampled, ((int)blockIdx.z + 1) * per);
   if(!glob || q < 4)
 #pragma unroll 4
-    for(int s = l; s < nsampled; s += FINISH_LANES) v += src[(size_t)s * step];
+    for(int s = (int)blockIdx.z * per + l; s < last; s += FINISH_LANES)
+      v += src[(size_t)s * step];
   part[l][q] = v;
   __syncthreads();
   if(l) return;
   v = 0;
   for(int k = 0; k < FINISH_LANES; ++k) v += part[k][q];
-  if(!glob) T.rcv[(size_t)r * NRCV_Q * 2 + q] = v;
-  else if(q < 4) T.global[q < 2 ? 2 * G_COS + q : 2 * G_SHADOW + q - 2] = v;
+  if(glob && q >= 4) return;
+  double* dst = glob ? T.global + (q < 2 ? 2 * G_COS + q : 2 * G_SHADOW + q - 2)
+                     : T.rcv + (size_t)r * NRCV_Q * 2 + q;
+  if(gridDim.z == 1) *dst = v;
+  else red_add_global(dst, v);
+}
+template<class R>
+__global__ void __launch_bounds__(256) finish_clear
+  (const DScene<R>* scenes, const DTallies* tallies, const DTallies one, int nrcv)
+{
+  const DTallies& T = tallies ? tallies[blockIdx.x] : one;
+  if(scenes) nrcv = scenes[blockIdx.x].nrcv;
+  for(int i = threadIdx.x; i < nrcv * NRCV_Q * 2; i += blockDim.x) T.rcv[i] = 0.0;
+  if(threadIdx.x < 2) {
+    T.global[2 * G_COS + threadIdx.x] = 0.0;
+    T.global[2 * G_SHADOW + threadIdx.x] = 0.0;
+  }
+}
+
+/* Sampled instances that one block adds up by itself, and those of a slice
+ * where there are more. One block for all of a receiver side's grew with the
+ * plant: us a plan launch of 1e4 paths, one receiver side, one block / slices:
+ * 2000 sampled instances 124 / 123 (of two launches), 2500 126 / 122, 5000
+ * 138 / 125, 20,000 198 / 128, 1e5 418 / 127. */
+constexpr int FINISH_SINGLE = 2048, FINISH_SLICE = 1024, FINISH_SLICES_MAX = 64;
+template<class R>
+static void launch_finish(const DScene<R>* scenes, const DTallies* tallies, const DTallies& one,
+                          int nitems, int nrcv, int nsampled, cudaStream_t st)
+{
+  const int slices = nsampled <= FINISH_SINGLE ? 1
+    : std::min((nsampled + FINISH_SLICE - 1) / FINISH_SLICE, FINISH_SLICES_MAX);
+  if(slices > 1) finish_clear<R><<<(unsigned)nitems, 256, 0, st>>>(scenes, tallies, one, nrcv);
+  for(int i = 0; i < nitems; i += 65535)
+    finish_tallies<R><<<dim3((unsigned)nrcv + 1, (unsigned)std::min(nitems - i, 65535),
+                             (unsigned)slices), FINISH_LANES * NRCV_Q * 2, 0, st>>>
+      (scenes ? scenes + i : nullptr, tallies ? tallies + i : nullptr, one, nrcv, nsampled);
 }
 
 /*******************************************************************************
@@ -2546,8 +2584,7 @@ static int launch_variant
     realisation_kernel<R, MINB, TRACK, FEAT><<<(unsigned)blocks, block, smem, st>>>
       (S, T, seed, first, count, cfg.max_segments, T.counters + 3, tr, nullptr,
        1u, 1u, ctl);
-    finish_tallies<R><<<S.nrcv + 1, FINISH_LANES * NRCV_Q * 2, 0, st>>>
-      (nullptr, nullptr, T, S.nrcv, S.nsampled);
+    launch_finish<R>(nullptr, nullptr, T, 1, S.nrcv, S.nsampled, st);
     return (int)cudaGetLastError();
   }
   for(uint64_t c0 = 0; c0 < count; c0 += chunk) {
@@ -2562,8 +2599,7 @@ static int launch_variant
       (S, T, seed, first + c0, n, cfg.max_segments, T.counters + 3, tr,
        sort.sorted_off, seg_len, segment_stride(nseg), ctl);
   }
-  finish_tallies<R><<<S.nrcv + 1, FINISH_LANES * NRCV_Q * 2, 0, st>>>
-    (nullptr, nullptr, T, S.nrcv, S.nsampled);
+  launch_finish<R>(nullptr, nullptr, T, 1, S.nrcv, S.nsampled, st);
   cudaFreeAsync(sort.buf, st);
   return (int)cudaGetLastError();
 }
@@ -2604,17 +2640,6 @@ static int launch_impl
   }
 }
 
-template<class R>
-static void finish_batch(const DScene<R>* scenes, const DTallies* tallies, int nitems,
-                         int max_nrcv, cudaStream_t st)
-{
-  const DTallies none = {};
-  for(int i = 0; i < nitems; i += 65535)
-    finish_tallies<R><<<dim3((unsigned)max_nrcv + 1, (unsigned)std::min(nitems - i, 65535)),
-                        FINISH_LANES * NRCV_Q * 2, 0, st>>>
-      (scenes + i, tallies + i, none, 0, 0);
-}
-
 template<class R, int MINB, int FEAT>
 static int launch_batch_variant(const BatchLaunch<R>& b, const LaunchConfig& cfg,
                                 void* stream)
@@ -2649,7 +2674,7 @@ static int launch_batch_variant(const BatchLaunch<R>& b, const LaunchConfig& cfg
   batch_kernel<R, MINB, FEAT><<<(unsigned)blocks, block, smem, st>>>
     (b.scenes, b.tallies, b.prefix, b.firsts, b.nitems, b.seed, cfg.max_segments,
      b.next_items, b.stats, regen_lanes(cfg.features), o.sorted_off, o.seg_mul);
-  finish_batch<R>(b.scenes, b.tallies, b.nitems, cfg.max_nrcv, st);
+  launch_finish<R>(b.scenes, b.tallies, {}, b.nitems, cfg.max_nrcv, cfg.max_nsampled, st);
   return (int)cudaGetLastError();
 }
 

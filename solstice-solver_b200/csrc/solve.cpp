@@ -1979,13 +1979,15 @@ static LaunchConfig batch_config(const ssol_b200_batch* b)
   cfg.max_segments = b->opt.max_segments;
   cfg.min_blocks = b->opt.min_blocks_per_sm;
   cfg.count_work = b->opt.count_work != 0;
-  size_t nrcv = 0;
+  size_t nrcv = 0, nsampled = 0;
   cfg.features = 0;
   for(const FlatMeta& m : b->meta) {
     nrcv = std::max(nrcv, m.rcv.size());
+    nsampled = std::max(nsampled, m.sampled.size());
     cfg.features |= m.features;
   }
   cfg.max_nrcv = (int)nrcv;
+  cfg.max_nsampled = (int)nsampled;
   return cfg;
 }
 
