@@ -1781,8 +1781,8 @@ realisation_kernel
     bool start = false;
     uint64_t off = 0;
     /* Early stop: every 4th fetch of the warp (of 32 realisations or so)
-     * reads the stop and abort words (one L2 sector); a halted warp takes no new realisation and ends
-     * once its paths in flight end */
+     * reads the stop and abort words (one L2 sector); a halted warp takes no
+     * new realisation, also for the lanes whose paths end later */
     bool halt = false;
     if(need && polled && (fetches++ & 3u) == 0u) {
       const int leader = __ffs(need) - 1;
@@ -1794,7 +1794,7 @@ realisation_kernel
       halt = __shfl_sync(0xffffffffu, h, leader) != 0;
     }
     if(halt) {
-      if(p.phase == PH_NONE) done = true;
+      done = true;
     } else if(need && sorted_off) {
       /* Segments of SORT_SEG sorted realisations (one or two primitives) go
        * to warps whole, in a strided order, so that a warp's lanes start on
