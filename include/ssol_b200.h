@@ -38,12 +38,12 @@ enum ssol_b200_precision {
  *    FP32 (bvh_leaf_size is ignored); the fastest to build. A tree deeper than the
  *    traversal stack allows (more than 30 levels) is rebuilt on the host with
  *    the SAH builder, with a warning;
- *  - SSOL_B200_BVH_AUTO (the default): ssol_solve, ssol_solve_ex and (with
- *    leaves of one primitive) ssol_solve_adjoint use the device builder for
- *    at most SSOL_B200_BVH_AUTO_MAX_PATHS realisations, where building is a
- *    large part of the call. Larger solves
- *    start on the device's tree and, after their first 6e6 realisations,
- *    trace on the SAH tree that the host threads built meanwhile. Plans,
+ *  - SSOL_B200_BVH_AUTO (the default): ssol_solve, ssol_solve_ex (whatever
+ *    bvh_leaf_size) and, when bvh_leaf_size is 0, ssol_solve_adjoint use the
+ *    device builder for at most SSOL_B200_BVH_AUTO_MAX_PATHS realisations,
+ *    where building is a large part of the call. Larger solves start on the
+ *    device's tree and, after their first 6e6 realisations, trace on the SAH
+ *    tree that the host threads built meanwhile. Plans,
  *    which do not know how many realisations they will trace, use the SAH
  *    builder.
  * A path hits the same triangles with both trees: one whose own box the rounded
@@ -52,10 +52,10 @@ enum ssol_b200_precision {
  * the exception: which of them is hit, and so which per-primitive estimate the
  * path adds to, is the tree's choice (about one path in 1e9 too). With leaves
  * of two or more that the caller asks for (bvh_leaf_size), the box that counts
- * is the leaf's. Batches always use the SAH builder. The renderers
- * use the device builder by default for images of at most
- * SSOL_B200_BVH_AUTO_MAX_SAMPLES camera samples (with leaves of one
- * primitive), the SAH builder above. */
+ * is the leaf's. Batches always use the SAH
+ * builder. The renderers use the device builder by default (bvh_leaf_size 0)
+ * for images of at most SSOL_B200_BVH_AUTO_MAX_SAMPLES camera samples, the SAH
+ * builder above. */
 enum ssol_b200_bvh_builder {
   SSOL_B200_BVH_AUTO = 0,
   SSOL_B200_BVH_SAH = 1,

@@ -702,9 +702,9 @@ res_T ssolb_snapshot_create
   BvhBuildParams bp;
   bp.max_leaf = opt.bvh_leaf_size;
   bp.threads = host_threads();
-  /* The device's tree does not take the caller's leaf size */
+  /* The device's tree does not take a leaf size that the caller gives */
   bp.device = opt.bvh_builder == SSOL_B200_BVH_LBVH
-    || (opt.bvh_builder == SSOL_B200_BVH_AUTO && bp.max_leaf <= 1
+    || (opt.bvh_builder == SSOL_B200_BVH_AUTO && bp.max_leaf == 0
         && samples <= SSOL_B200_BVH_AUTO_MAX_SAMPLES);
   out.precision = opt.precision;
   std::unique_ptr<FlatScene<float>> f32;
@@ -794,7 +794,6 @@ static res_T plan_create_impl
   if(!builder_ok(opt.bvh_builder)) return RES_BAD_ARG;
   /* a plan does not know how many realisations it will trace */
   if(opt.bvh_builder == SSOL_B200_BVH_AUTO) opt.bvh_builder = SSOL_B200_BVH_SAH;
-  if(opt.bvh_builder == SSOL_B200_BVH_LBVH) opt.bvh_leaf_size = 1;
 
   BvhBuildParams bp;
   bp.max_leaf = opt.bvh_leaf_size;
@@ -1003,7 +1002,9 @@ static res_T swap_sah(ssol_b200_plan* p, const FlatScene<R>& f, DScene<R>& S)
     boxes[i].ref = f.prim_ref[i];
   }
   BvhBuildParams bp;
+  /* The caller's leaf size, where own boxes keep the paths of the first part */
   bp.max_leaf = default_leaf(f);
+  if(bp.max_leaf > 1 && p->opt.bvh_leaf_size) bp.max_leaf = p->opt.bvh_leaf_size;
   bp.threads = host_threads();
   BvhResult r;
   build_bvh(std::move(boxes), bp, r);
@@ -1210,7 +1211,7 @@ extern "C" res_T ssol_solve_adjoint
    * heliostats the host's tree takes 3 ms longer to build and traces both
    * passes 0.4 ms faster */
   ssol_b200_options opt = options ? *options : SSOL_B200_OPTIONS_DEFAULT;
-  if(opt.bvh_builder == SSOL_B200_BVH_AUTO && opt.bvh_leaf_size <= 1
+  if(opt.bvh_builder == SSOL_B200_BVH_AUTO && opt.bvh_leaf_size == 0
   && (unsigned long long)n <= SSOL_B200_BVH_AUTO_MAX_PATHS)
     opt.bvh_builder = SSOL_B200_BVH_LBVH;
   ssol_b200_plan* plan = nullptr;
