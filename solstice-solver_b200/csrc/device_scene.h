@@ -245,7 +245,7 @@ template<typename R> struct DScene {
    * paths of a scene without any need not sample theirs */
   int32_t spectral;
   /* A triangle in a leaf of several counts as hit only where its own box is
-   * hit too (trace_ray) */
+   * hit too (test_triangle) */
   int32_t own_boxes;
 
   const DSampTri<R>* samp;

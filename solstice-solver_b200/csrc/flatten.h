@@ -101,7 +101,7 @@ template<class R> struct FlatScene {
  * tests (7.7 for 7.2), which a warp makes together. Plan launches, leaves of
  * 1 / 2 / 3 / 4 without own boxes: field of 1000, 5e7 paths, 30.8 / 29.1 /
  * 29.1 / 30.4 ms; of 317, 2e7, 11.0 / 10.4 / 10.4 / 10.9; one mirror, 5e6,
- * 1.36 / 1.28 / 1.28 / 1.31. Own boxes (trace_ray) take 2 of the 6 %.
+ * 1.36 / 1.28 / 1.28 / 1.31. Own boxes (test_triangle) take 2 of the 6 %.
  * One with punched surfaces, whose test costs more than a node visit
  * (beam-down, 1e7, 13.8 / 14.4 / 14.9 / 15.6); one in FP64, where own boxes
  * cost more than the leaves give (field of 500, solve of 2e6, 3.80 ms, with

@@ -4,10 +4,9 @@
  * kernels_*.cu translation units, each of which instantiates some of the
  * launchers, so that they compile in parallel.
  *
- *
- * One thread traces whole optical paths, persistent over a grid-stride range
- * of realisations. Per path it restates, on the flat device scene of
- * device_scene.h:
+ * One thread traces whole optical paths; the warps of a persistent grid take
+ * realisations, or segments of sorted ones, from a counter. Per path it
+ * restates, on the flat device scene of device_scene.h:
  *   point_init             src/ssol_solver.c:207-358
  *   trace_radiative_path   src/ssol_solver.c:873-1127
  *   point_update_from_hit  src/ssol_solver.c:360-411
@@ -2002,8 +2001,8 @@ realisation_kernel
  * and their realisation budgets in one persistent launch. Global work index
  * g maps to item it = max{i : prefix[i] <= g} and to realisation
  * firsts[it] + g - prefix[it] of that item's streams. Every item has its own
- * tallies; the per-thread FP64 global sums are flushed when a thread moves
- * to another item. The launch's total is prefix[nitems], read from device
+ * tallies; a warp's tiles are keyed by the item they sum for and flushed when
+ * it commits for another one. The launch's total is prefix[nitems], read from device
  * memory so that a captured CUDA graph replays with new budgets. */
 template<class R, int MINB, int FEAT>
 __global__ void __launch_bounds__(MAX_BLOCK, sizeof(R) == 4 && MINB == 3 ? 4 : MINB)
@@ -2124,7 +2123,7 @@ batch_kernel
           /* Coherent order: the item's full warp segments of SORT_SEG
            * sorted realisations in a strided order (so that the warps of an
            * item group spread over its primitives), the ragged last one
-           * last; each record gives the realisation and its primary draw */
+           * last; each record is a realisation's offset in the item */
           uint64_t off = g;
           if(sorted_off) {
             const unsigned long long nfull = (prefix[it + 1] - prefix[it]) / SORT_SEG;

@@ -30,8 +30,8 @@
  *      the root's height is the tree depth, which the host reads back to check
  *      the traversal stack bound;
  *   7. the internal nodes are renumbered depth first, slot 0 first, so that
- *      a node's first child follows it in memory; in scenes of meshes a node of
- *      two primitives becomes a leaf of two.
+ *      a node's first child follows it in memory; in FP32 scenes of meshes a
+ *      node of two primitives becomes a leaf of two.
  * Scenes of at most SMALL_BUILD primitives go through all of them in one
  * launch.
  */
@@ -663,7 +663,7 @@ __device__ __forceinline__ void lbvh_box(const R* box, const uint32_t* vals, int
   }
 }
 
-/* Step 6: depth-first order of the internal nodes (slot 0 first), as the
+/* Step 7: depth-first order of the internal nodes (slot 0 first), as the
  * host builder numbers them, so that a node's first child follows it in
  * memory: a node's index is the sum, over the path from the root, of one
  * per step plus, where the path takes slot 1, the internal nodes of the
@@ -689,9 +689,9 @@ __device__ __forceinline__ int lbvh_index(const DNode<R>* nodes, const int32_t* 
 /* With `pairs`, a node of two primitives becomes a leaf of two in its parent,
  * whose references are listed at its own index (the node's place stays, unread):
  * fewer node visits for a few more tests, which a warp makes together, as in
- * the host's tree of mesh scenes (default_leaf). Adjoint, 1e7 paths, 13.1 ->
- * 11.2 ms; field of 317 under Buie's sun, 5.1e6, 5.96 -> 5.79; FP64 field, 2e6,
- * 3.73 -> 3.53; one mirror, 1e6, 0.405 -> 0.389; path-traced view 8.2 -> 7.8. */
+ * the host's tree of mesh scenes (default_leaf). With own boxes (test_triangle),
+ * adjoint, 1e7 paths, 12.7 -> 10.7 ms; field of 317 under Buie's sun, 5.1e6,
+ * 5.91 -> 5.80; one mirror, 1e6, 0.387 -> 0.373. */
 template<class R>
 __device__ __forceinline__ void lbvh_permute(const DNode<R>* src, DNode<R>* dst,
                                              const int32_t* newidx, uint32_t* pairs, int i)
