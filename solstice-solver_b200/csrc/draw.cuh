@@ -171,7 +171,7 @@ __device__ __forceinline__ R microfacet_g(R nh, R no, R ni, R oh)
 template<class R>
 __device__ __forceinline__ R draw_bsdf_eval(const DrawBsdf<R>& f, V3<R> wo, V3<R> N, V3<R> wi)
 {
-  const R no = dot(wo, N), ni = dot(wi, N);
+  const R no = dot_yx_rn(wo, N), ni = dot_yx(wi, N);
   if(!(no > R(0)) || !(ni > R(0))) return R(0);
   if(f.m.type == MTL_MATTE) return f.refl * R(0.31830988618379067154);
   if(f.m.type == MTL_MIRROR && f.rough > R(0)) {
@@ -326,7 +326,7 @@ __device__ __forceinline__ bool draw_radiance
     const V3<R> wo = -wo_in;
     /* sun_lighting (src/ssol_draw_pt.c:92-121) */
     {
-      const R c = dot(to_sun, N);
+      const R c = dot_yx(to_sun, N);
       if(c >= R(0) && !(fabs(c) <= R(1e-6))) {
         const R fv = draw_bsdf_eval(f, wo, N, to_sun);
         if(fv > R(0)) {

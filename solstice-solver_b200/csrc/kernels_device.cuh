@@ -107,6 +107,9 @@ template<class R> __device__ __forceinline__ V3<R> normalize(V3<R> v)
  * order, where the code has always rounded so */
 template<class R> __device__ __forceinline__ R dot_yx(V3<R> a, V3<R> b)
 { return sum3(a.y, b.y, a.x, b.x, a.z, b.z); }
+/* The same with the last product rounded on its own, too */
+template<class R> __device__ __forceinline__ R dot_yx_rn(V3<R> a, V3<R> b)
+{ return mul_rn(a.z, b.z) + fma(a.y, b.y, mul_rn(a.x, b.x)); }
 template<class R> __device__ __forceinline__ V3<R> normalize_hit(V3<R> v)
 {
   const R len = sq_rt(dot_yx(v, v));
