@@ -60,7 +60,7 @@ __device__ __forceinline__ V3<R> draw_shading_normal
 {
   b1 = b2 = R(0);
   if(!(FEAT & FEAT_ATTRIBUTES) || !S.tshade || gid < 0) return N;
-  const float2 uv = tri_uv(S, gid, pos);
+  const float2 uv = tri_uv<R, true>(S, gid, pos);
   b1 = (R)uv.x;
   b2 = (R)uv.y;
   const DTriShade<R>& ts = S.tshade[gid];

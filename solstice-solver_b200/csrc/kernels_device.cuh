@@ -216,7 +216,7 @@ __device__ __forceinline__ R baked_value
   const R v0 = shader_lerp(S.shader_wl, S.shader_nodes, tab, which, wl);
   const R v1 = shader_lerp(S.shader_wl, S.shader_nodes, tab + stride, which, wl);
   const R v2 = shader_lerp(S.shader_wl, S.shader_nodes, tab + 2 * stride, which, wl);
-  return v0 * (R(1) - b1 - b2) + v1 * b1 + v2 * b2;
+  return sum3(v0, R(1) - b1 - b2, v1, b1, v2, b2);
 }
 
 /*******************************************************************************
@@ -821,8 +821,9 @@ __host__ __device__ constexpr int ps_count(int feat)
 { return feat & FEAT_ATTRIBUTES ? 11 : 10; }
 
 /* Barycentric weights (b1, b2) of vertices 1 and 2 of triangle gid at the
- * point x of its plane */
-template<class R>
+ * point x of its plane. DRAW: the determinant with its other product fused, as
+ * the renderers have always rounded it. */
+template<class R, bool DRAW = false>
 __device__ __forceinline__ float2 tri_uv(const DScene<R>& S, int gid, V3<R> x)
 {
   const DTri<R>& T = S.tris[gid];
@@ -830,10 +831,10 @@ __device__ __forceinline__ float2 tri_uv(const DScene<R>& S, int gid, V3<R> x)
   const V3<R> e1 = ld3(T.v1) - a, e2 = ld3(T.v2) - a, q = x - a;
   const R d11 = dot(e1, e1), d12 = dot(e1, e2), d22 = dot(e2, e2);
   const R q1 = dot(q, e1), q2 = dot(q, e2);
-  const R den = d11 * d22 - d12 * d12;
+  const R den = DRAW ? fma(d11, d22, -mul_rn(d12, d12)) : fma(-d12, d12, mul_rn(d11, d22));
   if(!(den != R(0))) return make_float2(0.f, 0.f);
-  return make_float2((float)((d22 * q1 - d12 * q2) / den),
-                     (float)((d11 * q2 - d12 * q1) / den));
+  return make_float2((float)(fma(d22, q1, -mul_rn(d12, q2)) / den),
+                     (float)(fma(d11, q2, -mul_rn(d12, q1)) / den));
 }
 
 /* Barycentric weights (b1, b2) of the current point, kept as two floats in
