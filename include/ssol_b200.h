@@ -34,28 +34,27 @@ enum ssol_b200_precision {
  *  - SSOL_B200_BVH_LBVH: linear BVH built on the device from the uploaded
  *    primitive boxes (Morton codes, radix sort, Karras' hierarchy, bottom-up
  *    boxes, treelet restructuring for a lower SAH cost, depth-first node
- *    order), one primitive per leaf, or up to two in scenes of meshes in
- *    FP32 (bvh_leaf_size is ignored); the fastest to build. A tree deeper than the
- *    traversal stack allows (more than 30 levels) is rebuilt on the host with
- *    the SAH builder, with a warning;
+ *    order), one primitive per leaf, with the same pairs of triangles as the
+ *    default leaves (bvh_leaf_size is ignored); the fastest to build. A tree
+ *    deeper than the traversal stack allows (more than 30 levels) is rebuilt on
+ *    the host with the SAH builder, with a warning;
  *  - SSOL_B200_BVH_AUTO (the default): ssol_solve, ssol_solve_ex (whatever
  *    bvh_leaf_size) and, when bvh_leaf_size is 0, ssol_solve_adjoint use the
  *    device builder for at most SSOL_B200_BVH_AUTO_MAX_PATHS realisations,
  *    where building is a large part of the call. Larger solves start on the
  *    device's tree and, after their first 6e6 realisations, trace on the SAH
- *    tree that the host threads built meanwhile. Plans,
- *    which do not know how many realisations they will trace, use the SAH
- *    builder.
+ *    tree that the host threads built meanwhile. Plans, which do not know how
+ *    many realisations they will trace, use the SAH builder.
  * A path hits the same triangles with both trees: one whose own box the rounded
  * box test misses (at a corner of the box, about one path in 1e9) is missed by
  * either. Two triangles met at the same distance, on the edge they share, are
  * the exception: which of them is hit, and so which per-primitive estimate the
- * path adds to, is the tree's choice (about one path in 1e9 too). With leaves
- * of two or more that the caller asks for (bvh_leaf_size), the box that counts
- * is the leaf's. Batches always use the SAH
- * builder. The renderers use the device builder by default (bvh_leaf_size 0)
- * for images of at most SSOL_B200_BVH_AUTO_MAX_SAMPLES camera samples, the SAH
- * builder above. */
+ * path adds to, is the tree's choice (one path in 1e9, or in 1e6 on a receiver
+ * whose axes are the scene's). With leaves of two or more that the caller asks
+ * for (bvh_leaf_size), the box that counts is the leaf's. Batches always use
+ * the SAH builder. The renderers use the device builder by default
+ * (bvh_leaf_size 0) for images of at most SSOL_B200_BVH_AUTO_MAX_SAMPLES camera
+ * samples, the SAH builder above. */
 enum ssol_b200_bvh_builder {
   SSOL_B200_BVH_AUTO = 0,
   SSOL_B200_BVH_SAH = 1,
@@ -69,9 +68,8 @@ struct ssol_b200_options {
   int block_size; /* threads per block, <= 256; 0 => 256 */
   int grid_blocks; /* 0 => one persistent wave sized from occupancy */
   int waves; /* persistent grid multiplier when grid_blocks == 0 */
-  int bvh_leaf_size; /* primitives per BVH leaf; 0 => by the scene: 2 for meshes
-                      * in FP32, 1 in FP64 and with punched surfaces or
-                      * dielectrics */
+  int bvh_leaf_size; /* primitives per BVH leaf; 0 => 1, with pairs of triangles
+                      * joined in FP32 scenes of meshes without dielectrics */
   unsigned long long max_segments; /* path segment budget; 0 => 1e6 */
   int min_blocks_per_sm; /* register budget of the kernel variant: 1, 2, 3;
                           * 0 => 3 in FP32, 2 in FP64 */

@@ -419,6 +419,30 @@ template<class R> std::vector<DNode<R>> bvh_nodes(const BvhResult& b)
   return nodes;
 }
 
+template<class R> void join_pairs(std::vector<DNode<R>>& nodes, std::vector<uint32_t>& primrefs)
+{
+  std::vector<int32_t> at(nodes.size()); /* new index, or the pair's child value */
+  size_t kept = 0;
+  for(size_t i = 0; i < nodes.size(); ++i) {
+    const DNode<R>& n = nodes[i];
+    if(i && n.count[0] == 1 && n.count[1] == 1) {
+      at[i] = PAIR_LEAF | (int32_t)primrefs.size();
+      primrefs.push_back((uint32_t)n.child[0]);
+      primrefs.push_back((uint32_t)n.child[1]);
+    } else {
+      at[i] = (int32_t)kept++;
+    }
+  }
+  for(size_t i = 0; i < nodes.size(); ++i) {
+    if(at[i] & PAIR_LEAF) continue;
+    DNode<R> n = nodes[i];
+    for(int k = 0; k < 2; ++k)
+      if(n.count[k] == 0) n.child[k] = at[n.child[k]];
+    nodes[at[i]] = n;
+  }
+  nodes.resize(kept);
+}
+
 template<class R> void round_box_outward(const PrimBox& b, R out[6])
 {
   for(int c = 0; c < 3; ++c) {
@@ -429,6 +453,8 @@ template<class R> void round_box_outward(const PrimBox& b, R out[6])
 
 template void round_box_outward<float>(const PrimBox&, float*);
 template void round_box_outward<double>(const PrimBox&, double*);
+template void join_pairs<float>(std::vector<DNode<float>>&, std::vector<uint32_t>&);
+template void join_pairs<double>(std::vector<DNode<double>>&, std::vector<uint32_t>&);
 template std::vector<DNode<float>> bvh_nodes<float>(const BvhResult&);
 template std::vector<DNode<double>> bvh_nodes<double>(const BvhResult&);
 

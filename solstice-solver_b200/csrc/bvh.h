@@ -19,7 +19,7 @@ struct PrimBox {
 };
 
 struct BvhBuildParams {
-  int max_leaf = 4; /* primitives per leaf; a snapshot takes 0 as default_leaf */
+  int max_leaf = 4; /* primitives per leaf; a snapshot takes 0 as 1, and may join pairs */
   int bins = 16; /* SAH bins per axis */
   int max_depth = 30; /* the device traversal stack holds 32 entries */
   int threads = 1; /* host threads for the subtrees of large scenes */
@@ -43,6 +43,10 @@ template<class R> void round_box_outward(const PrimBox& b, R out[6]);
 
 /* Convert to device nodes of precision R, rounding boxes outward */
 template<class R> std::vector<DNode<R>> bvh_nodes(const BvhResult& b);
+
+/* Turn each node of two single primitives, but the root, into a pair in its
+ * parent (PAIR_LEAF), its slot 0 first; the pairs' references are appended */
+template<class R> void join_pairs(std::vector<DNode<R>>& nodes, std::vector<uint32_t>& primrefs);
 
 } /* namespace ssolb */
 

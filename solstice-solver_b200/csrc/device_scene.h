@@ -176,8 +176,10 @@ struct DCarving {
 };
 
 /* Binary BVH node holding its children's boxes. count == 0: child is a node
- * index; count == 1: child is the leaf's prim reference itself; count > 1:
- * child is the leaf's first entry in primrefs; count < 0: empty slot. */
+ * index, or PAIR_LEAF and the first of a pair of triangles in primrefs; count
+ * == 1: child is the leaf's prim reference itself; count > 1: child is the
+ * leaf's first entry in primrefs; count < 0: empty slot. */
+constexpr int32_t PAIR_LEAF = 1 << 30;
 template<typename R> struct alignas(16) DNode {
   R lo[2][3];
   R hi[2][3];
@@ -207,9 +209,9 @@ enum : int32_t {
   FEAT_NOCOUNT = 8
 };
 
-/* Kernel variants that keep to DScene::own_boxes: FP32 without quadrics or
- * dielectrics, and FP32 with everything */
-template<class R, int FEAT> struct OwnBoxes {
+/* Kernel variants that know pairs of triangles (PAIR_LEAF): FP32 without
+ * quadrics or dielectrics, and FP32 with everything */
+template<class R, int FEAT> struct Pairs {
   static constexpr bool value = sizeof(R) == sizeof(float)
     && (!(FEAT & (FEAT_QUADRIC | FEAT_DIELECTRIC)) || (FEAT & FEAT_ATTRIBUTES));
 };
@@ -244,9 +246,6 @@ template<typename R> struct DScene {
   /* Some material, medium or baked shader depends on the wavelength; the
    * paths of a scene without any need not sample theirs */
   int32_t spectral;
-  /* A triangle in a leaf of several counts as hit only where its own box is
-   * hit too (test_triangle) */
-  int32_t own_boxes;
 
   const DSampTri<R>* samp;
   const float* alias_prob;

@@ -979,8 +979,7 @@ static res_T flatten_impl
   if(bvh_params.device && boxes.size() >= 2) {
     const size_t n = boxes.size();
     out.device_bvh = true;
-    out.pairs = default_leaf(out) == 2;
-    out.own_boxes = out.pairs;
+    out.pairs = joins_pairs(out);
     out.prim_box.resize(6 * n);
     out.prim_ref.resize(n);
     for(size_t i = 0; i < n; ++i) {
@@ -993,11 +992,12 @@ static res_T flatten_impl
   }
   BvhBuildParams prm = bvh_params;
   if(prm.max_leaf == 0) {
-    prm.max_leaf = default_leaf(out);
-    out.own_boxes = prm.max_leaf > 1;
+    prm.max_leaf = 1;
+    out.pairs = joins_pairs(out);
   }
   build_bvh(boxes, prm, out.bvh);
   out.nodes = bvh_nodes<R>(out.bvh);
+  if(out.pairs) join_pairs(out.nodes, out.bvh.primrefs);
   return RES_OK;
 }
 

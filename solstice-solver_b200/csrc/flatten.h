@@ -63,8 +63,7 @@ template<class R> struct FlatScene {
    * n - 1 zeroed nodes the device builder fills, and bvh.depth is unknown
    * (0) until it has run */
   bool device_bvh = false;
-  bool pairs = false; /* the device builder joins pairs of triangles in leaves */
-  bool own_boxes = false; /* DScene::own_boxes */
+  bool pairs = false; /* the tree joins pairs of triangles */
   std::vector<R> prim_box;
   std::vector<uint32_t> prim_ref;
   std::vector<DTri<R>> tris;
@@ -94,22 +93,19 @@ template<class R> struct FlatScene {
   int32_t air_medium = 0;
 };
 
-/* Primitives per leaf of the host's tree where the caller leaves the choice,
- * and at most so many of the device's.
- * Two for meshes: a rectangle's two triangles are one leaf, so a ray makes
- * fewer node visits (field 40.4 for 44.3 a path) for a few more triangle
- * tests (7.7 for 7.2), which a warp makes together. Plan launches, leaves of
- * 1 / 2 / 3 / 4 without own boxes: field of 1000, 5e7 paths, 30.8 / 29.1 /
- * 29.1 / 30.4 ms; of 317, 2e7, 11.0 / 10.4 / 10.4 / 10.9; one mirror, 5e6,
- * 1.36 / 1.28 / 1.28 / 1.31. Own boxes (test_triangle) take 2 of the 6 %.
- * One with punched surfaces, whose test costs more than a node visit
- * (beam-down, 1e7, 13.8 / 14.4 / 14.9 / 15.6); one in FP64, where own boxes
- * cost more than the leaves give (field of 500, solve of 2e6, 3.80 ms, with
- * two 3.94); and one with dielectrics, whose kernel variant has quadrics too. */
-template<class R> int default_leaf(const FlatScene<R>& f)
+/* Whether a tree that the library chooses joins pairs of triangles: a node of
+ * two triangles gives way to a pair in its parent, so that a ray makes fewer
+ * node visits for a few more triangle tests, which a warp makes together.
+ * Leaves of their own / pairs: field of 1000, plan launch of 1e8 paths, 63.4 /
+ * 62.1 ms; adjoint, 1e7, 12.1 / 11.0; batch of 32 suns 29.6 / 29.1; path-traced
+ * view 7.63 / 7.54.
+ * Not in FP64, where the test of own boxes costs more than the pairs give
+ * (field of 500, solve of 2e6, 3.80 ms, with pairs 3.94), and not with punched
+ * surfaces, whose test costs more than a node visit, or dielectrics, whose
+ * kernel variant has punched surfaces too. */
+template<class R> bool joins_pairs(const FlatScene<R>& f)
 {
-  return sizeof(R) == sizeof(float) && !(f.meta.features & (FEAT_QUADRIC | FEAT_DIELECTRIC))
-    ? 2 : 1;
+  return sizeof(R) == sizeof(float) && !(f.meta.features & (FEAT_QUADRIC | FEAT_DIELECTRIC));
 }
 
 /* for_draw: snapshot for the renderers, which sample no instance (no

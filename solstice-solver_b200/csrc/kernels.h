@@ -148,7 +148,7 @@ int launch_track_f64(const TrackArgs& A, void* stream);
 /* Device-built linear BVH (lbvh.cu) over n >= 2 primitive boxes (device
  * array of 6 R per primitive: lo xyz, hi xyz, already rounded outward) and
  * their references; writes the n - 1 nodes of DNode<R> (root 0, one
- * primitive per leaf, or with `pairs`, 2 (n - 1) references, also two) and the
+ * primitive per leaf, or with `pairs`, 2 (n - 1) references, pairs too) and the
  * depth of the tree of single primitives (device int). The scratch pointers
  * come from lbvh_bind_scratch over lbvh_scratch_bytes(n) bytes. */
 struct LbvhArgs {

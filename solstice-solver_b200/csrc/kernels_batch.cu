@@ -259,11 +259,12 @@ template<class R>
 __device__ void leaf_box(const DNode<R>& node, int k, const DTri<R>* tris,
                          const uint32_t* primrefs, R lo[3], R hi[3])
 {
-  const int cnt = node.count[k];
+  const bool pair = node.count[k] == 0 && (node.child[k] & PAIR_LEAF);
+  const int cnt = pair ? 2 : node.count[k], first = pair ? node.child[k] ^ PAIR_LEAF : node.child[k];
   bool quad = false;
   for(int c = 0; c < 3; ++c) { lo[c] = rmax<R>(); hi[c] = -rmax<R>(); }
   for(int i = 0; i < cnt; ++i) {
-    const uint32_t ref = cnt == 1 ? (uint32_t)node.child[k] : primrefs[node.child[k] + i];
+    const uint32_t ref = cnt == 1 ? (uint32_t)first : primrefs[first + i];
     if(primref_kind(ref) != PRIM_TRIANGLE) { quad = true; continue; }
     const DTri<R>& T = tris[primref_index(ref)];
     for(int c = 0; c < 3; ++c) {
@@ -293,7 +294,7 @@ __global__ void __launch_bounds__(256) track_refit_kernel(const TrackArgs A)
         const int cnt = node.count[k];
         if(cnt < 0) continue;
         R lo[3], hi[3];
-        if(cnt > 0) {
+        if(cnt > 0 || (node.child[k] & PAIR_LEAF)) {
           leaf_box(node, k, tris, A.primrefs, lo, hi);
         } else {
           const DNode<R>& ch = nodes[node.child[k]];

@@ -609,20 +609,20 @@ __device__ __forceinline__ bool own_box(const DTri<R>& T, V3<R> inv, V3<R> oinv,
  * a ray crossing a virtual quad on its diagonal is not counted twice.
  * Ng = e2 x e1 is Star-3D's front face.
  *
- * With `own` (the triangle is in a leaf of several) its own box must be hit
- * too, so that a ray meets the same triangles whatever the leaves. The box
- * test rounds: a triangle that is hit at a corner of its box can have the box
- * missed by an ulp of the distance and its leaf's larger box hit, where a leaf
- * of its own would not have been tested: 2 of 1.6e9 paths of the field of
- * 1000, 3e-8 of its estimates. (A leaf's box is never missed where a
- * triangle's own is hit: the rounded products are monotone in the bounds.)
- * Asked of accepted hits only, with the vertices read again rather than kept
- * in registers: field, 1e8 paths, 59.2 -> 60.3 ms; asked once, of the hit a
- * traversal ends with, 60.9. */
+ * A triangle of a pair (`own`) must have its own box hit too, before tleaf, so
+ * that a ray meets the triangles that it would meet in leaves of their own. The
+ * box test rounds: a triangle that is hit at a corner of its box can have the
+ * box missed by an ulp of the distance and the pair's larger box hit, where a
+ * leaf of its own would not have been tested: 2 of 1.6e9 paths of the field of
+ * 1000, 3e-8 of its estimates. (A pair's box is never missed where a triangle's
+ * own is hit: the rounded products are monotone in the bounds.) Asked of
+ * accepted hits only, with the vertices read again rather than kept in
+ * registers; asked once, of the hit a traversal ends with, 1 % slower. */
 template<class R, int FEAT>
 __device__ __forceinline__ void test_triangle
   (const DScene<R>& S, int idx, V3<R> o, V3<R> d, const Shear<R>& sh, R tmin,
-   R eps, const SelfInfo& self, bool own, V3<R> inv, V3<R> oinv, Hit<R>& best, bool& found)
+   R eps, const SelfInfo& self, bool own, V3<R> inv, V3<R> oinv, R tleaf, Hit<R>& best,
+   bool& found)
 {
   const DTri<R> T = load_tri(S.tris + idx);
   const V3<R> p0 = ld3(T.v0), p1 = ld3(T.v1), p2 = ld3(T.v2);
@@ -640,10 +640,10 @@ __device__ __forceinline__ void test_triangle
   const R den = dot(ng, d);
   const R t = dot(ng, a) / den;
   if(!(t < best.t) || t <= eps || t <= tmin || T.gid == self.gid) return;
-  if constexpr(OwnBoxes<R, FEAT>::value) {
+  if constexpr(Pairs<R, FEAT>::value) {
     if(own) {
       asm volatile("" : "+r"(idx)); /* not the registers of the loads above */
-      if(!own_box(load_tri(S.tris + idx), inv, oinv, tmin, best.t)) return;
+      if(!own_box(load_tri(S.tris + idx), inv, oinv, tmin, tleaf)) return;
     }
   }
   const int side = den < R(0) ? 1 : 2;
@@ -759,14 +759,14 @@ __device__ bool trace_ray
    * lane's test. Each lane still meets nodes and primitives in the same order.
    * Beam-down, 6e7 paths, 115 -> 104 ms; the field is neutral. */
   for(;;) {
-    while(lc0 == 0 && node >= 0) {
+    while(lc0 == 0 && node >= 0 && !(Pairs<R, FEAT>::value && (node & PAIR_LEAF))) {
       const DNode<R> N = load_node(S.nodes + node);
       if(!(FEAT & FEAT_NOCOUNT)) ++cnt.nodes;
       R te[2];
       bool h[2];
-      h[0] = slab<OwnBoxes<R, FEAT>::value>(N.lo[0], N.hi[0], inv, oinv, tmin, best.t, te[0])
+      h[0] = slab<Pairs<R, FEAT>::value>(N.lo[0], N.hi[0], inv, oinv, tmin, best.t, te[0])
           && N.count[0] >= 0;
-      h[1] = slab<OwnBoxes<R, FEAT>::value>(N.lo[1], N.hi[1], inv, oinv, tmin, best.t, te[1])
+      h[1] = slab<Pairs<R, FEAT>::value>(N.lo[1], N.hi[1], inv, oinv, tmin, best.t, te[1])
           && N.count[1] >= 0;
       const bool l0 = h[0] && N.count[0] > 0, l1 = h[1] && N.count[1] > 0;
       lc0 = l0 ? N.count[0] : l1 ? N.count[1] : 0;
@@ -788,8 +788,19 @@ __device__ bool trace_ray
         node = stack[sp];
       }
     }
+    /* A pair's turn comes where its node's would, so that of two triangles
+     * met at one distance, on the edge they share, the same one is hit as in
+     * leaves of their own. (Tested with the node that lists them, sooner, field,
+     * 1e8 paths, 60.6 for 62.1 ms, but some hits changed places in flux maps.) */
+    if(Pairs<R, FEAT>::value && lc0 == 0 && node >= 0 && (node & PAIR_LEAF)) {
+      lc0 = 2 | PAIR_LEAF;
+      lf0 = node ^ PAIR_LEAF;
+      node = sp ? stack[--sp] : -1;
+    }
     if(lc0 == 0) break;
-    const int lc = lc0, first = lf0;
+    const bool own = Pairs<R, FEAT>::value && (lc0 & PAIR_LEAF);
+    const int lc = Pairs<R, FEAT>::value ? lc0 & ~PAIR_LEAF : lc0, first = lf0;
+    const R tleaf = best.t;
     lc0 = lc1;
     lf0 = lf1;
     lc1 = 0;
@@ -798,8 +809,7 @@ __device__ bool trace_ray
       if(!(FEAT & FEAT_QUADRIC) || primref_kind(ref) == PRIM_TRIANGLE) {
         if(!(FEAT & FEAT_NOCOUNT)) ++cnt.tris;
         test_triangle<R, FEAT>(S, (int)primref_index(ref), o, d, sh, tmin, eps, self,
-                               OwnBoxes<R, FEAT>::value && lc > 1 && S.own_boxes, inv, oinv,
-                               best, found);
+                               own, inv, oinv, tleaf, best, found);
       } else {
         if(!(FEAT & FEAT_NOCOUNT)) ++cnt.quads;
         test_quadric(S, (int)primref_index(ref), o, d, tmin, self, best, found);

@@ -686,12 +686,9 @@ __device__ __forceinline__ int lbvh_index(const DNode<R>* nodes, const int32_t* 
   return x;
 }
 
-/* With `pairs`, a node of two primitives becomes a leaf of two in its parent,
- * whose references are listed at its own index (the node's place stays, unread):
- * fewer node visits for a few more tests, which a warp makes together, as in
- * the host's tree of mesh scenes (default_leaf). With own boxes (test_triangle),
- * adjoint, 1e7 paths, 12.7 -> 10.7 ms; field of 317 under Buie's sun, 5.1e6,
- * 5.91 -> 5.80; one mirror, 1e6, 0.387 -> 0.373. */
+/* With `pairs`, a node of two primitives becomes a pair in its parent, whose
+ * references are listed at the node's index (its place stays, unread), as in
+ * the host's tree (joins_pairs). */
 template<class R>
 __device__ __forceinline__ void lbvh_permute(const DNode<R>* src, DNode<R>* dst,
                                              const int32_t* newidx, uint32_t* pairs, int i)
@@ -704,8 +701,7 @@ __device__ __forceinline__ void lbvh_permute(const DNode<R>* src, DNode<R>* dst,
     if(pairs && C.count[0] == 1 && C.count[1] == 1) {
       pairs[2 * at] = (uint32_t)C.child[0];
       pairs[2 * at + 1] = (uint32_t)C.child[1];
-      N.count[k] = 2;
-      N.child[k] = 2 * at;
+      N.child[k] = PAIR_LEAF | (2 * at);
     } else {
       N.child[k] = at;
     }

@@ -466,7 +466,6 @@ static void bind_scene(DScene<R>& S, const FlatScene<R>& f, const Blob& b,
   for(const DMaterial& m : f.mtls) S.spectral |= m.uniform != 3;
   for(const DMedium& m : f.media)
     S.spectral |= m.extinction.spectrum >= 0 || m.refractive_index.spectrum >= 0;
-  S.own_boxes = f.own_boxes;
   S.nsamp = (int32_t)f.samp.size();
   S.sun_type = f.sun_type;
   for(int c = 0; c < 3; ++c) S.sun_dir[c] = f.sun_dir[c];
@@ -507,7 +506,9 @@ static bool validate(const FlatScene<R>& f, bool need_samp = true)
   for(const DNode<R>& n : f.nodes) {
     if(f.device_bvh) break;
     for(int k = 0; k < 2; ++k) {
-      if(n.count[k] == 0) {
+      if(n.count[k] == 0 && (n.child[k] & PAIR_LEAF)) {
+        if(!f.pairs || (int64_t)(n.child[k] ^ PAIR_LEAF) + 2 > nrefs) return false;
+      } else if(n.count[k] == 0) {
         if(n.child[k] <= 0 || n.child[k] >= nnodes) return false;
       } else if(n.count[k] == 1) {
         const uint32_t ref = (uint32_t)n.child[k];
@@ -1002,14 +1003,13 @@ static res_T swap_sah(ssol_b200_plan* p, const FlatScene<R>& f, DScene<R>& S)
     boxes[i].ref = f.prim_ref[i];
   }
   BvhBuildParams bp;
-  /* The caller's leaf size, where own boxes keep the paths of the first part */
-  bp.max_leaf = default_leaf(f);
-  if(bp.max_leaf > 1 && p->opt.bvh_leaf_size) bp.max_leaf = p->opt.bvh_leaf_size;
+  bp.max_leaf = 1; /* as the device's: the same paths */
   bp.threads = host_threads();
   BvhResult r;
   build_bvh(std::move(boxes), bp, r);
   if(r.depth > 30) return RES_OK;
-  const std::vector<DNode<R>> nodes = bvh_nodes<R>(r);
+  std::vector<DNode<R>> nodes = bvh_nodes<R>(r);
+  if(f.pairs) join_pairs(nodes, r.primrefs);
   Blob b;
   const size_t o_nodes = b.add(nodes);
   const size_t o_refs = b.add(r.primrefs);
@@ -1028,7 +1028,6 @@ static res_T swap_sah(ssol_b200_plan* p, const FlatScene<R>& f, DScene<R>& S)
   unsigned char* base = (unsigned char*)p->d_bvh2;
   S.nodes = (const DNode<R>*)(base + o_nodes);
   S.primrefs = (const uint32_t*)(base + o_refs);
-  S.own_boxes = bp.max_leaf > 1;
   p->bvh_device = false;
   p->bvh_depth = r.depth;
   p->bvh_nodes = nodes.size();
@@ -1602,14 +1601,14 @@ extern "C" res_T ssol_b200_batch_create
   if(opt.precision == SSOL_B200_FP32) f32.resize(nscenes);
   else f64.resize(nscenes);
   parallel_for(nscenes, snapshot);
-  /* One kernel variant traces every item: where it does not keep to own boxes
-   * (OwnBoxes), the items that count on them get leaves of one */
+  /* One kernel variant traces every item: where it does not know pairs
+   * (Pairs), the items that have some get leaves of one */
   int features = 0;
   for(const FlatScene<float>& f : f32) features |= f.meta.features;
   if((features & (FEAT_QUADRIC | FEAT_DIELECTRIC)) && !(features & FEAT_ATTRIBUTES)) {
     bp.max_leaf = bp.max_leaf ? bp.max_leaf : 1;
     parallel_for(nscenes, [&](size_t i) {
-      if(item_res[i] == RES_OK && f32[i].own_boxes) snapshot(i);
+      if(item_res[i] == RES_OK && f32[i].pairs) snapshot(i);
     });
   }
   for(size_t i = 0; i < nscenes; ++i) {
@@ -1753,7 +1752,7 @@ static res_T tracking_upload
   int maxd = 0;
   for(size_t i = 0; i < nnodes; ++i)
     for(int k = 0; k < 2; ++k)
-      if(f.nodes[i].count[k] == 0) {
+      if(f.nodes[i].count[k] == 0 && !(f.nodes[i].child[k] & PAIR_LEAF)) {
         const int c = f.nodes[i].child[k];
         depth[c] = depth[i] + 1;
         maxd = std::max(maxd, depth[c]);
