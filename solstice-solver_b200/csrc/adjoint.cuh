@@ -356,7 +356,7 @@ __device__ __forceinline__ void adjoint_flush(const AdjointArgs& A, int slot, do
  * local memory 4.65 and 5.8; and with 4 blocks of 64 registers an SM instead
  * of 2 of 128 in the mesh variant, 3.9 and 5.2 (3 blocks 4.2 and 5.3). */
 template<class R, int PASS, int FEAT>
-__global__ void __launch_bounds__(MAX_BLOCK, FEAT == 0 ? 4 : 2)
+__global__ void __launch_bounds__(MAX_BLOCK, FEAT & FEAT_ALL ? 2 : 4)
 adjoint_kernel(const DScene<R> S, const AdjointArgs A, uint64_t seed, uint64_t first,
                uint32_t count, const uint32_t* sorted_off, uint32_t seg_len, uint32_t seg_mul)
 {
@@ -463,9 +463,9 @@ static int launch_adjoint_impl
 {
   const cudaStream_t s = (cudaStream_t)stream;
   if constexpr(sizeof(R) == sizeof(float)) {
-    if(A.features == 0)
-      return pass == 0 ? launch_adjoint_variant<R, 0, 0>(S, A, seed, first, count, s)
-                       : launch_adjoint_variant<R, 1, 0>(S, A, seed, first, count, s);
+    if((A.features & FEAT_ALL) == 0)
+      return pass == 0 ? launch_adjoint_variant<R, 0, FEAT_PAIRS>(S, A, seed, first, count, s)
+                       : launch_adjoint_variant<R, 1, FEAT_PAIRS>(S, A, seed, first, count, s);
   }
   return pass == 0 ? launch_adjoint_variant<R, 0, FEAT_ALL>(S, A, seed, first, count, s)
                    : launch_adjoint_variant<R, 1, FEAT_ALL>(S, A, seed, first, count, s);

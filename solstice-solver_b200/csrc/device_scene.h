@@ -206,14 +206,16 @@ enum : int32_t {
   FEAT_ALL = 7,
   /* Not a scene feature: the plain kernel variant that does not count rays,
    * node visits and primitive tests (one instruction per node visit) */
-  FEAT_NOCOUNT = 8
+  FEAT_NOCOUNT = 8,
+  /* Nor this: the tree has pairs of triangles (PAIR_LEAF); set in the features
+   * of a snapshot whose tree joins some */
+  FEAT_PAIRS = 16
 };
 
-/* Kernel variants that know pairs of triangles (PAIR_LEAF): FP32 without
- * quadrics or dielectrics, and FP32 with everything */
+/* Kernel variants that know pairs of triangles, in FP32 only: those made for
+ * them, and the one with every scene feature */
 template<class R, int FEAT> struct Pairs {
-  static constexpr bool value = sizeof(R) == sizeof(float)
-    && (!(FEAT & (FEAT_QUADRIC | FEAT_DIELECTRIC)) || (FEAT & FEAT_ATTRIBUTES));
+  static constexpr bool value = sizeof(R) == sizeof(float) && (FEAT & (FEAT_PAIRS | FEAT_ATTRIBUTES));
 };
 
 /* Counters for the roofline model (see kernels_device.cuh) */

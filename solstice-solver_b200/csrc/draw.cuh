@@ -367,7 +367,7 @@ __device__ __forceinline__ bool draw_radiance
  * registers, four blocks an SM, 6.0 (80: 6.3). The draft's kernel, 0.62 ->
  * 0.42 ms, is fastest in the registers it takes by itself (64). */
 template<class R, int FEAT>
-__global__ void __launch_bounds__(256, FEAT == 0 ? 4 : 1) pt_kernel(const DScene<R> S, const DrawArgs A)
+__global__ void __launch_bounds__(256, FEAT & FEAT_ALL ? 1 : 4) pt_kernel(const DScene<R> S, const DrawArgs A)
 {
   int px, py;
   draw_pixel_of(blockIdx.x, threadIdx.x, A.width, px, py);
@@ -431,8 +431,8 @@ static int launch_draw(const DScene<R>& S, const DrawArgs& A, bool pt, void* str
   const unsigned grid = (unsigned)(ntx * nty);
   const cudaStream_t st = (cudaStream_t)stream;
   if constexpr(sizeof(R) == sizeof(float)) {
-    if(A.features == 0) {
-      launch_draw_variant<R, 0>(S, A, pt, grid, st);
+    if((A.features & FEAT_ALL) == 0) {
+      launch_draw_variant<R, FEAT_PAIRS>(S, A, pt, grid, st);
       return (int)cudaGetLastError();
     }
   }

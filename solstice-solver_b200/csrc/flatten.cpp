@@ -980,6 +980,7 @@ static res_T flatten_impl
     const size_t n = boxes.size();
     out.device_bvh = true;
     out.pairs = joins_pairs(out);
+    if(out.pairs) out.meta.features |= FEAT_PAIRS;
     out.prim_box.resize(6 * n);
     out.prim_ref.resize(n);
     for(size_t i = 0; i < n; ++i) {
@@ -997,7 +998,10 @@ static res_T flatten_impl
   }
   build_bvh(boxes, prm, out.bvh);
   out.nodes = bvh_nodes<R>(out.bvh);
-  if(out.pairs) join_pairs(out.nodes, out.bvh.primrefs);
+  if(out.pairs) {
+    join_pairs(out.nodes, out.bvh.primrefs);
+    out.meta.features |= FEAT_PAIRS;
+  }
   return RES_OK;
 }
 

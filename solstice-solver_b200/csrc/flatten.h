@@ -96,8 +96,8 @@ template<class R> struct FlatScene {
 /* Whether a tree that the library chooses joins pairs of triangles: a node of
  * two triangles gives way to a pair in its parent, so that a ray makes fewer
  * node visits for a few more triangle tests, which a warp makes together.
- * Leaves of their own / pairs: field of 1000, plan launch of 1e8 paths, 63.4 /
- * 62.1 ms; adjoint, 1e7, 12.1 / 11.0; batch of 32 suns 29.6 / 29.1; path-traced
+ * Leaves of their own / pairs: field of 1000, plan launch of 1e8 paths, 62.1 /
+ * 61.1 ms; adjoint, 1e7, 12.1 / 11.0; batch of 32 suns 29.6 / 29.1; path-traced
  * view 7.63 / 7.54.
  * Not in FP64, where the test of own boxes costs more than the pairs give
  * (field of 500, solve of 2e6, 3.80 ms, with pairs 3.94), and not with punched

@@ -110,16 +110,17 @@ static int launch_batch_noalloc_impl
    const unsigned long long* h_prefix, const unsigned long long* h_firsts,
    const LaunchConfig& cfg, void* stream)
 {
-  if(sizeof(R) == sizeof(float) && cfg.features == 0) {
-    switch(cfg.min_blocks) {
-      case 1: return launch_batch_noalloc_variant<R, 1, 0>
-        (scenes, tallies, nitems, seed, h_prefix, h_firsts, cfg, stream);
-      case 3: return launch_batch_noalloc_variant<R, 3, 0>
-        (scenes, tallies, nitems, seed, h_prefix, h_firsts, cfg, stream);
-      default: return launch_batch_noalloc_variant<R, 2, 0>
-        (scenes, tallies, nitems, seed, h_prefix, h_firsts, cfg, stream);
+  if constexpr(sizeof(R) == sizeof(float))
+    if((cfg.features & FEAT_ALL) == 0) {
+      switch(cfg.min_blocks) {
+        case 1: return launch_batch_noalloc_variant<R, 1, FEAT_PAIRS>
+          (scenes, tallies, nitems, seed, h_prefix, h_firsts, cfg, stream);
+        case 3: return launch_batch_noalloc_variant<R, 3, FEAT_PAIRS>
+          (scenes, tallies, nitems, seed, h_prefix, h_firsts, cfg, stream);
+        default: return launch_batch_noalloc_variant<R, 2, FEAT_PAIRS>
+          (scenes, tallies, nitems, seed, h_prefix, h_firsts, cfg, stream);
+      }
     }
-  }
   switch(cfg.min_blocks) {
     case 1: return launch_batch_noalloc_variant<R, 1, FEAT_ALL>
       (scenes, tallies, nitems, seed, h_prefix, h_firsts, cfg, stream);

@@ -1588,27 +1588,17 @@ extern "C" res_T ssol_b200_batch_create
   std::vector<FlatScene<double>> f64;
   /* Snapshots of the items in parallel on the host threads */
   std::vector<res_T> item_res(nscenes, RES_OK);
-  auto snapshot = [&](size_t i) {
-    if(opt.precision == SSOL_B200_FP32) {
-      f32[i] = FlatScene<float>();
+  if(opt.precision == SSOL_B200_FP32) {
+    f32.resize(nscenes);
+    parallel_for(nscenes, [&](size_t i) {
       item_res[i] = flatten_scene(scenes[i], bp, f32[i]);
       if(item_res[i] == RES_OK && !validate(f32[i])) item_res[i] = RES_UNKNOWN_ERR;
-    } else {
+    });
+  } else {
+    f64.resize(nscenes);
+    parallel_for(nscenes, [&](size_t i) {
       item_res[i] = flatten_scene(scenes[i], bp, f64[i]);
       if(item_res[i] == RES_OK && !validate(f64[i])) item_res[i] = RES_UNKNOWN_ERR;
-    }
-  };
-  if(opt.precision == SSOL_B200_FP32) f32.resize(nscenes);
-  else f64.resize(nscenes);
-  parallel_for(nscenes, snapshot);
-  /* One kernel variant traces every item: where it does not know pairs
-   * (Pairs), the items that have some get leaves of one */
-  int features = 0;
-  for(const FlatScene<float>& f : f32) features |= f.meta.features;
-  if((features & (FEAT_QUADRIC | FEAT_DIELECTRIC)) && !(features & FEAT_ATTRIBUTES)) {
-    bp.max_leaf = bp.max_leaf ? bp.max_leaf : 1;
-    parallel_for(nscenes, [&](size_t i) {
-      if(item_res[i] == RES_OK && f32[i].pairs) snapshot(i);
     });
   }
   for(size_t i = 0; i < nscenes; ++i) {

@@ -49,20 +49,18 @@ def test_leaves_and_builders_trace_the_same_paths(product, elevation, azimuth, d
     assert _worst(device[:-flux], one[:-flux]) < 1e-10
 
 
-def test_mixed_batch_has_leaves_of_one(product):
-    """Items without quadrics in a batch with them: the variant that traces
-    them all takes leaves of one (the same node visits), and the estimates are
-    those of the item alone."""
+def test_mixed_batch(product):
+    """An item whose tree has pairs in a batch with quadrics and dielectrics: the
+    estimates are those of the item alone."""
     field = W.heliostat_field(product, n_helio=37, receiver_cells=7)[0]
     down = W.beam_down(product, n_helio=60, receiver_cells=5)[0]
-    got = []
-    for leaf in (0, 1):
-        b = P.Batch(product, [field, down], P.options(leaf=leaf, count=1))
+    for launch in ("launch", "launch_noalloc"):
+        b = P.Batch(product, [field, down])
         rng = field.rng(seed=3)
-        b.launch(rng, [30011, 20011])
-        est = b.finish(rng)
-        got.append((est[0].globals(), est[0].stats()["node_visits"]))
-    assert got[0][1] == got[1][1]
-    alone = field.solve(30011, seed=3).globals()
-    for k in alone:
-        assert got[0][0][k][0] == pytest.approx(alone[k][0], rel=1e-10, abs=1e-10), k
+        getattr(b, launch)(rng, [30011, 20011])
+        got = b.finish(rng)
+        for s, e, n in ((field, got[0], 30011), (down, got[1], 20011)):
+            alone, mixed = s.solve(n, seed=3).globals(), e.globals()
+            for k in alone:
+                assert mixed[k][0] == pytest.approx(alone[k][0], rel=1e-10, abs=1e-10), k
+        b.close()
