@@ -39,9 +39,10 @@ enum ssol_b200_precision {
  *    deeper than the traversal stack allows (more than 30 levels) is rebuilt on
  *    the host with the SAH builder, with a warning;
  *  - SSOL_B200_BVH_AUTO (the default): ssol_solve, ssol_solve_ex (whatever
- *    bvh_leaf_size) and, when bvh_leaf_size is 0, ssol_solve_adjoint use the
- *    device builder for at most SSOL_B200_BVH_AUTO_MAX_PATHS realisations,
- *    where building is a large part of the call. Larger solves start on the
+ *    bvh_leaf_size) and, when bvh_leaf_size is 0 and the scene has some
+ *    hundred primitives or more (449), ssol_solve_adjoint use the device
+ *    builder for at most SSOL_B200_BVH_AUTO_MAX_PATHS realisations, where
+ *    building is a large part of the call. Larger solves start on the
  *    device's tree and, after their first 6e6 realisations, trace on the SAH
  *    tree that the host threads built meanwhile. Plans, which do not know how
  *    many realisations they will trace, use the SAH builder.
@@ -53,8 +54,8 @@ enum ssol_b200_precision {
  * whose axes are the scene's). With leaves of two or more that the caller asks
  * for (bvh_leaf_size), the box that counts is the leaf's. Batches always use
  * the SAH builder. The renderers use the device builder by default
- * (bvh_leaf_size 0) for images of at most SSOL_B200_BVH_AUTO_MAX_SAMPLES camera
- * samples, the SAH builder above. */
+ * (bvh_leaf_size 0, 449 primitives or more) for images of at most
+ * SSOL_B200_BVH_AUTO_MAX_SAMPLES camera samples, the SAH builder otherwise. */
 enum ssol_b200_bvh_builder {
   SSOL_B200_BVH_AUTO = 0,
   SSOL_B200_BVH_SAH = 1,

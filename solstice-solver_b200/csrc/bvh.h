@@ -24,9 +24,20 @@ struct BvhBuildParams {
   int max_depth = 30; /* the device traversal stack holds 32 entries */
   int threads = 1; /* host threads for the subtrees of large scenes */
   /* Leave the tree to the device builder (lbvh.cu): the snapshot keeps the
-   * primitive boxes instead (scenes of at least 2 primitives) */
+   * primitive boxes instead (scenes of at least device_min primitives, 2 or
+   * more) */
   bool device = false;
+  size_t device_min = 2;
 };
+
+/* device_min of the renderers and the adjoint, where the caller leaves the
+ * builder open: below, the host builds the tree in less time than the device's
+ * one block, its launch and the read-back of the depth take. us a call, host /
+ * device: draft of 64 x 64 pixels, 34 primitives 74 / 182, 130 110 / 265, 228
+ * 173 / 302, 328 218 / 297, 428 317 / 332, 528 410 / 360, 928 744 / 438;
+ * adjoint, 1e3 paths, 130 282 / 443, 328 483 / 549, 428 571 / 578, 528 668 /
+ * 615, 928 1084 / 743. */
+constexpr size_t DEVICE_BUILD_MIN = 449;
 
 struct BvhResult {
   std::vector<double> lo, hi; /* per node child boxes: node*2+k, 3 each */

@@ -976,7 +976,7 @@ static res_T flatten_impl
       out.meta.aabb_lo[c] = std::min(out.meta.aabb_lo[c], b.lo[c]);
       out.meta.aabb_hi[c] = std::max(out.meta.aabb_hi[c], b.hi[c]);
     }
-  if(bvh_params.device && boxes.size() >= 2) {
+  if(bvh_params.device && boxes.size() >= std::max<size_t>(bvh_params.device_min, 2)) {
     const size_t n = boxes.size();
     out.device_bvh = true;
     out.pairs = joins_pairs(out);

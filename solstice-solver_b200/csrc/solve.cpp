@@ -707,6 +707,7 @@ res_T ssolb_snapshot_create
   bp.device = opt.bvh_builder == SSOL_B200_BVH_LBVH
     || (opt.bvh_builder == SSOL_B200_BVH_AUTO && bp.max_leaf == 0
         && samples <= SSOL_B200_BVH_AUTO_MAX_SAMPLES);
+  if(opt.bvh_builder == SSOL_B200_BVH_AUTO) bp.device_min = DEVICE_BUILD_MIN;
   out.precision = opt.precision;
   std::unique_ptr<FlatScene<float>> f32;
   std::unique_ptr<FlatScene<double>> f64;
@@ -775,10 +776,11 @@ extern "C" res_T ssol_b200_plan_ref_put(ssol_b200_plan* p)
 }
 
 /* keep_flat: with a device-built tree, the plan keeps its snapshot for
- * plan_swap_sah */
+ * plan_swap_sah. Scenes of fewer than device_min primitives get the host's
+ * tree. */
 static res_T plan_create_impl
   (ssol_scene* scn, const ssol_b200_options* options, ssol_b200_plan** out,
-   bool keep_flat)
+   bool keep_flat, size_t device_min = 2)
 {
   if(!scn || !out) return RES_BAD_ARG;
   ssol_b200_options opt = options ? *options : SSOL_B200_OPTIONS_DEFAULT;
@@ -800,6 +802,7 @@ static res_T plan_create_impl
   bp.max_leaf = opt.bvh_leaf_size;
   bp.threads = host_threads();
   bp.device = opt.bvh_builder == SSOL_B200_BVH_LBVH;
+  bp.device_min = device_min;
 
   /* Snapshot on the host first: argument errors need no GPU */
   std::unique_ptr<FlatScene<float>> f32;
@@ -1208,13 +1211,16 @@ extern "C" res_T ssol_solve_adjoint
 
   /* The default builder by size, as for a solve: for 1e7 paths of 1000
    * heliostats the host's tree takes 3 ms longer to build and traces both
-   * passes 0.4 ms faster */
+   * passes 0.4 ms faster; by the scene's too, as for the renderers */
   ssol_b200_options opt = options ? *options : SSOL_B200_OPTIONS_DEFAULT;
+  size_t device_min = 2;
   if(opt.bvh_builder == SSOL_B200_BVH_AUTO && opt.bvh_leaf_size == 0
-  && (unsigned long long)n <= SSOL_B200_BVH_AUTO_MAX_PATHS)
+  && (unsigned long long)n <= SSOL_B200_BVH_AUTO_MAX_PATHS) {
     opt.bvh_builder = SSOL_B200_BVH_LBVH;
+    device_min = DEVICE_BUILD_MIN;
+  }
   ssol_b200_plan* plan = nullptr;
-  res_T res = ssol_b200_plan_create(scn, &opt, &plan);
+  res_T res = plan_create_impl(scn, &opt, &plan, false, device_min);
   if(res != RES_OK) return res;
   const cudaStream_t s = plan_stream(plan, nullptr);
   const size_t ncell = (size_t)map->nx * map->ny;
