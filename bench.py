@@ -43,27 +43,29 @@ WORKLOAD = ("1000 flat 10x10 heliostats (radial staggered, r 100-600 m, Beckmann
 # of 2^24 paths each)
 # (dram__bytes_read.sum + dram__bytes_write.sum);
 # the traffic scales with the paths traced (per-thread frames written back)
-DRAM_BYTES_PER_PATH = {"field": (121.6e6 + 2698.4e6) / 16777216,
-                       "beamdown": (447.9e6 + 4585.7e6) / 16777216}
+DRAM_BYTES_PER_PATH = {"field": (115.1e6 + 2852.5e6) / 16777216,
+                       "beamdown": (482.6e6 + 4845.3e6) / 16777216}
 
 # Kernels of one plain launch of n realisations: the realisation kernel, with
 # the coherent order's presort (count, scan, scatter) before it from SORT_MIN
 # realisations on (more with quadrics, never with one sampled mirror), per
-# chunk of at most 2^24; and the sums that follow from others, once
+# chunk of at most 2^24; and the sums that follow from others, once (cleared
+# first for the 5000 heliostats of the beam-down plant)
 SORT_MIN = {"field": 200_000, "beamdown": 1_000_000}
 SORT_CHUNK = 1 << 24
 
 
 def launches_per_plain_launch(n, config):
+    finish = 2 if config == "beamdown" else 1
     if n < SORT_MIN.get(config, n + 1):
-        return 2
-    return 4 * ((n + SORT_CHUNK - 1) // SORT_CHUNK) + 1
+        return 1 + finish
+    return 4 * ((n + SORT_CHUNK - 1) // SORT_CHUNK) + finish
 
 
 # Both passes of the adjoint kernel on the field, from a capture of 4e6 paths
-ADJOINT_DRAM_BYTES_PER_PATH = (24.6e6 + 61.1e6 + 152.2e6 + 1395.3e6) / 4e6
-# Same for the batched kernel, from a capture of 32 suns (18907863 paths)
-BATCH_DRAM_BYTES_PER_PATH = (208.5e6 + 4448.8e6) / 18907863
+ADJOINT_DRAM_BYTES_PER_PATH = (26.2e6 + 88.1e6 + 154.1e6 + 1317.6e6) / 4e6
+# Same for the batched kernel, from a capture of 32 suns (24018813 paths)
+BATCH_DRAM_BYTES_PER_PATH = (271.1e6 + 6010.3e6) / 24018813
 
 
 def flops_per_run(st):
