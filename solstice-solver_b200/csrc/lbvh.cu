@@ -30,8 +30,8 @@
  *      the root's height is the tree depth, which the host reads back to check
  *      the traversal stack bound;
  *   7. the internal nodes are renumbered depth first, slot 0 first, so that
- *      a node's first child follows it in memory; in FP32 scenes of meshes a
- *      node of two primitives becomes a leaf of two.
+ *      a node's first child follows it in memory; where the tree joins pairs
+ *      (joins_pairs), a node of two primitives becomes one of its parent.
  * Scenes of at most SMALL_BUILD primitives go through all of them in one
  * launch.
  */
