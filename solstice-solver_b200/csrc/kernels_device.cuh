@@ -1598,41 +1598,62 @@ static __device__ __forceinline__ void commit_warp
 
 /* The sums that follow from others, once a launch (block y: the item): a
  * receiver side's from its samp_rcv slots, the global cosine and shadowed
- * from the samp slots. Block x < nrcv: that receiver side; the last one: the
- * globals. Block z: its slice of the sampled instances; slices add up in what
+ * from the samp slots. Block x: that group of `group` receiver sides, whose
+ * slots of one sampled instance are neighbours; the last one: the globals.
+ * Block z: its slice of the sampled instances; slices add up in what
  * finish_clear has zeroed, a single one stores. */
-constexpr int FINISH_LANES = 48; /* sampled instances in flight per quantity */
+constexpr int FINISH_BLOCK = 960;
 template<class R>
-__global__ void __launch_bounds__(FINISH_LANES * NRCV_Q * 2) finish_tallies
+__global__ void __launch_bounds__(FINISH_BLOCK) finish_tallies
   (const DScene<R>* scenes, const DTallies* tallies, const DTallies one, int nrcv,
-   int nsampled)
+   int nsampled, int group)
 {
-  __shared__ double part[FINISH_LANES][NRCV_Q * 2];
+  __shared__ double2 part[FINISH_BLOCK];
   const DTallies& T = tallies ? tallies[blockIdx.y] : one;
   if(scenes) { nrcv = scenes[blockIdx.y].nrcv; nsampled = scenes[blockIdx.y].nsampled; }
-  const int r = (int)blockIdx.x;
-  const int q = threadIdx.x % (NRCV_Q * 2), l = threadIdx.x / (NRCV_Q * 2);
-  const bool glob = r == (int)gridDim.x - 1;
+  const bool glob = blockIdx.x == gridDim.x - 1;
+  const int r = (int)blockIdx.x * group;
   if(!glob && r >= nrcv) return;
-  const double* src = glob ? T.samp + q : T.samp_rcv + (size_t)r * NRCV_Q * 2 + q;
-  const size_t step = glob ? 4 : (size_t)nrcv * NRCV_Q * 2;
-  double v = 0;
+  /* Sums in pairs (16-byte loads): 10 of a receiver side, 2 of the globals */
+  const int width = glob ? 2 : min(group, nrcv - r) * NRCV_Q;
+  const int lanes = FINISH_BLOCK / width;
+  const int q = threadIdx.x % width, l = threadIdx.x / width;
+  const double2* src = reinterpret_cast<const double2*>
+    (glob ? T.samp : T.samp_rcv + (size_t)r * NRCV_Q * 2) + q;
+  const size_t step = glob ? 2 : (size_t)nrcv * NRCV_Q;
+  double2 v = make_double2(0.0, 0.0);
   const int per = (nsampled + (int)gridDim.z - 1) / (int)gridDim.z;
   const int last = min(nsampled, ((int)blockIdx.z + 1) * per);
-  if(!glob || q < 4)
-#pragma unroll 4
-    for(int s = (int)blockIdx.z * per + l; s < last; s += FINISH_LANES)
-      v += src[(size_t)s * step];
-  part[l][q] = v;
-  __syncthreads();
+  if(l < lanes)
+#pragma unroll 8
+    for(int s = (int)blockIdx.z * per + l; s < last; s += lanes) {
+      const double2 w = __ldcs(src + (size_t)s * step); /* the scene stays in the L2 */
+      v.x += w.x;
+      v.y += w.y;
+    }
+  part[threadIdx.x] = v;
+  /* Halves of the lanes, then the sums of the first one */
+  for(int n = lanes; n > 1; ) {
+    const int h = (n + 1) / 2;
+    __syncthreads();
+    if(l < n - h) {
+      const double2 w = part[threadIdx.x + h * width];
+      v.x += w.x;
+      v.y += w.y;
+      part[threadIdx.x] = v;
+    }
+    n = h;
+  }
   if(l) return;
-  v = 0;
-  for(int k = 0; k < FINISH_LANES; ++k) v += part[k][q];
-  if(glob && q >= 4) return;
-  double* dst = glob ? T.global + (q < 2 ? 2 * G_COS + q : 2 * G_SHADOW + q - 2)
-                     : T.rcv + (size_t)r * NRCV_Q * 2 + q;
-  if(gridDim.z == 1) *dst = v;
-  else red_add_global(dst, v);
+  double* dst = glob ? T.global + (q == 0 ? 2 * G_COS : 2 * G_SHADOW)
+                     : T.rcv + (size_t)r * NRCV_Q * 2 + 2 * q;
+  if(gridDim.z == 1) {
+    dst[0] = v.x;
+    dst[1] = v.y;
+  } else {
+    red_add_global(dst, v.x);
+    red_add_global(dst + 1, v.y);
+  }
 }
 template<class R>
 __global__ void __launch_bounds__(256) finish_clear
@@ -1651,19 +1672,36 @@ __global__ void __launch_bounds__(256) finish_clear
  * where there are more. One block for all of a receiver side's grew with the
  * plant: us a plan launch of 1e4 paths, one receiver side, one block / slices:
  * 2000 sampled instances 124 / 123 (of two launches), 2500 126 / 122, 5000
- * 138 / 125, 20,000 198 / 128, 1e5 418 / 127. */
+ * 138 / 125, 20,000 198 / 128, 1e5 418 / 127.
+ * Many receiver sides of many instances fill more than a share of the L2 and
+ * are bound by HBM. From 64 MB on a block takes FINISH_WIDE neighbouring sides
+ * (1920 bytes of a row), in as many slices as one wave of blocks has, of
+ * FINISH_DEEP rows a thread or more; below, the same takes as long. Plan launches
+ * of 1e4 paths, a side a block / so: 20,000 x 100 sides (320 MB) 237 / 209 us,
+ * 5000 x 400 227 / 207, 5000 x 100 168 / 160. */
 constexpr int FINISH_SINGLE = 2048, FINISH_SLICE = 1024, FINISH_SLICES_MAX = 64;
+constexpr int FINISH_WIDE = 12, FINISH_DEEP = 8, FINISH_WAVE = 2 * 148;
+constexpr uint64_t FINISH_WIDE_SLOTS = 400000;
 template<class R>
 static void launch_finish(const DScene<R>* scenes, const DTallies* tallies, const DTallies& one,
                           int nitems, int nrcv, int nsampled, cudaStream_t st)
 {
-  const int slices = nsampled <= FINISH_SINGLE ? 1
-    : std::min((nsampled + FINISH_SLICE - 1) / FINISH_SLICE, FINISH_SLICES_MAX);
+  int group = 1, slices = 1;
+  if(nrcv > 1 && (uint64_t)nitems * nrcv * nsampled >= FINISH_WIDE_SLOTS) {
+    group = std::min(nrcv, FINISH_WIDE);
+    const int rows = FINISH_DEEP * (FINISH_BLOCK / (group * NRCV_Q));
+    const int64_t blocks = (int64_t)nitems * ((nrcv + group - 1) / group + 1);
+    slices = (int)std::min<int64_t>((nsampled + rows - 1) / rows,
+                                    std::max<int64_t>(FINISH_WAVE / blocks, 1));
+  } else if(nsampled > FINISH_SINGLE) {
+    slices = std::min((nsampled + FINISH_SLICE - 1) / FINISH_SLICE, FINISH_SLICES_MAX);
+  }
   if(slices > 1) finish_clear<R><<<(unsigned)nitems, 256, 0, st>>>(scenes, tallies, one, nrcv);
+  const unsigned groups = (unsigned)((nrcv + group - 1) / group);
   for(int i = 0; i < nitems; i += 65535)
-    finish_tallies<R><<<dim3((unsigned)nrcv + 1, (unsigned)std::min(nitems - i, 65535),
-                             (unsigned)slices), FINISH_LANES * NRCV_Q * 2, 0, st>>>
-      (scenes ? scenes + i : nullptr, tallies ? tallies + i : nullptr, one, nrcv, nsampled);
+    finish_tallies<R><<<dim3(groups + 1, (unsigned)std::min(nitems - i, 65535),
+                             (unsigned)slices), FINISH_BLOCK, 0, st>>>
+      (scenes ? scenes + i : nullptr, tallies ? tallies + i : nullptr, one, nrcv, nsampled, group);
 }
 
 /*******************************************************************************

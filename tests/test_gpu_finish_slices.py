@@ -1,7 +1,8 @@
 """The sums that follow from others (a receiver side's, the global cosine and
 shadowed) around the numbers of sampled instances at which one block no longer
-adds them all up (2048) and at which its slices grow (65536): they are the sums
-of the per-instance ones, after each of two launches, in plans and batches. Both
+adds them all up (2048) and at which its slices grow (65536), and of the slots
+(400000) from which a block takes several receiver sides: they are the sums of
+the per-instance ones, after each of two launches, in plans and batches. Both
 are sums of the same positive FP64 numbers, so they differ by their order only
 (n 2^-53 = 1e-11 at most; 1e-10)."""
 import ctypes as C
@@ -14,8 +15,9 @@ import pyssol as P
 pytestmark = pytest.mark.gpu
 
 
-def _scene(lib, n):
-    """n mirrors of 1 m2 in a square grid under two receivers, front and back."""
+def _scene(lib, n, k=0):
+    """n mirrors of 1 m2 in a square grid under two receivers, front and back, or
+    under k x k ones."""
     s = P.Scene(lib)
     m, rm = s.mirror(0.9, 1e-3), s.mirror(0.05, 0.0)
     o = s.object([(s.rectangle(0.5, 0.5), m, m)])
@@ -23,7 +25,13 @@ def _scene(lib, n):
     for i in range(n):
         s.instance(o, P.transform_from(None, (1.5 * (i % side), 1.5 * (i // side), 0.0)))
     w = 0.75 * side
-    for x in (0.3 * w, 1.5 * w):
+    if k:
+        rect = s.object([(s.rectangle(0.6 * w / k, 0.6 * w / k), rm, rm)])
+    for i in range(k * k):
+        s.instance(rect, P.transform_from(P.rotation_pitch_pi(),
+                                          (w * (2 * (i % k) + 1) / k, w * (2 * (i // k) + 1) / k, 1.0)),
+                   receiver=P.SSOL_FRONT | P.SSOL_BACK, sample=0)
+    for x in () if k else (0.3 * w, 1.5 * w):
         s.instance(s.object([(s.rectangle(0.5 * w, w), rm, rm)]),
                    P.transform_from(P.rotation_pitch_pi(), (x, w, 30.0)),
                    receiver=P.SSOL_FRONT | P.SSOL_BACK, sample=0)
@@ -44,9 +52,11 @@ def _check(sums, n, nrcv=4):
     torch.testing.assert_close(glob[[0, 1, 4, 5]], want, rtol=1e-10, atol=0)
 
 
-@pytest.mark.parametrize("n", [2047, 2048, 2049, 4097, 65537])
-def test_sums_of_slices(product, n):
-    s = _scene(product, n)
+@pytest.mark.parametrize("n,k", [(2047, 0), (2048, 0), (2049, 0), (4097, 0), (65537, 0),
+                                 (887, 15), (889, 15), (95, 46), (97, 46), (22222, 3), (22223, 3),
+                                 (99999, 0), (100000, 0)])
+def test_sums_of_slices(product, n, k):
+    s = _scene(product, n, k)
     h = C.c_void_p()
     opt = P.options()
     product.call("ssol_b200_plan_create", s.scn, C.byref(opt), C.byref(h))
@@ -56,7 +66,7 @@ def test_sums_of_slices(product, n):
             product.call("ssol_b200_plan_launch", h, rng, first, 150001, None)
             torch.cuda.synchronize()
             sums, _ = P.plan_tallies(product, h)
-            _check(torch.as_tensor(sums, device="cuda"), n)
+            _check(torch.as_tensor(sums, device="cuda"), n, 2 * k * k or 4)
     finally:
         product.raw("ssol_b200_plan_ref_put", h)
 
